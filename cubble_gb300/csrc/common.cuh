@@ -155,6 +155,20 @@ struct Ctrl {
     unsigned int done[DC_COUNT];
 };
 
+// What a resident run's blocks (below) reduce into and wait on, in global
+// memory: zero between launches.
+struct RunAcc {
+    double sum[2];       // predict: area, area over radius
+    double osum[2];      // pairs: overlap area, overlap area over radius
+    double csum[5];      // correct: volume; mixed form: the candidates' sums
+    long long cmax[3];   // correct: error, radius, expansion (bits of doubles >= 0)
+    int cnt[2];          // correct: deletions, non-finite values
+};
+struct RunSync {
+    RunAcc acc[2];  // of even and odd attempts
+    unsigned arrive, pad_[31], exits, pad2_[31];
+};
+
 // Every device buffer of a context; kernels take it by value.
 struct Bufs {
     Ctrl *ctrl;
@@ -189,6 +203,7 @@ struct Bufs {
     int *stash;         // cap x kStash(dim): pair partners found by the counting pass
     double *dbg_ov;     // optional copy of the overlap row (cb_attempt)
     double *energy;     // per-bubble energies
+    RunSync *run;       // resident run: reductions and grid barrier
 };
 
 // ------------------------------------------------------------- helpers
@@ -609,6 +624,210 @@ __device__ void finish_attempt(Ctrl *c, const DevConst &k, double fErr, double f
     }
 }
 
+// ---------------------------------------------------------- resident runs
+// Small foams run their attempts inside one cooperative kernel (k_run in
+// step.cu, k_run_mx in step_mixed.cu): the three attempt bodies in a loop with
+// a grid barrier after each, until a bubble has to be deleted, the neighbours
+// searched, or the steps are done. At N = 10^4 an attempt's arithmetic takes
+// about 2 us, its three launches (a wave of ~600-1200 blocks each, every one
+// with a fence and an atomic on the same counter) and the two condition nodes
+// 55 us. The control block, the constants and the row tables live in shared
+// memory, one identical copy per block: every block folds all partials in the
+// same order after the barrier and takes the same decisions, so no second
+// barrier publishes them; block 0 writes the control block back at the end.
+//
+// The launch is cooperative (all blocks resident), so every arrival comes;
+// still each wait is bounded, and a block that gives up tells the others.
+struct RunCtx {
+    RunSync *g;
+    RunAcc *acc;     // of this attempt
+    unsigned phase;  // arrivals that complete the next barrier
+    unsigned vg;
+    int *failed;     // shared
+};
+constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: seconds in all
+constexpr int kRunMaxAttempts = 1 << 15;   // per launch (bounds the arrival counter)
+constexpr unsigned kRunGaveUp = 1u << 28;  // added to the arrivals by a block that gave up
+
+__device__ __forceinline__ void run_barrier(RunCtx *rx) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        rx->phase += rx->vg;
+        __threadfence();  // this block's writes (ordered before by the barrier above)
+        atomicAdd(&rx->g->arrive, 1u);
+        unsigned v;
+        int it = 0, past;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];"
+                         : "=r"(v) : "l"(&rx->g->arrive) : "memory");
+            past = (int)(v - rx->phase);
+        } while (past < 0 && ++it < kRunPolls);
+        if (past < 0) atomicAdd(&rx->g->arrive, kRunGaveUp);  // releases every other wait
+        if (past < 0 || past >= (int)(kRunGaveUp / 2)) *rx->failed = 1;
+    }
+    __syncthreads();
+}
+
+// First item of this thread of block vb of vg (stride vg * blockDim.x). A
+// resident run deals the warps out over the blocks first, so that a small
+// foam's FP64 work spreads over the SMs (2 FP64 lanes per SM and cycle).
+template <bool RES>
+__device__ __forceinline__ int first_item(int vb, int vg) {
+    return RES ? (int)((((threadIdx.x >> 5) * vg + vb) << 5) + (threadIdx.x & 31))
+               : (int)(vb * blockDim.x + threadIdx.x);
+}
+
+// The block's sums (FP64), maxima (bit patterns of doubles >= 0) and counts
+// into the run's global accumulators: warp by warp, across the warps through
+// shared memory, then one reduction each. Read after the next run_barrier.
+// (Partials per block folded by every block after the barrier, in a fixed
+// order, took 1900-3900 cycles of latency there against ~700 for reading the
+// result; the forces' reductions leave the order free already.)
+struct RunRed {
+    double s[5][kBlock / 32];
+    long long m[3][kBlock / 32];
+    int c[2][kBlock / 32];
+};
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+// Maximum over the warp of bit patterns >= 0: the high words' maximum, then
+// the low words of the lanes that hold it (negative patterns lose against 0).
+__device__ __forceinline__ long long warp_max_bits(long long v) {
+    v = max(v, 0LL);
+    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return (long long)(((unsigned long long)mh << 32) | ml);
+}
+template <int NS, int NM, int NC>
+__device__ __forceinline__ void run_reduce(const double *s, const long long *m, const int *c,
+                                           double *gs, long long *gm, int *gc, RunRed *sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double ws[NS];
+    long long wm[NM > 0 ? NM : 1];
+    int wc[NC > 0 ? NC : 1];
+#pragma unroll
+    for (int q = 0; q < NS; q++) ws[q] = warp_sum(s[q]);
+#pragma unroll
+    for (int q = 0; q < NM; q++) wm[q] = warp_max_bits(m[q]);
+#pragma unroll
+    for (int q = 0; q < NC; q++) wc[q] = __reduce_add_sync(0xffffffffu, c[q]);
+    __syncthreads();
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < NS; q++) sm->s[q][warp] = ws[q];
+#pragma unroll
+        for (int q = 0; q < NM; q++) sm->m[q][warp] = wm[q];
+#pragma unroll
+        for (int q = 0; q < NC; q++) sm->c[q][warp] = wc[q];
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t < NS) {
+        double v[kBlock / 32];
+#pragma unroll
+        for (int w = 0; w < kBlock / 32; w++) v[w] = w < nw ? sm->s[t][w] : 0.0;
+        if (nw > 4)
+#pragma unroll
+            for (int w = 0; w < 4; w++) v[w] += v[w + 4];
+        const double r = (v[0] + v[1]) + (v[2] + v[3]);
+        if (r != 0.0) atomicAdd(gs + t, r);
+    } else if (t < NS + NM) {
+        long long r = 0;
+        for (int w = 0; w < nw; w++) r = max(r, sm->m[t - NS][w]);
+        if (r) atomicMax(gm + (t - NS), r);
+    } else if (t < NS + NM + NC) {
+        int r = 0;
+        for (int w = 0; w < nw; w++) r += sm->c[t - NS - NM][w];
+        if (r) atomicAdd(gc + (t - NS - NM), r);
+    }
+}
+
+// The shared-memory copies of a resident block and the way in and out.
+struct RunShared {
+    Ctrl c;
+    DevConst k;
+    double *ds[ND_ROLES];
+    int *is[NI_ROLES];
+    int *ps[NP_ROLES];
+    int failed;
+};
+
+template <typename T>
+__device__ __forceinline__ void run_copy(T *dst, const T *src) {
+    static_assert(sizeof(T) % 4 == 0, "copied word by word");
+    for (int w = threadIdx.x; w < (int)(sizeof(T) / 4); w += blockDim.x)
+        reinterpret_cast<int *>(dst)[w] = __ldcg(reinterpret_cast<const int *>(src) + w);
+}
+
+__device__ __forceinline__ void run_enter(RunShared *s, Bufs &b, long long n_steps) {
+    run_copy(&s->c, b.ctrl);
+    run_copy(&s->k, b.k);
+    if (threadIdx.x < ND_ROLES) s->ds[threadIdx.x] = b.ds[threadIdx.x];
+    if (threadIdx.x < NI_ROLES) s->is[threadIdx.x] = b.is[threadIdx.x];
+    if (threadIdx.x < NP_ROLES) s->ps[threadIdx.x] = b.ps[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s->failed = 0;
+        s->c.graph_mode = 0;
+        if (n_steps >= 0) s->c.steps_target = s->c.steps + n_steps;
+    }
+    __syncthreads();
+    b.ctrl = &s->c;
+    b.k = &s->k;
+    b.ds = s->ds;
+    b.is = s->is;
+    b.ps = s->ps;
+}
+
+// Whether the next attempt runs in this launch (uniform over all blocks).
+__device__ __forceinline__ bool run_more(const RunShared *s, int attempts) {
+    const Ctrl &c = s->c;
+    if (s->failed || c.status != CB_OK || attempts >= kRunMaxAttempts) return false;
+    if (c.too_large) return true;
+    return !c.need_delete && !c.need_search && c.steps < c.steps_target && !c.stop_hit;
+}
+
+// Attempt `attempt` uses the accumulators of its parity. The other ones are
+// free once every block has passed the first barrier of this attempt (each
+// has then read the last attempt's results): cleared by block 0 between its
+// last two barriers.
+__device__ __forceinline__ void run_begin(RunCtx *rx, int attempt) {
+    rx->acc = &rx->g->acc[attempt & 1];
+}
+__device__ __forceinline__ void run_clear_other(RunCtx *rx, int vb) {
+    if (vb != 0) return;
+    int *o = reinterpret_cast<int *>(rx->acc == &rx->g->acc[0] ? &rx->g->acc[1] : &rx->g->acc[0]);
+    if (threadIdx.x < sizeof(RunAcc) / 4) o[threadIdx.x] = 0;
+}
+
+// Block 0 writes the control block to `ctrl` and, if given, to the host's
+// mirror; the last block out clears the accumulators and the barrier.
+__device__ __forceinline__ void run_exit(RunShared *s, Ctrl *ctrl, Ctrl *mirror, RunCtx *rx,
+                                         int vb) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0 && s->failed) s->c.status = CB_ERR_CUDA;
+    __syncthreads();
+    if (vb == 0)
+        for (int w = threadIdx.x; w < (int)(sizeof(Ctrl) / 4); w += blockDim.x) {
+            const int v = reinterpret_cast<const int *>(&s->c)[w];
+            reinterpret_cast<int *>(ctrl)[w] = v;
+            if (mirror) reinterpret_cast<int *>(mirror)[w] = v;
+        }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&rx->g->exits, 1u) == rx->vg - 1;
+    }
+    __syncthreads();
+    if (last)
+        for (int w = threadIdx.x; w < (int)(sizeof(RunSync) / 4); w += blockDim.x)
+            reinterpret_cast<int *>(rx->g)[w] = 0;
+}
+
 // ------------------------------------------------------ kernel launchers
 struct Launch {
     int grid;         // upper bound of the blocks of a grid-stride kernel
@@ -732,13 +951,40 @@ inline int wave_grid(K kernel, const Launch &l, int want = 0) {
     return g < l.grid ? g : l.grid;
 }
 
+// Launch of a resident run: `steps` accepted steps from the control block's
+// count on `grid` blocks of `block` threads; the control block is also
+// written to `mirror` (pinned host memory).
+struct RunLaunch {
+    int grid, block;
+    cudaStream_t stream;
+    long long steps;
+    Ctrl *mirror;
+    long long *launches;
+};
+template <typename K>
+inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)r.grid);
+    cfg.blockDim = dim3((unsigned)r.block);
+    cfg.stream = r.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, b, r.mirror, r.steps);
+    *r.launches += 1;
+}
+
 // step.cu
+void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode, bool ff);
 void launch_predict(const Launch &l, const Bufs &b, int dim);
 void launch_pairs(const Launch &l, const Bufs &b, int dim, int mode,
                   bool ff);  // mode: gas 1 | flow 2; ff: float-float kernel
 void launch_correct(const Launch &l, const Bufs &b, int dim);
 void launch_boot(const Launch &l, const Bufs &b, int dim, int phase);
 // step_mixed.cu (mixed form)
+void launch_run_mx(const RunLaunch &r, const Bufs &b, int dim, int mode, bool walls);
 void launch_predict_mx(const Launch &l, const Bufs &b, int dim);
 void launch_pairs_mx(const Launch &l, const Bufs &b, int dim, int mode);
 void launch_correct_mx(const Launch &l, const Bufs &b, int dim, int mode, bool walls);

@@ -186,6 +186,72 @@ int run_search(cb_context *c) {
     return c->check_launch();
 }
 
+// Contexts of up to this many bubbles run their attempts inside one
+// cooperative kernel (resident run, common.cuh); larger ones a launch per
+// phase. us per attempt on one GB300 (searches included), launches per phase
+// -> resident run:
+//   2D FP64   N = 10^3 52 -> 20, 10^4 52 -> 20, 2 10^5 97 -> 65, 5 10^5 162 -> 133
+//   2D mixed  N = 10^4 34 -> 15, 2 10^5 45 -> 35, 5 10^5 68 -> 64, 10^6 105 -> 114
+//   3D FP64   N = 4 10^3 53 -> 19, 3 10^4 59 -> 30, 3 10^5 145 -> 124,
+//             5 10^5 203 -> 195, 10^6 351 -> 359
+//   3D mixed  N = 4 10^3 34 -> 14, 3 10^5 67 -> 59, 5 10^5 95 -> 91, 10^6 150 -> 166
+// (two blocks per SM, the registers of the largest phase, against the four
+// blocks of the pair kernels: past the latency-bound sizes that costs more
+// than the launches).
+constexpr int kRunCapacity2 = 600000, kRunCapacity3 = 400000;
+
+bool resident(const cb_context *c) {
+    return c->coop && c->hk.cap <= (c->hk.dim == 3 ? kRunCapacity3 : kRunCapacity2);
+}
+
+// Blocks and threads of a resident run: a warp per 32 items (the mixed form's
+// threads take two pairs) over as many SMs as that fills, at most two blocks
+// per SM; blocks of four warps while they reach, so that the warps of a small
+// foam spread over the SMs (N = 10^4, 2D: 20.1 us per attempt with four, 22.3
+// with two, 20.5 with eight).
+RunLaunch run_launch(cb_context *c, int64_t n_steps) {
+    const double per = c->hk.dim == 3 ? 4.7 : 2.4;  // listed pairs per bubble
+    const int items = (int)(per * c->hk.cap) / (c->hk.mixed ? 2 : 1);
+    const int warps = std::max(1, (items + 31) / 32);
+    RunLaunch r;
+    r.block = warps <= 4 * 2 * c->sms ? 128 : kBlock;
+    r.grid = std::min(2 * c->sms, (32 * warps + r.block - 1) / r.block);
+    r.stream = c->stream;
+    r.steps = n_steps;
+    r.mirror = c->hctrl;
+    r.launches = &c->launches;
+    return r;
+}
+
+// integrate() of a small foam: resident runs of attempts, each until a
+// deletion, a search or the end; the control block comes back with the run.
+// Expects hctrl to hold the device's control block.
+int integrate_resident(cb_context *c, int64_t n_steps) {
+    const long long target = c->hctrl->steps + n_steps;
+    for (;;) {
+        const RunLaunch r = run_launch(c, target - c->hctrl->steps);
+        if (c->hk.mixed)
+            launch_run_mx(r, c->bufs, c->hk.dim, c->mode(), c->hk.any_wall != 0);
+        else
+            launch_run(r, c->bufs, c->hk.dim, c->mode(), c->hk.ffpair != 0);
+        int rc = c->check_launch();
+        if (rc) return rc;
+        CB_CUDA(cudaStreamSynchronize(c->stream));
+        const Ctrl &h = *c->hctrl;
+        if (h.status != CB_OK) return fail(h.status, status_text(h.status));
+        if (h.too_large) continue;
+        const bool del = h.need_delete, search = h.need_search;
+        if (del) {
+            NvtxRange nv("Removal");
+            launch_remove(c->launch, c->bufs, c->hk.dim);
+            if ((rc = c->check_launch())) return rc;
+        }
+        if (search && (rc = run_search(c))) return rc;
+        if ((del || search) && (rc = sync_status(c))) return rc;
+        if (h.stop_hit || h.steps >= target) return CB_OK;
+    }
+}
+
 // Eager integrate(): one control-block read per attempt.
 int integrate_eager(cb_context *c, int64_t n_steps) {
     for (int64_t s = 0; s < n_steps; s++) {
@@ -418,6 +484,7 @@ int cbg::create_context(const cb_config *cfg, cb_context **out, bool graph) {
     };
     if (cudaGetDevice(&c->dev) != cudaSuccess) return bail(fail(CB_ERR_CUDA, "cudaGetDevice"));
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev);
+    cudaDeviceGetAttribute(&c->coop, cudaDevAttrCooperativeLaunch, c->dev);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(CB_ERR_CUDA, "cudaStreamCreate"));
     cudaEventCreate(&c->ev0);
@@ -471,6 +538,7 @@ int cbg::create_context(const cb_config *cfg, cb_context **out, bool graph) {
     if ((rc = c->alloc(&b.keep, pcap + 1))) return bail(rc);
     if ((rc = c->alloc(&b.keepScan, pcap + 1))) return bail(rc);
     if ((rc = c->alloc(&b.stash, cap * (size_t)kStash(c->hk.dim)))) return bail(rc);
+    if ((rc = c->alloc(&b.run, 1))) return bail(rc);
     if ((rc = c->alloc(&b.energy, std::max<size_t>(cap, 8)))) return bail(rc);
     if (cudaMemcpyAsync(c->d_dslots, c->dslot, sizeof(c->dslot), cudaMemcpyHostToDevice,
                         c->stream) != cudaSuccess ||
@@ -509,7 +577,7 @@ int cbg::create_context(const cb_config *cfg, cb_context **out, bool graph) {
     }
     if ((rc = c->upload_const())) return bail(rc);
     if ((rc = c->push())) return bail(rc);
-    if (graph && cfg->use_graph && (rc = build_graph(c))) return bail(rc);
+    if (graph && cfg->use_graph && !resident(c) && (rc = build_graph(c))) return bail(rc);
     *out = c;
     return CB_OK;
 }
@@ -895,6 +963,7 @@ static int integrate_impl(cb_context *c, int64_t n_steps, bool fresh) {
     }
     if (c->hctrl->status != CB_OK) return fail(c->hctrl->status, status_text(c->hctrl->status));
     if (n_steps == 0) return CB_OK;
+    if (resident(c)) return integrate_resident(c, n_steps);
     return c->cfg.use_graph ? integrate_graph(c, n_steps) : integrate_eager(c, n_steps);
 }
 
@@ -905,7 +974,7 @@ int cb_integrate(cb_context *c, int64_t n_steps, cb_report *r) {
     CB_ENTER(c);
     c->mirror_call = ~0ull;
     const int rc = integrate_impl(c, n_steps, fresh);
-    if (rc == CB_OK && c->cfg.use_graph) c->mirror_call = cbg::g_calls.load(std::memory_order_relaxed);
+    if (rc == CB_OK && (c->cfg.use_graph || resident(c))) c->mirror_call = cbg::g_calls.load(std::memory_order_relaxed);
     // integrate_impl leaves hctrl as read from the device after its last
     // launch (or before, when it returned early)
     if (r) fill_report(c, r);

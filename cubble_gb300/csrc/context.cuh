@@ -40,7 +40,7 @@ using cbg::Launch;
 
 struct cb_context {
     cb_config cfg{};
-    int dev = 0, sms = 0;
+    int dev = 0, sms = 0, coop = 0;
     cudaStream_t stream = nullptr;
     DevConst hk{};
     DevConst *dk = nullptr;

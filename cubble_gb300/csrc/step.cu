@@ -50,8 +50,10 @@ __device__ __forceinline__ void add_d(double *p, ff v) {
 }
 
 // ---------------------------------------------------------------- predict
-template <int DIM>
-__device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, const int vg) {
+// RES: as a phase of a resident run (common.cuh)
+template <int DIM, bool RES = false>
+__device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, const int vg,
+                                               RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     __shared__ double smem[32];
     const Ctrl *c = b.ctrl;
     const int n = c->n;
@@ -65,7 +67,7 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
                  *O3 = drow(b, c, RVO3);
     double sA = 0.0, sAr = 0.0;
     int na = 0;
-    for (int i = vb * blockDim.x + threadIdx.x; i < n; i += vg * blockDim.x) {
+    for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
         // p + 0.5 ts (3 v - vo), src/kernels.cu:48-50
         const double xp = fma(h, fma(3.0, V0[i], -O0[i]), X[i]);
         const double yp = fma(h, fma(3.0, V1[i], -O1[i]), Y[i]);
@@ -101,6 +103,12 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
     }
     if (DIM == 2) sAr = (double)na;
     constexpr double kArea = DIM == 3 ? 4.0 * kPi : 2.0 * kPi;
+    if (RES) {  // the sums are read after the pair phase
+        const double v[2] = {sA, sAr};
+        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->sum, nullptr, nullptr, rsm);
+        run_barrier(rx);
+        return;
+    }
     const double tA = kArea * block_reduce(sA, OpSum(), smem);
     const double tAr = kArea * block_reduce(sAr, OpSum(), smem);
     if (threadIdx.x == 0) {
@@ -160,16 +168,37 @@ constexpr int kQueue = 64;  // per-warp queue of overlapping pairs
 // is pi (chord radius)^2), 2 in 2D (an overlap length is 2 (half chord)).
 __host__ __device__ constexpr double ov_unit(int dim) { return dim == 3 ? kPi : 2.0; }
 
-// The last block of a pair kernel: the attempt's total overlap area and
-// overlap area per radius (src/kernels.cu:264-267; each pair adds 2 A_overlap)
-// from the blocks' partial sums, which are in units of ov_unit, and the
+// The end of a pair kernel: the attempt's total overlap area and overlap area
+// per radius (src/kernels.cu:264-267; each pair adds 2 A_overlap) from the
+// threads' sums sAo and sAor, which are in units of ov_unit, and the
 // mean-field factors of every bubble (src/kernels.cu:399-404).
-template <int DIM>
-__device__ __forceinline__ void pairs_fold(const Bufs &b, const int vb, const int vg,
-                                           double *smem) {
-    if (!last_block(&b.ctrl->done[DC_PAIRS], vg)) return;
-    const double fAo = fold_partials(b.part + 2 * vg, vg, false, smem);
-    const double fAor = fold_partials(b.part + 3 * vg, vg, false, smem);
+template <int DIM, bool RES>
+__device__ __forceinline__ void pairs_fold(const Bufs &b, const int vb, const int vg, double sAo,
+                                           double sAor, double *smem, RunCtx *rx, RunRed *rsm) {
+    double fAo, fAor;
+    if (RES) {
+        const double v[2] = {sAo, sAor};
+        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->osum, nullptr, nullptr, rsm);
+        run_barrier(rx);
+        run_clear_other(rx, vb);
+        if (threadIdx.x == 0) {
+            constexpr double kArea = DIM == 3 ? 4.0 * kPi : 2.0 * kPi;
+            fAo = __ldcg(&rx->acc->osum[0]);
+            fAor = __ldcg(&rx->acc->osum[1]);
+            b.ctrl->sumA = kArea * __ldcg(&rx->acc->sum[0]);
+            b.ctrl->sumAr = kArea * __ldcg(&rx->acc->sum[1]);
+        }
+    } else {
+        const double tAo = block_reduce(sAo, OpSum(), smem);
+        const double tAor = block_reduce(sAor, OpSum(), smem);
+        if (threadIdx.x == 0) {
+            b.part[2 * vg + vb] = tAo;
+            b.part[3 * vg + vb] = tAor;
+        }
+        if (!last_block(&b.ctrl->done[DC_PAIRS], vg)) return;
+        fAo = fold_partials(b.part + 2 * vg, vg, false, smem);
+        fAor = fold_partials(b.part + 3 * vg, vg, false, smem);
+    }
     if (threadIdx.x == 0) {
         Ctrl *cc = b.ctrl;
         cc->sumAo = (2.0 * ov_unit(DIM)) * fAo;
@@ -192,8 +221,9 @@ static __device__ __noinline__ bool overlap_exact(double dx, double dy, double d
     return nonneg_bits(fma(radii, radii, -m));
 }
 
-template <int DIM, bool GAS, bool FLOW>
-__device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool GAS, bool FLOW, bool RES = false>
+__device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const int vg,
+                                             RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     constexpr int kW = kBlock / 32;
     __shared__ double smem[32];
     // queue slots: dx, dy, (3D: dz), r1, r2
@@ -285,7 +315,8 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
 
     int cnt = 0;  // queued pairs of this warp (uniform over its lanes)
     const int nch = (np + 31) >> 5;
-    for (int ch = vb * kW + w; ch < nch; ch += vg * kW) {
+    const int wb = RES ? blockDim.x >> 5 : kW;  // warps of this block
+    for (int ch = RES ? w * vg + vb : vb * kW + w; ch < nch; ch += vg * wb) {
         const int p = (ch << 5) + lane;
         bool over = false;
         int i = 0, j = 0;
@@ -354,13 +385,7 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     }
     if (lane < cnt) process(lane);
 
-    const double tAo = block_reduce(sAo, OpSum(), smem);
-    const double tAor = block_reduce(sAor, OpSum(), smem);
-    if (threadIdx.x == 0) {
-        b.part[2 * vg + vb] = tAo;
-        b.part[3 * vg + vb] = tAor;
-    }
-    pairs_fold<DIM>(b, vb, vg, smem);
+    pairs_fold<DIM, RES>(b, vb, vg, sAo, sAor, smem, rx, rsm);
 }
 CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs, (<DIM, GAS, FLOW>), __launch_bounds__(kBlock))
 
@@ -382,12 +407,14 @@ CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs, (<DIM, GAS, F
 // the i-side sums stay in float-float registers and go out once per row; the
 // j-side contributions go out per pair. Both are rounded to double on the
 // integer pipe and added to the FP64 accumulator rows with FP64 atomics.
-constexpr int kRun = 4;
 constexpr float kAmb = 0x1p-38f;
 
 
-template <int DIM, bool GAS, bool FLOW>
-__device__ __forceinline__ void k_pairs_ff_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool GAS, bool FLOW, bool RES = false>
+__device__ __forceinline__ void k_pairs_ff_body(const Bufs &b, const int vb, const int vg,
+                                                RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
+    // a resident run has pairs for a fraction of the resident threads only
+    constexpr int kRun = RES ? 1 : 4;
     __shared__ double smem[32];
     const Ctrl *c = b.ctrl;
     const DevConst &k = *b.k;
@@ -402,7 +429,7 @@ __device__ __forceinline__ void k_pairs_ff_body(const Bufs &b, const int vb, con
     const double Lx = k.iv[0], Ly = k.iv[1], Lz = k.iv[2];
     ff sAo = {0.f, 0.f}, sAor = {0.f, 0.f};
     const int nrun = (np + kRun - 1) / kRun;
-    for (int g = vb * blockDim.x + threadIdx.x; g < nrun; g += vg * blockDim.x) {
+    for (int g = first_item<RES>(vb, vg); g < nrun; g += vg * blockDim.x) {
         const int p0 = g * kRun;
         int cur = -1;
         double4_32a a;
@@ -533,13 +560,7 @@ __device__ __forceinline__ void k_pairs_ff_body(const Bufs &b, const int vb, con
         }
         if (hit) flush(cur);
     }
-    const double tAo = block_reduce(ff_to_double(sAo), OpSum(), smem);
-    const double tAor = block_reduce(ff_to_double(sAor), OpSum(), smem);
-    if (threadIdx.x == 0) {
-        b.part[2 * vg + vb] = tAo;
-        b.part[3 * vg + vb] = tAor;
-    }
-    pairs_fold<DIM>(b, vb, vg, smem);
+    pairs_fold<DIM, RES>(b, vb, vg, ff_to_double(sAo), ff_to_double(sAor), smem, rx, rsm);
 }
 CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs_ff, (<DIM, GAS, FLOW>), __launch_bounds__(kBlock, 3))
 
@@ -636,8 +657,9 @@ __device__ __forceinline__ double norm_ffd(double a, double b, double c) {
     return ff_to_double(ff_sqrt(s));
 }
 
-template <int DIM>
-__device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool RES = false>
+__device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, const int vg,
+                                               RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     __shared__ double smem[32];
     __shared__ int ismem[32];
     Ctrl *c = b.ctrl;
@@ -670,7 +692,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     long long merr = 0, mrad = 0, mexp = 0;
     double vol = 0.0;
     int ndel = 0, bad = 0;
-    for (int i = vb * blockDim.x + threadIdx.x; i < n; i += vg * blockDim.x) {
+    for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
         double *acc = b.acc + (size_t)i * kAcc;
         const double4_32a a0 = reinterpret_cast<const double4_32a *>(acc)[0];
         double4_32a a1;
@@ -759,6 +781,22 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         reinterpret_cast<double4_32a *>(acc)[0] = zero;
         if (gas || flow) reinterpret_cast<double4_32a *>(acc)[1] = zero;
     }
+    if (RES) {
+        const long long m[3] = {merr, mrad, mexp};
+        const int cn[2] = {ndel, bad};
+        run_reduce<1, 3, 2>(&vol, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
+        run_barrier(rx);
+        if (threadIdx.x == 0) {
+            const RunAcc *g = rx->acc;
+            const double e = __longlong_as_double(__ldcg(&g->cmax[0])),
+                         r = __longlong_as_double(__ldcg(&g->cmax[1])),
+                         x = __longlong_as_double(__ldcg(&g->cmax[2])), v = __ldcg(&g->csum[0]);
+            const int nd = __ldcg(&g->cnt[0]), nb = __ldcg(&g->cnt[1]);
+            finish_attempt<DIM>(c, k, e, r, x, v, (double)nd, (double)nb);
+        }
+        __syncthreads();
+        return;
+    }
     long long *lsm = reinterpret_cast<long long *>(smem);
     const double tErr = __longlong_as_double(block_max_bits(merr, lsm));
     const double tRad = __longlong_as_double(block_max_bits(mrad, lsm));
@@ -787,6 +825,33 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
 }
 CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBlock))
 
+
+// ----------------------------------------------------------- resident run
+// Attempts of a small foam inside one cooperative launch (see common.cuh).
+// Measured against the launch per phase, one GB300: see kRunCapacity
+// (context.cu).
+template <int DIM, bool GAS, bool FLOW, bool FF>
+__global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, Ctrl *mirror, long long n_steps) {
+    __shared__ RunShared rs;
+    __shared__ RunRed rsm;
+    const int vb = blockIdx.x, vg = gridDim.x;
+    Ctrl *ctrl = b.ctrl;
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed};
+    run_enter(&rs, b, n_steps);
+    int attempts = 0;
+    do {
+        run_begin(&rx, attempts);
+        k_predict_body<DIM, true>(b, vb, vg, &rx, &rsm);
+        __syncthreads();
+        if (FF)
+            k_pairs_ff_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
+        else
+            k_pairs_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
+        __syncthreads();
+        k_correct_body<DIM, true>(b, vb, vg, &rx, &rsm);
+    } while (run_more(&rs, ++attempts));
+    run_exit(&rs, ctrl, mirror, &rx, vb);
+}
 
 // --------------------------------------------------------------- bootstrap
 // phase 0: pred := (x, r), vo := 0, path := 0
@@ -945,6 +1010,29 @@ void launch_correct(const Launch &l, const Bufs &b, int dim) {
         CB_LAUNCH(l, k_correct, (<3>), wave_grid(k_correct<3>, l, l.step_bps), b);
     else
         CB_LAUNCH(l, k_correct, (<2>), wave_grid(k_correct<2>, l, l.step_bps), b);
+}
+
+void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode, bool ff) {
+    const bool gas = mode & 1, flow = mode & 2;
+#define CB_RUN(D, G, F)                                  \
+    do {                                                 \
+        if (ff)                                          \
+            launch_coop(k_run<D, G, F, true>, r, b);     \
+        else                                             \
+            launch_coop(k_run<D, G, F, false>, r, b);    \
+    } while (0)
+    if (dim == 3) {
+        if (gas && flow) CB_RUN(3, true, true);
+        else if (gas) CB_RUN(3, true, false);
+        else if (flow) CB_RUN(3, false, true);
+        else CB_RUN(3, false, false);
+    } else {
+        if (gas && flow) CB_RUN(2, true, true);
+        else if (gas) CB_RUN(2, true, false);
+        else if (flow) CB_RUN(2, false, true);
+        else CB_RUN(2, false, false);
+    }
+#undef CB_RUN
 }
 
 void launch_boot(const Launch &l, const Bufs &b, int dim, int phase) {

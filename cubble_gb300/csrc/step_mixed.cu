@@ -178,11 +178,20 @@ __device__ __forceinline__ const double *pred_base(const Bufs &b, const Ctrl *c,
     return s == 0 ? b.pred : b.predc + (size_t)(s - 1) * 4 * cap;
 }
 
+// A state row's element: through the read-only path, or, in a resident run
+// (which writes the rows it reads later), an ordinary load.
+template <bool RES, typename T>
+__device__ __forceinline__ T ld_row(const T *p) {
+    return RES ? *p : __ldg(p);
+}
+
 // ---------------------------------------------------------------- predict
 // Skipped (every block returns at once) when the last correct already
 // wrote this attempt's prediction and its area sums.
-template <int DIM>
-__device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, const int vg) {
+// RES: as a phase of a resident run (common.cuh).
+template <int DIM, bool RES = false>
+__device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, const int vg,
+                                                  RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     __shared__ double smem[32];
     const Ctrl *c = b.ctrl;
     if (c->pred_ready) return;
@@ -199,7 +208,7 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
     // two bubbles per iteration, all loads of both issued before any store
     // (twice the loads in flight of a one-bubble loop)
     const int stride = vg * blockDim.x;
-    for (int i0 = vb * blockDim.x + threadIdx.x; i0 < n; i0 += 2 * stride) {
+    for (int i0 = first_item<RES>(vb, vg); i0 < n; i0 += 2 * stride) {
         const int i1 = i0 + stride < n ? i0 + stride : i0;
         const int ii[2] = {i0, i1};
         double x[2], y[2], z[2], r[2];
@@ -207,15 +216,15 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int i = ii[u];
-            x[u] = __ldg(X + i);
-            y[u] = __ldg(Y + i);
-            z[u] = DIM == 3 ? __ldg(Z + i) : 0.0;
-            r[u] = __ldg(R + i);
+            x[u] = ld_row<RES>(X + i);
+            y[u] = ld_row<RES>(Y + i);
+            z[u] = DIM == 3 ? ld_row<RES>(Z + i) : 0.0;
+            r[u] = ld_row<RES>(R + i);
             // AB2 direction 3 v - vo
-            d[0][u] = fmaf(3.f, __ldg(V0 + i), -__ldg(O0 + i));
-            d[1][u] = fmaf(3.f, __ldg(V1 + i), -__ldg(O1 + i));
-            d[2][u] = DIM == 3 ? fmaf(3.f, __ldg(V2 + i), -__ldg(O2 + i)) : 0.f;
-            d[3][u] = gas ? fmaf(3.f, __ldg(V3 + i), -__ldg(O3 + i)) : 0.f;
+            d[0][u] = fmaf(3.f, ld_row<RES>(V0 + i), -ld_row<RES>(O0 + i));
+            d[1][u] = fmaf(3.f, ld_row<RES>(V1 + i), -ld_row<RES>(O1 + i));
+            d[2][u] = DIM == 3 ? fmaf(3.f, ld_row<RES>(V2 + i), -ld_row<RES>(O2 + i)) : 0.f;
+            d[3][u] = gas ? fmaf(3.f, ld_row<RES>(V3 + i), -ld_row<RES>(O3 + i)) : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -234,6 +243,12 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
                 sAr += apr;
             }
         }
+    }
+    if (RES) {  // the sums are read after the pair phase
+        const double v[2] = {(double)sA, (double)sAr};
+        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->sum, nullptr, nullptr, rsm);
+        run_barrier(rx);
+        return;
     }
     const double tA = block_sum_f(sA, smem);
     const double tAr = block_sum_f(sAr, smem);
@@ -373,7 +388,7 @@ __device__ __forceinline__ bool contained_exact(long long ex, long long ey, long
 
 // Last block of the pair kernel: the listed pairs decided again (see above).
 // Returns this thread's changes of the summed overlap area and of the summed
-// area over radius.
+// area over radius; without AV only those.
 template <int DIM>
 __device__ __forceinline__ float2 recheck_containment(const int2 *RC, double *const *ds,
                                                       const Ctrl *c, const DevConst *kp,
@@ -398,7 +413,8 @@ __device__ __forceinline__ float2 recheck_containment(const int2 *RC, double *co
                         overlap_area<DIM>(r1, r2, r1sq, r2sq, pp, m, rs, fast);
         const float inv1 = __fdividef(1.f, r1), inv2 = __fdividef(1.f, r2);
         const float dg = d * (inv2 - inv1);
-        if (DIM == 3) {
+        if (!AV) {
+        } else if (DIM == 3) {
             atomicAdd(AO + pr.x, d);
             atomicAdd(AO + pr.y, d);
             red_add4(AV + pr.x, 0.f, 0.f, 0.f, dg);
@@ -441,8 +457,9 @@ __device__ __forceinline__ void load_run(const int *P, int p0, int (&v)[RUN]) {
 // In 2D the overlap sum rides in the third lane of the velocity float4. RUN
 // (pairs per thread, 32 RUN per warp) is a tuning knob: 4 by default, 2 or 8
 // for the gas-exchange kernels without flow (cb_tuning.pair_run).
-template <int DIM, bool GAS, bool FLOW, int RUN>
-__device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool GAS, bool FLOW, int RUN, bool RES = false>
+__device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, const int vg,
+                                                RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     __shared__ double smem[32];
     const Ctrl *c = b.ctrl;
     const DevConst &k = *b.k;
@@ -457,9 +474,13 @@ __device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, con
     const float f0 = k.f0_f;
     const FixBox fb = fix_box(k, DIM);
     const double *PB = pred_base(b, c, cap);
+    // a new value for the compiler in every attempt: the record loads
+    // (ld_pred) are not volatile and must not move across a resident run's
+    // barriers
+    if (RES) asm volatile("" : "+l"(PB));
     float sAo = 0.f, sAor = 0.f;
     const int nrun = (np + RUN - 1) / RUN;
-    for (int g = vb * blockDim.x + threadIdx.x; g < nrun; g += vg * blockDim.x) {
+    for (int g = first_item<RES>(vb, vg); g < nrun; g += vg * blockDim.x) {
         const int p0 = g * RUN;
         int I[RUN], J[RUN];
         if (p0 + RUN <= np) {
@@ -560,6 +581,37 @@ __device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, con
         }
         if (hit) flush();
     }
+    if (RES) {
+        const double v[2] = {(double)sAo, (double)sAor};
+        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->osum, nullptr, nullptr, rsm);
+        run_barrier(rx);
+        run_clear_other(rx, vb);
+        double fAo = __ldcg(&rx->acc->osum[0]), fAor = __ldcg(&rx->acc->osum[1]);
+        if (GAS) {
+            int2 *RC = recheck_list(AV, cap);
+            if (__ldcg(&RC[0].x)) {  // the same for every block; rare
+                // every block needs the changed sums; block 0 also changes the
+                // two bubbles' rows, which the next phase reads
+                const float2 d = recheck_containment<DIM>(RC, b.ds, c, b.k, PB, vb ? nullptr : AV, AO);
+                fAo += block_sum_f(d.x, smem);
+                fAor += block_sum_f(d.y, smem);
+                run_barrier(rx);
+                if (vb == 0 && threadIdx.x == 0) RC[0].x = 0;  // every block has read it
+            }
+        }
+        if (threadIdx.x == 0) {
+            Ctrl *cc = b.ctrl;
+            if (!cc->pred_ready) {  // the prediction of this attempt's predict phase
+                cc->sumA = __ldcg(&rx->acc->sum[0]);
+                cc->sumAr = __ldcg(&rx->acc->sum[1]);
+            }
+            cc->sumAo = 2.0 * fAo;
+            cc->sumAor = fAor;
+            cc->mfa = (cc->sumAr - cc->sumAor) / (cc->sumA - cc->sumAo);
+            cc->mfb = k.kappa * k.ain * (double)cc->n / cc->sumA;
+        }
+        return;
+    }
     const double tAo = block_sum_f(sAo, smem);
     const double tAor = block_sum_f(sAor, smem);
     if (threadIdx.x == 0) {
@@ -656,10 +708,11 @@ __device__ __forceinline__ CorrRed block_reduce_corr(CorrRed v, CorrRed *smem) {
 // Grid-stride over the bubbles (one wave of blocks). The maxima and counts go
 // to the control block with integer atomics (order-independent); only the
 // volume sum keeps per-block partials for its in-order FP64 fold.
-template <int DIM, bool GAS, bool FLOW, bool WALLS>
-__device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool GAS, bool FLOW, bool WALLS, bool RES = false>
+__device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, const int vg,
+                                                  RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     __shared__ double smem[32];
-    __shared__ CorrRed rsm[kBlock / 32];
+    __shared__ CorrRed corr[kBlock / 32];
     __shared__ unsigned long long tab[ND_ROLES];
     Ctrl *c = b.ctrl;
     const DevConst &k = *b.k;
@@ -691,7 +744,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     float mexp = 0.f;
     double vol = 0.0;
     int ndel = 0, bad = 0;
-    for (int i = vb * blockDim.x + threadIdx.x; i < n; i += vg * blockDim.x) {
+    for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
         const float4 a = AV[i];
         float vpx = a.x, vpy = a.y, vpz = DIM == 3 ? a.z : 0.f, vpr = a.w;
         const float ovl = GAS ? (DIM == 3 ? AO[i] : a.z) : 0.f;  // overlap area sum
@@ -862,9 +915,30 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     }
 #undef CB_D
 #undef CB_F
+    if (RES) {
+        const double sv[5] = {vol, (double)cA0, (double)cA1, (double)cAr0, (double)cAr1};
+        const long long m[3] = {merr, mrad, __double_as_longlong(double_from_float(mexp))};
+        const int cn[2] = {ndel, bad};
+        run_reduce<GAS ? 5 : 1, 3, 2>(sv, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
+        run_barrier(rx);
+        if (threadIdx.x == 0) {
+            const RunAcc *g = rx->acc;
+            const double e = __longlong_as_double(__ldcg(&g->cmax[0])),
+                         r = __longlong_as_double(__ldcg(&g->cmax[1])),
+                         x = __longlong_as_double(__ldcg(&g->cmax[2])), v = __ldcg(&g->csum[0]);
+            const int nd = __ldcg(&g->cnt[0]), nb = __ldcg(&g->cnt[1]);
+            c->cand_sumA[0] = __ldcg(&g->csum[1]);
+            c->cand_sumA[1] = __ldcg(&g->csum[2]);
+            c->cand_sumAr[0] = __ldcg(&g->csum[3]);
+            c->cand_sumAr[1] = __ldcg(&g->csum[4]);
+            finish_attempt<DIM>(c, k, e, r, x, v, (double)nd, (double)nb);
+        }
+        __syncthreads();
+        return;
+    }
     CorrRed v{merr, mrad, __double_as_longlong(double_from_float(mexp)), vol, ndel, bad,
               {cA0, cA1}, {cAr0, cAr1}};
-    v = block_reduce_corr(v, rsm);
+    v = block_reduce_corr(v, corr);
     if (threadIdx.x == 0) {
         if (GAS) {
             atomicAdd(&c->cand_sumA[0], (double)v.cA[0]);
@@ -893,6 +967,30 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
 }
 CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_mx, (<DIM, GAS, FLOW, WALLS>), __launch_bounds__(kBlock, 4))
 
+
+// ----------------------------------------------------------- resident run
+// Attempts of a small foam inside one cooperative launch (see common.cuh);
+// after an accepted attempt the next prediction is ready (two barriers then,
+// three otherwise).
+template <int DIM, bool GAS, bool FLOW, bool WALLS>
+__global__ void __launch_bounds__(kBlock, 2) k_run_mx(Bufs b, Ctrl *mirror, long long n_steps) {
+    __shared__ RunShared rs;
+    __shared__ RunRed rsm;
+    const int vb = blockIdx.x, vg = gridDim.x;
+    Ctrl *ctrl = b.ctrl;
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed};
+    run_enter(&rs, b, n_steps);
+    int attempts = 0;
+    do {
+        run_begin(&rx, attempts);
+        k_predict_mx_body<DIM, true>(b, vb, vg, &rx, &rsm);
+        __syncthreads();
+        k_pairs_mx_body<DIM, GAS, FLOW, 2, true>(b, vb, vg, &rx, &rsm);
+        __syncthreads();
+        k_correct_mx_body<DIM, GAS, FLOW, WALLS, true>(b, vb, vg, &rx, &rsm);
+    } while (run_more(&rs, ++attempts));
+    run_exit(&rs, ctrl, mirror, &rx, vb);
+}
 
 // --------------------------------------------------------------- bootstrap
 // phase 0: pred := fixed point of (x, r), vo := 0, path := 0
@@ -998,6 +1096,29 @@ void launch_correct_mx(const Launch &l, const Bufs &b, int dim, int mode, bool w
         else
             launch_correct_mx_t<2, false>(l, b, flow, walls);
     }
+}
+
+void launch_run_mx(const RunLaunch &r, const Bufs &b, int dim, int mode, bool walls) {
+    const bool gas = mode & 1, flow = mode & 2;
+#define CB_RUN(D, G, F)                                   \
+    do {                                                  \
+        if (walls)                                        \
+            launch_coop(k_run_mx<D, G, F, true>, r, b);   \
+        else                                              \
+            launch_coop(k_run_mx<D, G, F, false>, r, b);  \
+    } while (0)
+    if (dim == 3) {
+        if (gas && flow) CB_RUN(3, true, true);
+        else if (gas) CB_RUN(3, true, false);
+        else if (flow) CB_RUN(3, false, true);
+        else CB_RUN(3, false, false);
+    } else {
+        if (gas && flow) CB_RUN(2, true, true);
+        else if (gas) CB_RUN(2, true, false);
+        else if (flow) CB_RUN(2, false, true);
+        else CB_RUN(2, false, false);
+    }
+#undef CB_RUN
 }
 
 void launch_boot_mx(const Launch &l, const Bufs &b, int dim, int phase) {
