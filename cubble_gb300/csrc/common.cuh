@@ -644,6 +644,7 @@ struct RunCtx {
     unsigned phase;  // arrivals that complete the next barrier
     unsigned vg;
     int *failed;     // shared
+    int threads;     // of the correct kernel in a launch per phase (mixed form)
 };
 constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: seconds in all
 constexpr int kRunMaxAttempts = 1 << 15;   // per launch (bounds the arrival counter)
@@ -745,6 +746,11 @@ __device__ __forceinline__ void run_reduce(const double *s, const long long *m, 
         if (r) atomicAdd(gc + (t - NS - NM), r);
     }
 }
+
+// Batched run: block vb of the vg blocks of one foam.
+struct RunBlock {
+    int foam, vb, vg;
+};
 
 // The shared-memory copies of a resident block and the way in and out.
 struct RunShared {
@@ -952,14 +958,18 @@ inline int wave_grid(K kernel, const Launch &l, int want = 0) {
 }
 
 // Launch of a resident run: `steps` accepted steps from the control block's
-// count on `grid` blocks of `block` threads; the control block is also
-// written to `mirror` (pinned host memory).
+// count (< 0: to its steps_target) on `grid` blocks of `block` threads; the
+// control block is also written to `mirror` (pinned host memory) if given.
+// Batched: `foams` and `map` (device) say what every block works on.
 struct RunLaunch {
     int grid, block;
+    int threads;  // of the correct kernel in a launch per phase (mixed form)
     cudaStream_t stream;
     long long steps;
     Ctrl *mirror;
     long long *launches;
+    const Bufs *foams = nullptr;
+    const RunBlock *map = nullptr;
 };
 template <typename K>
 inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
@@ -972,7 +982,7 @@ inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, b, r.mirror, r.steps);
+    cudaLaunchKernelEx(&cfg, kernel, b, r.foams, r.map, r.mirror, r.steps, r.threads);
     *r.launches += 1;
 }
 

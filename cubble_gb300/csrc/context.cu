@@ -216,6 +216,7 @@ RunLaunch run_launch(cb_context *c, int64_t n_steps) {
     RunLaunch r;
     r.block = warps <= 4 * 2 * c->sms ? 128 : kBlock;
     r.grid = std::min(2 * c->sms, (32 * warps + r.block - 1) / r.block);
+    r.threads = 4 * c->sms * kBlock;
     r.stream = c->stream;
     r.steps = n_steps;
     r.mirror = c->hctrl;

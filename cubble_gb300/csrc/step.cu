@@ -831,12 +831,21 @@ CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBloc
 // Measured against the launch per phase, one GB300: see kRunCapacity
 // (context.cu).
 template <int DIM, bool GAS, bool FLOW, bool FF>
-__global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, Ctrl *mirror, long long n_steps) {
+__global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, const Bufs *foams,
+                                                    const RunBlock *map, Ctrl *mirror,
+                                                    long long n_steps, int threads) {
     __shared__ RunShared rs;
     __shared__ RunRed rsm;
-    const int vb = blockIdx.x, vg = gridDim.x;
+    int vb = blockIdx.x, vg = gridDim.x;
+    if (map) {  // batched: every foam its own blocks, barrier and loop
+        const RunBlock w = map[blockIdx.x];
+        b = foams[w.foam];
+        vb = w.vb;
+        vg = w.vg;
+        if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
+    }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
     do {

@@ -185,6 +185,33 @@ __device__ __forceinline__ T ld_row(const T *p) {
     return RES ? *p : __ldg(p);
 }
 
+// The sum of area over radius in 2D, 2 pi for every bubble, with the FP32
+// rounding of the kernels launched per phase: each of their `threads` sums
+// its bubbles' constants, and in the correct kernel (BLOCK) a block its eight
+// warps' sums. That rounding (up to 10^-7 of the sum) shifts every bubble's gas
+// flux alike and shows in the total volume at 10^-9 over 300 steps, so a
+// resident run uses the same value: a foam must not depend on the path that
+// runs it.
+template <bool BLOCK>
+__device__ __forceinline__ double area_over_radius_2d(int n, int threads) {
+    constexpr float c = 2.f * (float)kPi;
+    const int each = n / threads, more = n - each * threads;
+    float s = 0.f;
+    for (int q = 0; q < each; q++) s += c;
+    const float s1 = s + c;
+    if (!BLOCK) return (double)s * (threads - more) + (double)s1 * more;
+    float b = 0.f, b1 = 0.f;  // blocks whose threads all sum s, s1
+    for (int w = 0; w < kBlock / 32; w++) {
+        b += 32.f * s;
+        b1 += 32.f * s1;
+    }
+    const int full1 = more / kBlock, part = more - full1 * kBlock;
+    const int full = threads / kBlock - full1 - (part ? 1 : 0);
+    double t = (double)b * full + (double)b1 * full1;
+    if (part) t += (double)s1 * part + (double)s * (kBlock - part);
+    return t;
+}
+
 // ---------------------------------------------------------------- predict
 // Skipped (every block returns at once) when the last correct already
 // wrote this attempt's prediction and its area sums.
@@ -240,7 +267,7 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
             if (gas) {
                 const float apr = DIM == 3 ? (4.f * (float)kPi) * rp : 2.f * (float)kPi;
                 sA = fmaf(apr, rp, sA);
-                sAr += apr;
+                if (!(RES && DIM == 2)) sAr += apr;  // 2D: area_over_radius_2d
             }
         }
     }
@@ -603,7 +630,8 @@ __device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, con
             Ctrl *cc = b.ctrl;
             if (!cc->pred_ready) {  // the prediction of this attempt's predict phase
                 cc->sumA = __ldcg(&rx->acc->sum[0]);
-                cc->sumAr = __ldcg(&rx->acc->sum[1]);
+                cc->sumAr = DIM == 3 ? __ldcg(&rx->acc->sum[1])
+                                     : area_over_radius_2d<false>(cc->n, rx->threads);
             }
             cc->sumAo = 2.0 * fAo;
             cc->sumAor = fAor;
@@ -900,10 +928,10 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
                     const float apr = DIM == 3 ? (4.f * (float)kPi) * rp1 : 2.f * (float)kPi;
                     if (u) {
                         cA1 = fmaf(apr, rp1, cA1);
-                        cAr1 += apr;
+                        if (!(RES && DIM == 2)) cAr1 += apr;  // area_over_radius_2d
                     } else {
                         cA0 = fmaf(apr, rp1, cA0);
-                        cAr0 += apr;
+                        if (!(RES && DIM == 2)) cAr0 += apr;
                     }
                 }
             }
@@ -919,19 +947,24 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
         const double sv[5] = {vol, (double)cA0, (double)cA1, (double)cAr0, (double)cAr1};
         const long long m[3] = {merr, mrad, __double_as_longlong(double_from_float(mexp))};
         const int cn[2] = {ndel, bad};
-        run_reduce<GAS ? 5 : 1, 3, 2>(sv, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
+        run_reduce<!GAS ? 1 : (DIM == 2 ? 3 : 5), 3, 2>(sv, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
         run_barrier(rx);
         if (threadIdx.x == 0) {
             const RunAcc *g = rx->acc;
             const double e = __longlong_as_double(__ldcg(&g->cmax[0])),
                          r = __longlong_as_double(__ldcg(&g->cmax[1])),
                          x = __longlong_as_double(__ldcg(&g->cmax[2])), v = __ldcg(&g->csum[0]);
-            const int nd = __ldcg(&g->cnt[0]), nb = __ldcg(&g->cnt[1]);
+            const int nd = __ldcg(&g->cnt[0]), nx = __ldcg(&g->cnt[1]);
             c->cand_sumA[0] = __ldcg(&g->csum[1]);
             c->cand_sumA[1] = __ldcg(&g->csum[2]);
-            c->cand_sumAr[0] = __ldcg(&g->csum[3]);
-            c->cand_sumAr[1] = __ldcg(&g->csum[4]);
-            finish_attempt<DIM>(c, k, e, r, x, v, (double)nd, (double)nb);
+            if (DIM == 3) {
+                c->cand_sumAr[0] = __ldcg(&g->csum[3]);
+                c->cand_sumAr[1] = __ldcg(&g->csum[4]);
+            } else {
+                c->cand_sumAr[0] = c->cand_sumAr[1] =
+                    area_over_radius_2d<true>(n, rx->threads);
+            }
+            finish_attempt<DIM>(c, k, e, r, x, v, (double)nd, (double)nx);
         }
         __syncthreads();
         return;
@@ -973,19 +1006,31 @@ CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_
 // after an accepted attempt the next prediction is ready (two barriers then,
 // three otherwise).
 template <int DIM, bool GAS, bool FLOW, bool WALLS>
-__global__ void __launch_bounds__(kBlock, 2) k_run_mx(Bufs b, Ctrl *mirror, long long n_steps) {
+__global__ void __launch_bounds__(kBlock, 2) k_run_mx(Bufs b, const Bufs *foams,
+                                                    const RunBlock *map, Ctrl *mirror,
+                                                    long long n_steps, int threads) {
     __shared__ RunShared rs;
     __shared__ RunRed rsm;
-    const int vb = blockIdx.x, vg = gridDim.x;
+    int vb = blockIdx.x, vg = gridDim.x;
+    if (map) {  // batched: every foam its own blocks, barrier and loop
+        const RunBlock w = map[blockIdx.x];
+        b = foams[w.foam];
+        vb = w.vb;
+        vg = w.vg;
+        if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
+    }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed};
+    // threads of the launch per phase (area_over_radius_2d): the virtual grid
+    // of a batched foam, else four resident blocks per SM
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed,
+              map ? b.ctrl->vgrid_a * kBlock : threads};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
     do {
         run_begin(&rx, attempts);
         k_predict_mx_body<DIM, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
-        k_pairs_mx_body<DIM, GAS, FLOW, 2, true>(b, vb, vg, &rx, &rsm);
+        k_pairs_mx_body<DIM, GAS, FLOW, 4, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
         k_correct_mx_body<DIM, GAS, FLOW, WALLS, true>(b, vb, vg, &rx, &rsm);
     } while (run_more(&rs, ++attempts));

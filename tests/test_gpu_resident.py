@@ -82,3 +82,41 @@ def test_resident_deletions_and_stops(precision):
     sa, sb = a.get_state(), b.get_state()
     assert (sa["index"] == sb["index"]).all()
     assert_rows_close(sa, sb, ["x", "y", "r"], 1e-6 if precision == 1 else 1e-11, "resident ")
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("dim,options,kw", [
+    (2, "gas", {}), (3, "walls", {}), (3, "flow", {}),
+    (2, "gas", dict(rstd=0.3, rclip=(0.01, 2.0), min_rad=0.2))])
+def test_resident_batch_matches_batched_launches(dim, options, kw, precision):
+    """A batch of small foams (resident: every foam its own blocks and loop)
+    against the same batch with one foam's capacity beyond the resident
+    total (the batched launches): the foams search, delete and finish at
+    different attempts."""
+    sizes = (1, 700, 5003, 2048, 12001)
+    reports, states, launches = [], [], []
+    for beyond in (0, 1):
+        items = []
+        for f, n in enumerate(sizes):
+            args = dict(seed=900 + f, kappa=0.01 * (f + 1), precision=precision, use_graph=1)
+            if beyond and f == 3:
+                args.update(capacity=1000001, pair_capacity=16 * n)
+            args.update(OPTIONS[options])
+            args.update(kw)
+            items.append(workloads.foam(n, dim, 0.9 if dim == 2 else 0.8, **args))
+        batch = cb.GpuFoamBatch([c for c, _ in items])
+        for (_, st), f in zip(items, batch.foams):
+            f.load_state(st)
+            workloads.prepare(f)
+        n0 = batch.launch_count()
+        reports.append(batch.integrate(40))
+        launches.append(batch.launch_count() - n0)
+        states.append([by_index(f.get_state()) for f in batch.foams])
+        batch.close()
+    assert launches[0] < launches[1]
+    for f in range(len(sizes)):
+        for k in ("steps", "attempts", "searches", "deleted", "count", "num_pairs"):
+            assert reports[0][f][k] == reports[1][f][k], (f, k)
+        assert_rows_close(states[0][f], states[1][f], ["x", "y", "z", "r", "dxdt", "drdt", "path"],
+                          1e-6 if precision == 1 else 1e-11, "batch ",
+                          floor=position_ulp(states[1][f]))
