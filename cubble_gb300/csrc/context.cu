@@ -137,6 +137,46 @@ __global__ void __launch_bounds__(kBlock) k_max_radius(const double *R, int n, C
                   (unsigned long long)m);
 }
 
+// The mixed form's FP32 rate rows to and from the host's FP64 rows, through
+// scratch rows on the device. Bound by its 12 bytes per element (3 10^6
+// bubbles, 8 rows: ~45 us); the same conversion on the host took 10 ms of a
+// cb_get_state of 3 10^6 bubbles and 3 ms at 10^6.
+constexpr int kRateRows = 8;
+struct RateRows {
+    float *f[kRateRows];
+    double *d[kRateRows];
+    int rows = 0;
+    void add(double *row, double *scratch) {
+        f[rows] = reinterpret_cast<float *>(row);
+        d[rows++] = scratch;
+    }
+};
+template <bool WIDEN>
+__global__ void __launch_bounds__(kBlock) k_rate_rows(RateRows p, int n) {
+    for (int r = 0; r < p.rows; r++)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            if (WIDEN)
+                p.d[r][i] = (double)p.f[r][i];
+            else
+                p.f[r][i] = (float)p.d[r][i];
+        }
+}
+// Scratch for row q: the search's partner stash, which holds nothing between
+// calls (16 or more int32 per bubble: room for kRateRows rows).
+double *rate_scratch(const cb_context *c, int q) {
+    static_assert(kStash(2) * 4 >= kRateRows * 8 && kStash(3) * 4 >= kRateRows * 8, "");
+    return reinterpret_cast<double *>(c->bufs.stash) + (size_t)q * c->hk.cap;
+}
+int convert_rates(cb_context *c, const RateRows &p, size_t n, bool widen) {
+    const int grid = std::min<int>(c->launch.grid, (int)((n + kBlock - 1) / kBlock));
+    if (widen)
+        k_rate_rows<true><<<grid, kBlock, 0, c->stream>>>(p, (int)n);
+    else
+        k_rate_rows<false><<<grid, kBlock, 0, c->stream>>>(p, (int)n);
+    c->launches += 1;
+    return c->check_launch();
+}
+
 }  // namespace
 
 namespace cbg {
@@ -635,14 +675,14 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
     drows[RS1] = s->saved_y;
     drows[RS2] = s->saved_z;
     drows[RS3] = s->saved_r;
-    std::vector<std::vector<float>> fl;
+    RateRows rates;
     for (int r = 0; r < ND_ROLES; r++) {
         double *dst = c->dslot[h.drole[r]];
         const bool rate = r >= RV0 && r <= RVP3;
-        if (drows[r] && c->hk.mixed && rate) {  // FP32 rate rows
-            fl.emplace_back(drows[r], drows[r] + n);
-            CB_CUDA(cudaMemcpyAsync(dst, fl.back().data(), n * 4, cudaMemcpyHostToDevice,
-                                    c->stream));
+        if (drows[r] && n && c->hk.mixed && rate) {  // FP32 rate rows
+            rates.add(dst, rate_scratch(c, rates.rows));
+            CB_CUDA(cudaMemcpyAsync(rates.d[rates.rows - 1], drows[r], n * 8,
+                                    cudaMemcpyHostToDevice, c->stream));
         } else if (drows[r]) {
             CB_CUDA(cudaMemcpyAsync(dst, drows[r], n * 8, cudaMemcpyHostToDevice, c->stream));
         } else if (r >= RS0 && r <= RS3 && n && drows[RX + (r - RS0)]) {
@@ -654,6 +694,7 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
             CB_CUDA(cudaMemsetAsync(dst, 0, (size_t)c->hk.cap * 8, c->stream));
         }
     }
+    if (rates.rows && (rc = convert_rates(c, rates, n, false))) return rc;
     const int32_t *irows[NI_ROLES] = {};
     irows[IWX] = s->wrap_count_x;
     irows[IWY] = s->wrap_count_y;
@@ -722,15 +763,22 @@ int cb_get_state(cb_context *c, cb_state_view *s) {
     drows[RS1] = s->saved_y;
     drows[RS2] = s->saved_z;
     drows[RS3] = s->saved_r;
-    std::vector<std::pair<double *, std::vector<float>>> fl;
+    RateRows rates;
+    double *to[kRateRows];
+    if (c->hk.mixed && n)  // FP32 rate rows
+        for (int r = RV0; r <= RVP3; r++)
+            if (drows[r]) {
+                to[rates.rows] = drows[r];
+                rates.add(c->dslot[h.drole[r]], rate_scratch(c, rates.rows));
+            }
+    if (rates.rows) {
+        if ((rc = convert_rates(c, rates, n, true))) return rc;
+        for (int q = 0; q < rates.rows; q++)
+            CB_CUDA(cudaMemcpyAsync(to[q], rates.d[q], n * 8, cudaMemcpyDeviceToHost, c->stream));
+    }
     for (int r = 0; r < ND_ROLES; r++) {
         if (!drows[r] || !n) continue;
-        if (c->hk.mixed && r >= RV0 && r <= RVP3) {  // FP32 rate rows
-            fl.emplace_back(drows[r], std::vector<float>(n));
-            CB_CUDA(cudaMemcpyAsync(fl.back().second.data(), c->dslot[h.drole[r]], n * 4,
-                                    cudaMemcpyDeviceToHost, c->stream));
-            continue;
-        }
+        if (c->hk.mixed && r >= RV0 && r <= RVP3) continue;
         CB_CUDA(cudaMemcpyAsync(drows[r], c->dslot[h.drole[r]], n * 8, cudaMemcpyDeviceToHost,
                                 c->stream));
     }
@@ -745,8 +793,6 @@ int cb_get_state(cb_context *c, cb_state_view *s) {
             CB_CUDA(cudaMemcpyAsync(irows[r], c->islot[h.irole[r]], n * 4, cudaMemcpyDeviceToHost,
                                     c->stream));
     CB_CUDA(cudaStreamSynchronize(c->stream));
-    for (auto &f : fl)
-        for (size_t i = 0; i < n; i++) f.first[i] = f.second[i];
     return CB_OK;
 }
 

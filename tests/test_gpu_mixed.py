@@ -229,3 +229,31 @@ def test_mixed_containment_threshold(oracle_mod, dim):
     for k in ("overlap", "drdtp", "dxdtp"):
         assert max_rel(ag[k][og], ao[k][oo]) <= 1e-6, k
     assert ag["total_overlap_area"] == pytest.approx(ao["total_overlap_area"], rel=1e-6)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [1, 255, 1001])
+def test_mixed_rate_rows_round_trip(dim, n):
+    """The FP32 rate rows through cb_load_state and cb_get_state: every value
+    comes back as its FP32 rounding (subnormals, infinities and NaN too),
+    whichever of the rows are given or asked for."""
+    cfg, st = workloads.foam(n, dim, 0.5, seed=5, precision=1)
+    rng = np.random.default_rng(9)
+    rates = ["dxdt", "dydt", "dzdt", "drdt", "dxdto", "dydto", "dzdto", "drdto"]
+    special = np.array([0.0, -0.0, 1e-41, -3e-45, 1e300, -np.inf, np.nan, 1.0 + 2.0 ** -24])
+    for k in rates:
+        st[k] = rng.normal(size=n) * 10.0 ** rng.integers(-12, 12, n)
+        m = min(n, len(special))
+        st[k][:m] = special[:m]
+    st.pop("dydto")
+    g = cb.GpuFoam(cfg)
+    g.load_state(st)
+    got = g.get_state()
+    with np.errstate(over="ignore"):
+        for k in rates:
+            want = st[k].astype(np.float32).astype(np.float64) if k in st else np.zeros(n)
+            assert np.array_equal(got[k], want, equal_nan=True), k
+            assert np.array_equal(np.signbit(got[k]), np.signbit(want)) or n > 6, k
+    part = g.get_state(rows=("drdt", "x", "dxdto"))
+    for k in part:
+        assert np.array_equal(part[k], got[k], equal_nan=True), k
