@@ -278,7 +278,7 @@ void launch_batch_run(cb_batch *b) {
     if (c->hk.mixed)
         launch_run_mx(r, c->bufs, c->hk.dim, c->mode(), c->hk.any_wall != 0);
     else
-        launch_run(r, c->bufs, c->hk.dim, c->mode(), c->hk.ffpair != 0);
+        launch_run(r, c->bufs, c->hk.dim, c->mode());
     k_batch_decide<<<1, 1024, 0, b->stream>>>(b->dbufs, (int)b->foams.size(), b->dbc, b->dwork,
                                               0);
     b->launches += 1;

@@ -8,8 +8,9 @@
 //     the cell-order permutation of a search (src/simulator.cu:96-147) are
 //     role swaps done on the device; no host round trip is needed;
 //   * `pred` packs the predicted state of a bubble into one 32-byte sector
-//     (3D: xp,yp,zp,rp; 2D: xp,yp,rp,1/rp) because the pair kernel gathers
-//     it for both members of every pair;
+//     (3D: xp,yp,zp,rp; 2D: xp,yp,rp,1/rp; FP64 form: positions and radius as
+//     fixed point) because the pair kernel gathers it for both members of
+//     every pair;
 //   * `acc` holds 8 FP64 accumulators per bubble (64 bytes: vx,vy,vz,vr,
 //     overlap, flow vx,vy,vz) that the pair kernel adds into with FP64
 //     atomics; it is all zero between attempts (the correct kernel reads
@@ -22,6 +23,7 @@
 
 #include "../../include/cubble_gb300.h"
 #include "ff.cuh"
+#include "fixpair.cuh"
 
 namespace cbg {
 
@@ -74,13 +76,16 @@ struct DevConst {
     // step_mixed.cu); lq / hq are the periodic box length and half of it in
     // those units.
     long long lq[3], hq[3];
+    // FP64 form: predicted positions and radii in units 2^-fix_b (fixpair.cuh)
+    // and the periodic box length and half of it in those units
+    long long flq[3], fhq[3];
+    double fix_unit;  // 2^-fix_b
+    int fix_b;
     int mixed;
     float f0_f;  // f0/mu0 as FP32
-    float f0_l;  // f0/mu0 - f0_f: the float-float f0 of k_pairs_ff
     // FP32 copies for the search's candidate tests (a double -> float
     // conversion is an FP64-pipe instruction)
     float skin_f, lbb_f[3];
-    int ffpair;  // CB_PRECISION_FP64_FF: pair terms in float-float
     float kq_f;  // K / (4 pi) in 3D, K / (2 pi) in 2D, as FP32
     float pre_margin;  // FP32 pair-search prefilter margin (length units)
     long long lbq[3];  // the box's lower corner in fixed point (x 2^40)
@@ -179,7 +184,6 @@ struct Bufs {
     double *pred;       // 4 doubles per bubble
     double *predc;      // mixed form: two candidate predictions, 8 doubles per bubble
     double *invr;       // FP64 form, 3D: (1 / rp, rp^2) per bubble
-    float4 *ffr;        // CB_PRECISION_FP64_FF: float-float (rp, 1 / rp), (rp^2, 0)
     double *acc;        // kAcc doubles per bubble
     double *part;       // kPartSlots x grid partials
     int *delflag;       // deletion marks of the last attempt
@@ -445,13 +449,6 @@ __device__ __forceinline__ double abs_bits(double x) {
     int hi;
     asm("and.b32 %0, %1, 0x7fffffff;" : "=r"(hi) : "r"(__double2hiint(x)));
     return __hiloint2double(hi, __double2loint(x));
-}
-__device__ __forceinline__ bool nonneg_bits(double x) { return __double2hiint(x) >= 0; }
-__device__ __forceinline__ bool less_nonneg(double a, double b) {
-    return __double_as_longlong(a) < __double_as_longlong(b);
-}
-__device__ __forceinline__ double min_nonneg(double a, double b) {
-    return __longlong_as_double(min(__double_as_longlong(a), __double_as_longlong(b)));
 }
 
 // Minimum image on a periodic axis: |d| > L/2 is tested on the 32-bit words
@@ -987,10 +984,9 @@ inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
 }
 
 // step.cu
-void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode, bool ff);
+void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode);
 void launch_predict(const Launch &l, const Bufs &b, int dim);
-void launch_pairs(const Launch &l, const Bufs &b, int dim, int mode,
-                  bool ff);  // mode: gas 1 | flow 2; ff: float-float kernel
+void launch_pairs(const Launch &l, const Bufs &b, int dim, int mode);  // mode: gas 1 | flow 2
 void launch_correct(const Launch &l, const Bufs &b, int dim);
 void launch_boot(const Launch &l, const Bufs &b, int dim, int phase);
 // step_mixed.cu (mixed form)

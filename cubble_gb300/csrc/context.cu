@@ -80,9 +80,7 @@ void fill_const(cb_context *c) {
         k.iv32[a] = (float)k.iv[a];
     }
     k.mixed = f.precision == CB_PRECISION_MIXED ? 1 : 0;
-    k.ffpair = f.precision == CB_PRECISION_FP64_FF ? 1 : 0;
     k.f0_f = (float)k.f0;
-    k.f0_l = (float)(k.f0 - (double)k.f0_f);
     k.skin_f = (float)k.skin;
     for (int a = 0; a < 3; a++) k.lbb_f[a] = (float)k.lbb[a];
     k.kq_f = (float)(k.dim == 3 ? k.K / (4.0 * 3.1415926535897932384626433832795) :
@@ -91,6 +89,17 @@ void fill_const(cb_context *c) {
         k.lq[a] = (long long)std::llround(k.iv[a] * 1099511627776.0);  // 2^40
         k.hq[a] = k.lq[a] / 2;
         k.lbq[a] = (long long)std::llround(k.lbb[a] * 1099511627776.0);
+    }
+    {  // 2^e bounds the box corners and edges with an eighth to spare for
+       // bubbles past the box between searches; positions reach 2^(e + 1)
+        int e = 0;
+        std::frexp(1.125 * std::max(std::max(maxabs, maxiv), 1e-300), &e);
+        k.fix_b = std::min(std::max(62 - e, -900), 900);
+        k.fix_unit = std::ldexp(1.0, -k.fix_b);
+        for (int a = 0; a < 3; a++) {
+            k.flq[a] = (long long)std::llround(std::ldexp(k.iv[a], k.fix_b));
+            k.fhq[a] = k.flq[a] / 2;
+        }
     }
     // Guard band of the FP32 pair prefilters. An FP32 coordinate carries up
     // to 2^-24 |x| rounding, a periodic shift or minimum image another
@@ -206,7 +215,7 @@ void launch_attempt_kernels(const cb_context *c, const Launch &l, const Bufs &b,
         if (which & 4) launch_correct_mx(l, b, dim, c->mode(), c->hk.any_wall != 0);
     } else {
         if (which & 1) launch_predict(l, b, dim);
-        if (which & 2) launch_pairs(l, b, dim, c->mode(), c->hk.ffpair != 0);
+        if (which & 2) launch_pairs(l, b, dim, c->mode());
         if (which & 4) launch_correct(l, b, dim);
     }
 }
@@ -274,7 +283,7 @@ int integrate_resident(cb_context *c, int64_t n_steps) {
         if (c->hk.mixed)
             launch_run_mx(r, c->bufs, c->hk.dim, c->mode(), c->hk.any_wall != 0);
         else
-            launch_run(r, c->bufs, c->hk.dim, c->mode(), c->hk.ffpair != 0);
+            launch_run(r, c->bufs, c->hk.dim, c->mode());
         int rc = c->check_launch();
         if (rc) return rc;
         CB_CUDA(cudaStreamSynchronize(c->stream));
@@ -557,7 +566,6 @@ int cbg::create_context(const cb_config *cfg, cb_context **out, bool graph) {
     if ((rc = c->alloc(&b.pred, 4 * cap))) return bail(rc);
     if (c->hk.mixed && (rc = c->alloc(&b.predc, 8 * cap))) return bail(rc);
     if ((rc = c->alloc(&b.invr, 2 * cap))) return bail(rc);
-    if (c->hk.ffpair && (rc = c->alloc(&b.ffr, 2 * cap))) return bail(rc);
     if ((rc = c->alloc(&b.acc, (size_t)kAcc * cap))) return bail(rc);
     if ((rc = c->alloc(&b.part, (size_t)kPartSlots * G))) return bail(rc);
     if ((rc = c->alloc(&b.delflag, cap + 1))) return bail(rc);
@@ -868,9 +876,9 @@ int cb_bootstrap(cb_context *c) {
         launch_boot_mx(c->launch, c->bufs, dim, 2);
     } else {
         launch_boot(c->launch, c->bufs, dim, 0);
-        launch_pairs(c->launch, c->bufs, dim, 0, c->hk.ffpair != 0);
+        launch_pairs(c->launch, c->bufs, dim, 0);
         launch_boot(c->launch, c->bufs, dim, 1);
-        launch_pairs(c->launch, c->bufs, dim, 0, c->hk.ffpair != 0);
+        launch_pairs(c->launch, c->bufs, dim, 0);
         launch_boot(c->launch, c->bufs, dim, 2);
     }
     int rc = c->check_launch();

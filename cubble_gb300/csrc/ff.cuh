@@ -1,11 +1,8 @@
-// Float-float ("double-FP32") arithmetic for the FP64 form's pair kernel.
-//
-// GB300 issues FP64 at 1/64 of the FP32 rate, so the pair geometry, the
-// overlap velocities and the gas-exchange terms of the FP64 form are carried
-// as unevaluated sums h + l of two floats (about 47 significant bits, relative
-// error per operation ~2^-46) on the FP32 and integer pipes. Only the
-// position differences stay FP64 instructions (the reference's
-// wrappedDifference, src/kernels.cu:1094-1114).
+// Float-float ("double-FP32") arithmetic: values carried as unevaluated sums
+// h + l of two floats (about 47 significant bits, relative error per
+// operation ~2^-46) on the FP32 and integer pipes, because GB300 issues FP64 at
+// 1/64 of the FP32 rate. Used where 2^-46 is enough (norms of differences) and
+// as the estimate that an FP64 residual completes (rcp_d, rsqrt_d).
 //
 // Methods (all from the published literature, written here from the maths):
 //   * error-free transformations: Knuth's TwoSum, Dekker's Fast2Sum, and the
@@ -263,12 +260,6 @@ CB_HD ff ff_mul(ff a, ff b) {
     e = ff_fma(a.l, b.h, e);
     return fast_two_sum(p, e);
 }
-CB_HD ff ff_mul_f(ff a, float b) {
-    const float p = ff_mulr(a.h, b);
-    float e = ff_fma(a.h, b, -p);
-    e = ff_fma(a.l, b, e);
-    return fast_two_sum(p, e);
-}
 CB_HD ff ff_sqr(ff a) {
     const float p = ff_mulr(a.h, a.h);
     float e = ff_fma(a.h, a.h, -p);
@@ -308,12 +299,6 @@ CB_HD ff ff_rsqrt(ff a) {
 CB_HD ff ff_sqrt(ff a) {
     if (!(a.h > 0.0f)) return {0.0f, 0.0f};
     return ff_mul(a, ff_rsqrt(a));
-}
-
-// a - b evaluated to ~2^-46 (|a| + |b|), as one float: for sign tests.
-CB_HD float ff_diff_f(ff a, ff b) {
-    const ff s = two_sum(a.h, -b.h);
-    return ff_addr(s.h, ff_addr(s.l, ff_subr(a.l, b.l)));
 }
 
 // ------------------------------------------- FP64 results with few FP64 ops

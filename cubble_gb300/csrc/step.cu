@@ -23,30 +23,28 @@ __device__ __forceinline__ double4_32a ld4(const double *p, int i) {
     return reinterpret_cast<const double4_32a *>(p)[i];
 }
 
-// Float-float records of the float-float pair kernel (CB_PRECISION_FP64_FF):
-// (r, 1/r) and (r^2, 0) per bubble, written where the predicted radius is
-// known.
-struct FfRec {
-    ff r, inv, rsq;
+// The packed predicted state of bubble i (positions and radius as fixed point,
+// fixpair.cuh; 2D: 1/r beside them): written and read back. The way back is
+// exact: the integer has no more bits than the double it was rounded from.
+template <int DIM>
+__device__ __forceinline__ void st_state(const Bufs &b, int i, double x, double y, double z,
+                                         double r, double inv, int fixb) {
+    double4_32a p;
+    const double qr = __longlong_as_double(fx_from_double(r, fixb));
+    p.x = __longlong_as_double(fx_from_double(x, fixb));
+    p.y = __longlong_as_double(fx_from_double(y, fixb));
+    p.z = DIM == 3 ? __longlong_as_double(fx_from_double(z, fixb)) : qr;
+    p.w = DIM == 3 ? qr : inv;
+    reinterpret_cast<double4_32a *>(b.pred)[i] = p;
+}
+struct State {
+    double x, y, z, r, inv;  // inv in 2D only
 };
-__device__ __forceinline__ FfRec ld_rec(const float4 *R, int i) {
-    const float4 u = R[2 * (size_t)i], v = R[2 * (size_t)i + 1];
-    return {{u.x, u.y}, {u.z, u.w}, {v.x, v.y}};
-}
-__device__ __forceinline__ void st_rec(float4 *R, int i, double r, double inv, double rsq) {
-    const ff a = ff_of(r), b = ff_of(inv), c = ff_of(rsq);
-    R[2 * (size_t)i] = make_float4(a.h, a.l, b.h, b.l);
-    R[2 * (size_t)i + 1] = make_float4(c.h, c.l, 0.f, 0.f);
-}
-__device__ __forceinline__ bool ff_less(ff a, ff b) {  // normalised pairs
-    return a.h < b.h || (a.h == b.h && a.l < b.l);
-}
-// Reduction of a float-float value into an FP64 row: both parts widened
-// exactly on the integer pipe and summed by one FP64 add (correctly rounded).
-// The float-float pair kernel is bound by issue slots and leaves the FP64
-// pipe mostly idle, so this costs fewer slots than the integer-pipe rounding.
-__device__ __forceinline__ void add_d(double *p, ff v) {
-    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(ff_f2d(v.h) + ff_f2d(v.l)));
+template <int DIM>
+__device__ __forceinline__ State ld_state(const Bufs &b, int i, int fixb) {
+    const double4_32a p = ld4(b.pred, i);
+    auto back = [&](double q) { return fx_to_double_signed(__double_as_longlong(q), -fixb); };
+    return {back(p.x), back(p.y), DIM == 3 ? back(p.z) : 0.0, back(DIM == 3 ? p.w : p.z), p.w};
 }
 
 // ---------------------------------------------------------------- predict
@@ -65,6 +63,7 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
                  *V3 = drow(b, c, RV3);
     const double *O0 = drow(b, c, RVO0), *O1 = drow(b, c, RVO1), *O2 = drow(b, c, RVO2),
                  *O3 = drow(b, c, RVO3);
+    const int fixb = b.k->fix_b;
     double sA = 0.0, sAr = 0.0;
     int na = 0;
     for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
@@ -75,21 +74,9 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
         if (gas) rp = fma(h, fma(3.0, V3[i], -O3[i]), rp);
         const double inv = rcp_d(rp);
         const double rsq = rp * rp;
-        if (b.ffr) st_rec(b.ffr, i, rp, inv, rsq);
-        double4_32a p;
-        if (DIM == 3) {
-            p.x = xp;
-            p.y = yp;
-            p.z = fma(h, fma(3.0, V2[i], -O2[i]), Z[i]);
-            p.w = rp;
-            reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
-        } else {
-            p.x = xp;
-            p.y = yp;
-            p.z = rp;
-            p.w = inv;
-        }
-        reinterpret_cast<double4_32a *>(b.pred)[i] = p;
+        const double zp = DIM == 3 ? fma(h, fma(3.0, V2[i], -O2[i]), Z[i]) : 0.0;
+        if (DIM == 3) reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
+        st_state<DIM>(b, i, xp, yp, zp, rp, inv, fixb);
         if (gas) {  // area and area per radius, src/kernels.cu:103-112, with
                     // the constant factor (4 pi, 2 pi) applied to the block sums
             if (DIM == 3) {
@@ -129,37 +116,31 @@ CB_KERNEL_PAIR((template <int DIM>), k_predict, (<DIM>), __launch_bounds__(kBloc
 
 
 // ------------------------------------------------------------------ pairs
-// Overlap velocities, pairwise gas flux and overlap areas in FP64
-// (pairwiseInteraction, src/kernels.cu:172-337). FP64-issue bound on GB300
-// (2 FP64 thread-instructions per SM and cycle), so:
-//   * each warp takes 32 consecutive pairs, computes their FP64 differences
-//     and overlap test (3 FP64 instructions a pair; the test in FP32 with a
-//     guard band), and queues the overlapping ones (about 70 % of the listed
-//     pairs) in shared memory; the distance, force and gas-exchange
-//     arithmetic then runs on full warps of overlapping pairs, not on warps
-//     with idle lanes;
-//   * minimum image by bit compare; 1/sqrt(m) and 1/(r1 + r2) to ~1 ulp by
-//     rsqrt_d / rcp_d (2 and 1 FP64 instructions, the rest on the FP32 and
-//     integer pipes); the division by m of the overlap formula as a product
-//     with (1/sqrt(m))^2; -w/4 on the exponent field; no product by f0 when
-//     it is 1;
-//   * contributions to both members go through FP64 reductions into the
-//     per-bubble accumulator rows;
-//   * overlap areas are accumulated in units of ov_unit (pi in 3D, 2 in 2D),
-//     one FP64 product less per overlapping pair; the unit is applied to the
-//     global sums and in the correct kernel.
+// Overlap velocities, pairwise gas flux and overlap areas
+// (pairwiseInteraction, src/kernels.cu:172-337) with FP64 results. GB300
+// issues 2 FP64 thread-instructions per SM and cycle and its L1 takes one
+// record of a scattered access per cycle, so:
+//   * the predicted positions and radii are 64-bit fixed point, and distance,
+//     reciprocals, force and overlap of a pair run on the integer pipe, more
+//     exactly than in FP64 (fixpair.cuh: force to 9e-17 of f0 at most, FP64
+//     4e-16; overlap to 3e-17 R^2, FP64 6e-16). FP64 is left for the gas flux
+//     and the sums: 5 instructions per overlapping pair (21 before);
+//   * each warp takes 32 consecutive pairs, tests their overlap in FP32 with
+//     a guard band (exact integers inside it), and queues the overlapping
+//     ones (about 70 % of the listed pairs) in shared memory; the force and
+//     gas-exchange arithmetic runs on full warps of overlapping pairs;
+//   * the results of 32 pairs are transposed through shared memory and added
+//     to the bubbles' rows with FP64 reductions by eight lanes a pair, so
+//     that the reductions of one bubble's 64-byte record make one request
+//     instead of five (alone: 202 -> 177 us);
+//   * overlap areas are accumulated in units of ov_unit (pi in 3D, 2 in 2D);
+//     the unit is applied to the global sums and in the correct kernel.
+// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 125 us (2D 117 -> 86, 3D
+// without gas exchange 141 -> 99). Nothing is saturated now: issue 57 %, L1 59 %
+// of its wavefronts, FP64 29 %; three or four blocks per SM make no difference,
+// record loads a chunk ahead (108 registers) cost 8 us.
 __device__ __forceinline__ void red_add(double *p, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v));
-}
-// -w/4, exact: the exponent field lowered by 2 and the sign flipped when the
-// exponent allows it (|w| > 2^-1020), else the FP64 product (a call, so that
-// it is not computed for every pair).
-static __device__ __noinline__ double neg_quarter_slow(double w) { return -0.25 * w; }
-__device__ __forceinline__ double neg_quarter(double w) {
-    const int hi = __double2hiint(w);
-    if ((hi & 0x7ff00000) > 0x00200000)
-        return __hiloint2double((hi - 0x00200000) ^ (int)0x80000000, __double2loint(w));
-    return neg_quarter_slow(w);
 }
 
 constexpr int kQueue = 64;  // per-warp queue of overlapping pairs
@@ -209,16 +190,52 @@ __device__ __forceinline__ void pairs_fold(const Bufs &b, const int vb, const in
     }
 }
 
-// The overlap test of the reference in FP64 (the sign of the exact
-// (r1 + r2)^2 - m), for pairs in the FP32 guard band.
+// The overlap test for pairs in the FP32 guard band: (r1 + r2)^2 >= d^2 from
+// the exact integers (R >= 0, a unit of 2^-60 R^2).
 template <int DIM>
-static __device__ __noinline__ bool overlap_exact(double dx, double dy, double dz, double r1,
-                                                  double r2) {
+static __device__ __noinline__ bool overlap_exact(long long ex, long long ey, long long ez,
+                                                  long long R) {
+    if (llabs(ex) > R || llabs(ey) > R || (DIM == 3 && llabs(ez) > R)) return false;
+    const int s = fx_clz((unsigned long long)R | 1ull) - 1;
+    long long m = fx_square(ex << s) + fx_square(ey << s);
+    if (DIM == 3) m += fx_square(ez << s);
+    return fx_square(R << s) >= m;
+}
+
+// The terms of a pair fx_pair does not take, in FP64: centres much closer
+// than the radii, a negative predicted radius. The force goes to rs[0],
+// rs[kT], ...; returns the overlap as FxTerms::oa.
+constexpr int kT = 33;  // row length of the transposed results (32 pairs)
+template <int DIM>
+static __device__ __noinline__ double pair_slow(long long ex, long long ey, long long ez,
+                                                long long q1, long long q2, double unit,
+                                                double f0, double *rs) {
+    const double dx = (double)ex * unit, dy = (double)ey * unit, dz = (double)ez * unit;
+    const double r1 = (double)q1 * unit, r2 = (double)q2 * unit;
     double m = dx * dx;
     m = fma(dy, dy, m);
     if (DIM == 3) m = fma(dz, dz, m);
-    const double radii = r1 + r2;
-    return nonneg_bits(fma(radii, radii, -m));
+    const double y = rsqrt_d(m), s = (y - rcp_d(r1 + r2)) * f0;
+    rs[0 * kT] = dx * s;
+    rs[1 * kT] = dy * s;
+    if (DIM == 3) rs[2 * kT] = dz * s;
+    const double r1sq = r1 * r1, r2sq = r2 * r2;
+    if (m < r1sq || m < r2sq) return fmin(r1sq, r2sq);
+    const double w = (r2sq - r1sq + m) * y;
+    return fabs(fma(-0.25 * w, w, r2sq));
+}
+
+// The force times f0 where it is not 1 (a call: inlined, its FP64 products
+// are predicated into every pair).
+template <int DIM>
+static __device__ __noinline__ void scale_force(double f0, double *rs) {
+#pragma unroll
+    for (int a = 0; a < DIM; a++) rs[a * kT] *= f0;
+}
+
+// A fixed-point length as FP32, in units of 2^62.
+__device__ __forceinline__ float fix_len(long long v) {
+    return fx_float((unsigned long long)(v < 0 ? -v : v)) * 0x1p-62f;
 }
 
 template <int DIM, bool GAS, bool FLOW, bool RES = false>
@@ -226,10 +243,13 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
                                              RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
     constexpr int kW = kBlock / 32;
     __shared__ double smem[32];
-    // queue slots: dx, dy, (3D: dz), r1, r2
-    constexpr int kR1 = DIM == 3 ? 3 : 2, kSlots = kR1 + 2;
-    __shared__ double qd[kW][kSlots][kQueue];
+    // queue slots: the differences, both radii
+    constexpr int kR1 = DIM, kSlots = kR1 + 2;
+    __shared__ long long qd[kW][kSlots][kQueue];
     __shared__ int qij[kW][2][kQueue];
+    // the results of 32 pairs, component by component
+    constexpr int kC = GAS ? DIM + 2 : DIM;
+    __shared__ double res[kW][kC * kT];
     const Ctrl *c = b.ctrl;
     const DevConst &k = *b.k;
     const int np = c->np;
@@ -237,93 +257,97 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     const int *PJ = b.ps[c->prole[PJ0]];
     const double *V0 = drow(b, c, RV0), *V1 = drow(b, c, RV1), *V2 = drow(b, c, RV2);
     const double f0 = k.f0;
+    const bool scaled = __double_as_longlong(f0) != 0x3ff0000000000000LL;
+    const int fixb = k.fix_b;
     const bool px = !k.wall[0], py = !k.wall[1], pz = DIM == 3 && !k.wall[2];
-    const double hx = k.half_iv[0], hy = k.half_iv[1], hz = k.half_iv[2];
-    const double Lx = k.iv[0], Ly = k.iv[1], Lz = k.iv[2];
+    const long long hx = k.fhq[0], hy = k.fhq[1], hz = k.fhq[2];
+    const long long Lx = k.flq[0], Ly = k.flq[1], Lz = k.flq[2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
-    double(*Q)[kQueue] = qd[w];
+    long long(*Q)[kQueue] = qd[w];
     int *QI = qij[w][0], *QJ = qij[w][1];
+    double *RS = res[w];
     double sAo = 0.0, sAor = 0.0;
+
+    // minimum image (wrappedDifference, src/kernels.cu:1094-1114), exact
+    auto image = [](long long d, long long half, long long len) {
+        if (d > half) d -= len;
+        else if (d < -half) d += len;
+        return d;
+    };
 
     // the force and gas-exchange terms of queued (overlapping) pair e
     auto process = [&](int e) {
         const int i = QI[e], j = QJ[e];
-        const double dx = Q[0][e], dy = Q[1][e], dz = DIM == 3 ? Q[2][e] : 0.0;
-        const double r1 = Q[kR1][e], r2 = Q[kR1 + 1][e];
-        double m = dx * dx;
-        m = fma(dy, dy, m);
-        if (DIM == 3) m = fma(dz, dz, m);
-        const double radii = r1 + r2;
-        double *ai = b.acc + (size_t)i * kAcc;
-        double *aj = b.acc + (size_t)j * kAcc;
-        // velocity f0 d (1/|d| - 1/(r1 + r2)), src/kernels.cu:218-233
-        const double rs = rsqrt_d(m);
-        double s = rs - rcp_d(radii);
-        if (f0 != 1.0) s *= f0;
-        const double fx = dx * s, fy = dy * s;
-        red_add(ai + 0, fx);
-        red_add(aj + 0, neg_bits(fx));
-        red_add(ai + 1, fy);
-        red_add(aj + 1, neg_bits(fy));
-        if (DIM == 3) {
-            const double fz = dz * s;
-            red_add(ai + 2, fz);
-            red_add(aj + 2, neg_bits(fz));
+        double inv1 = 0.0, inv2 = 0.0;
+        if (GAS) {  // 1/r of k_predict
+            inv1 = DIM == 3 ? b.invr[2 * (size_t)i] : b.pred[4 * (size_t)i + 3];
+            inv2 = DIM == 3 ? b.invr[2 * (size_t)j] : b.pred[4 * (size_t)j + 3];
         }
-        if (GAS) {  // pairwise gas exchange, src/kernels.cu:236-280
-            double r1sq, r2sq, inv1, inv2;
-            if (DIM == 3) {  // (1/r, r^2) records written by k_predict
-                const double2 e1 = reinterpret_cast<const double2 *>(b.invr)[i];
-                const double2 e2 = reinterpret_cast<const double2 *>(b.invr)[j];
-                inv1 = e1.x;
-                r1sq = e1.y;
-                inv2 = e2.x;
-                r2sq = e2.y;
-            } else {
-                r1sq = r1 * r1;
-                r2sq = r2 * r2;
-                inv1 = b.pred[4 * (size_t)i + 3];
-                inv2 = b.pred[4 * (size_t)j + 3];
-            }
-            const bool inside = less_nonneg(m, r1sq) || less_nonneg(m, r2sq);
-            // chord: r2^2 - t^2 / m with t = (r2^2 - r1^2 + m) / 2, as
-            // r2^2 - w^2 / 4 with w = (r2^2 - r1^2 + m) / |d|; the overlap
-            // area in units of ov_unit (pi in 3D, 2 in 2D)
-            double oa;
-            if (inside) {
-                oa = DIM == 3 ? min_nonneg(r1sq, r2sq) : min_nonneg(r1, r2);
-            } else {
-                const double wv = (r2sq - r1sq + m) * rs;
-                oa = abs_bits(fma(neg_quarter(wv), wv, r2sq));
-                if (DIM == 2) oa = __double_as_longlong(oa) > 0 ? oa * rsqrt_d(oa) : 0.0;
-            }
-            const double g = oa * (inv2 - inv1);
-            red_add(ai + 3, g);
-            red_add(aj + 3, neg_bits(g));
-            red_add(ai + 4, oa);
-            red_add(aj + 4, oa);
+        const long long ex = Q[0][e], ey = Q[1][e], ez = DIM == 3 ? Q[2][e] : 0;
+        const long long q1 = Q[kR1][e], q2 = Q[kR1 + 1][e];
+        double oa;
+        FxTerms t;
+        if (fx_pair<DIM, GAS>(ex, ey, ez, q1, q2, fixb, t)) {
+            RS[0 * kT + e] = t.fx;
+            RS[1 * kT + e] = t.fy;
+            if (DIM == 3) RS[2 * kT + e] = t.fz;
+            oa = t.oa;
+            if (scaled) scale_force<DIM>(f0, RS + e);
+        } else {
+            oa = pair_slow<DIM>(ex, ey, ez, q1, q2, k.fix_unit, f0, RS + e);
+        }
+        if (GAS) {  // pairwise gas exchange, src/kernels.cu:236-280; oa in units of ov_unit
+            if (DIM == 2) oa = __double_as_longlong(oa) > 0 ? oa * rsqrt_d(oa) : 0.0;
+            RS[DIM * kT + e] = oa * (inv2 - inv1);
+            RS[(DIM + 1) * kT + e] = oa;
             sAo += oa;
             sAor = fma(oa, inv1 + inv2, sAor);
         }
         if (FLOW) {  // src/kernels.cu:298-307 (overlapping pairs only)
+            double *ai = b.acc + (size_t)i * kAcc;
             red_add(ai + 5, V0[j]);
             red_add(ai + 6, V1[j]);
             if (DIM == 3) red_add(ai + 7, V2[j]);
         }
     };
+    // adds the results of queued pairs 0..m-1 to both bubbles' rows: eight
+    // lanes a pair, a component each
+    auto scatter = [&](int m) {
+        __syncwarp();
+        const int q = lane & 7;
+        const int slot = DIM == 2 && q >= 2 ? q + 1 : q;  // vx, vy, vz, vr, overlap
+#pragma unroll
+        for (int e0 = 0; e0 < 32; e0 += 4) {
+            const int e = e0 + (lane >> 3);
+            if (e < m && q < kC) {
+                const double v = RS[q * kT + e];
+                red_add(b.acc + (size_t)QI[e] * kAcc + slot, v);
+                red_add(b.acc + (size_t)QJ[e] * kAcc + slot, slot == 4 ? v : neg_bits(v));
+            }
+        }
+        __syncwarp();
+    };
 
     int cnt = 0;  // queued pairs of this warp (uniform over its lanes)
     const int nch = (np + 31) >> 5;
     const int wb = RES ? blockDim.x >> 5 : kW;  // warps of this block
-    for (int ch = RES ? w * vg + vb : vb * kW + w; ch < nch; ch += vg * wb) {
-        const int p = (ch << 5) + lane;
+    int p = ((RES ? w * vg + vb : vb * kW + w) << 5) + lane;
+    const int step = (vg * wb) << 5;
+    int i1 = 0, j1 = 0;  // the next chunk's pair, loaded a chunk ahead
+    if (p < np) {
+        i1 = PI[p];
+        j1 = PJ[p];
+    }
+    for (; (p >> 5) < nch; p += step) {
         bool over = false;
-        int i = 0, j = 0;
-        double dx = 0.0, dy = 0.0, dz = 0.0, r1 = 0.0, r2 = 0.0;
+        const int i = i1, j = j1;
+        long long ex = 0, ey = 0, ez = 0, q1 = 0, q2 = 0;
+        if (p + step < np) {
+            i1 = PI[p + step];
+            j1 = PJ[p + step];
+        }
         if (p < np) {
-            i = PI[p];
-            j = PJ[p];
             if (FLOW) {  // src/kernels.cu:191-207 (added for every pair)
                 double *aj = b.acc + (size_t)j * kAcc;
                 red_add(aj + 5, V0[i]);
@@ -331,48 +355,47 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
                 if (DIM == 3) red_add(aj + 7, V2[i]);
             }
             const double4_32a a = ld4(b.pred, i), q = ld4(b.pred, j);
-            r1 = DIM == 3 ? a.w : a.z;
-            r2 = DIM == 3 ? q.w : q.z;
-            // wrappedDifference, src/kernels.cu:1094-1114 (the FP64
-            // differences, exact, mostly on the integer pipe)
-            dx = sub_exact(a.x, q.x);
-            dy = sub_exact(a.y, q.y);
-            if (px) dx = min_image(dx, hx, Lx);
-            if (py) dy = min_image(dy, hy, Ly);
+            q1 = __double_as_longlong(DIM == 3 ? a.w : a.z);
+            q2 = __double_as_longlong(DIM == 3 ? q.w : q.z);
+            ex = __double_as_longlong(a.x) - __double_as_longlong(q.x);
+            ey = __double_as_longlong(a.y) - __double_as_longlong(q.y);
+            if (px) ex = image(ex, hx, Lx);
+            if (py) ey = image(ey, hy, Ly);
             if (DIM == 3) {
-                dz = sub_exact(a.z, q.z);
-                if (pz) dz = min_image(dz, hz, Lz);
+                ez = __double_as_longlong(a.z) - __double_as_longlong(q.z);
+                if (pz) ez = image(ez, hz, Lz);
             }
-            // overlap test (r1 + r2)^2 >= m: in FP32 on the exact differences
-            // (truncated, ~2^-21 relative) outside a 1e-5 guard band, by the
-            // FP64 test of the reference's sign inside it
-            const float fx = ff_f32(dx), fy = ff_f32(dy), fz = DIM == 3 ? ff_f32(dz) : 0.f;
+            // overlap test (r1 + r2)^2 >= d^2: in FP32 outside a 1e-5 guard
+            // band (the differences exact, ~2^-22 relative as FP32), else on
+            // the integers
+            const float fx = fix_len(ex), fy = fix_len(ey), fz = DIM == 3 ? fix_len(ez) : 0.f;
             float m32 = fx * fx;
             m32 = fmaf(fy, fy, m32);
             if (DIM == 3) m32 = fmaf(fz, fz, m32);
-            const float R32 = ff_f32(r1) + ff_f32(r2);
+            const long long R = q1 + q2;
+            const float R32 = fix_len(R);
             const float RR = R32 * R32;
             if (m32 < RR * (1.f - 1e-5f))
                 over = true;
             else if (!(m32 > RR * (1.f + 1e-5f)))
-                over = overlap_exact<DIM>(dx, dy, dz, r1, r2);
+                over = overlap_exact<DIM>(ex, ey, ez, llabs(R));
         }
         const unsigned mask = __ballot_sync(0xffffffffu, over);
         if (over) {
             const int e = cnt + __popc(mask & below);
             QI[e] = i;
             QJ[e] = j;
-            Q[0][e] = dx;
-            Q[1][e] = dy;
-            if (DIM == 3) Q[2][e] = dz;
-            Q[kR1][e] = r1;
-            Q[kR1 + 1][e] = r2;
+            Q[0][e] = ex;
+            Q[1][e] = ey;
+            if (DIM == 3) Q[2][e] = ez;
+            Q[kR1][e] = q1;
+            Q[kR1 + 1][e] = q2;
         }
         cnt += __popc(mask);
         __syncwarp();
         if (cnt >= 32) {  // a full warp of overlapping pairs
             process(lane);
-            __syncwarp();
+            scatter(32);
             cnt -= 32;
             if (lane < cnt) {
                 QI[lane] = QI[32 + lane];
@@ -384,185 +407,11 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         }
     }
     if (lane < cnt) process(lane);
+    scatter(cnt);
 
     pairs_fold<DIM, RES>(b, vb, vg, sAo, sAor, smem, rx, rsm);
 }
-CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs, (<DIM, GAS, FLOW>), __launch_bounds__(kBlock))
-
-
-// ------------------------------------------------------ pairs, float-float
-// CB_PRECISION_FP64_FF: the pair kernel of the FP64 form with its arithmetic
-// in float-float. Overlap velocities, pairwise gas flux and overlap areas
-// (pairwiseInteraction, src/kernels.cu:172-337). GB300 issues FP64 at 1/64 of
-// the FP32 rate, so apart from the three FP64 position differences
-// (wrappedDifference, src/kernels.cu:1094-1114) the pair arithmetic runs in
-// float-float (ff.cuh, ~2^-46 relative) on the FP32 and integer pipes, from
-// per-bubble float-float records (r, 1/r, r^2) written by k_predict. The
-// overlap test and the inside tests of the gas exchange are decided in
-// float-float unless the difference is within 2^-38 of its operands; then the
-// FP64 comparisons of the reference decide, so the classification of every
-// pair is the FP64 one.
-//
-// Each thread takes a run of kRun consecutive pairs (rows are grouped by i):
-// the i-side sums stay in float-float registers and go out once per row; the
-// j-side contributions go out per pair. Both are rounded to double on the
-// integer pipe and added to the FP64 accumulator rows with FP64 atomics.
-constexpr float kAmb = 0x1p-38f;
-
-
-template <int DIM, bool GAS, bool FLOW, bool RES = false>
-__device__ __forceinline__ void k_pairs_ff_body(const Bufs &b, const int vb, const int vg,
-                                                RunCtx *rx = nullptr, RunRed *rsm = nullptr) {
-    // a resident run has pairs for a fraction of the resident threads only
-    constexpr int kRun = RES ? 1 : 4;
-    __shared__ double smem[32];
-    const Ctrl *c = b.ctrl;
-    const DevConst &k = *b.k;
-    const int np = c->np;
-    const int *PI = b.ps[c->prole[PI0]];
-    const int *PJ = b.ps[c->prole[PJ0]];
-    const double *V0 = drow(b, c, RV0), *V1 = drow(b, c, RV1), *V2 = drow(b, c, RV2);
-    const float4 *REC = b.ffr;
-    const ff f0 = {k.f0_f, k.f0_l};
-    const bool px = !k.wall[0], py = !k.wall[1], pz = DIM == 3 && !k.wall[2];
-    const double hx = k.half_iv[0], hy = k.half_iv[1], hz = k.half_iv[2];
-    const double Lx = k.iv[0], Ly = k.iv[1], Lz = k.iv[2];
-    ff sAo = {0.f, 0.f}, sAor = {0.f, 0.f};
-    const int nrun = (np + kRun - 1) / kRun;
-    for (int g = first_item<RES>(vb, vg); g < nrun; g += vg * blockDim.x) {
-        const int p0 = g * kRun;
-        int cur = -1;
-        double4_32a a;
-        FfRec ra;
-        ff ax = {0.f, 0.f}, ay = ax, az = ax, ag = ax, ao = ax;
-        bool hit = false;
-        double vxi = 0.0, vyi = 0.0, vzi = 0.0;
-        auto flush = [&](int i) {
-            double *ai = b.acc + (size_t)i * kAcc;
-            add_d(ai + 0, ax);
-            add_d(ai + 1, ay);
-            if (DIM == 3) add_d(ai + 2, az);
-            if (GAS) {
-                add_d(ai + 3, ag);
-                add_d(ai + 4, ao);
-            }
-        };
-#pragma unroll 1  // one pair body: the unrolled run overflows the instruction cache
-        for (int t = 0; t < kRun; t++) {
-            if (p0 + t >= np) break;
-            const int i = PI[p0 + t], j = PJ[p0 + t];
-            if (i != cur) {
-                if (hit) flush(cur);
-                cur = i;
-                a = ld4(b.pred, i);
-                ra = ld_rec(REC, i);
-                ax = ay = az = ag = ao = ff{0.f, 0.f};
-                hit = false;
-                if (FLOW) {
-                    vxi = V0[i];
-                    vyi = V1[i];
-                    vzi = DIM == 3 ? V2[i] : 0.0;
-                }
-            }
-            double *aj = b.acc + (size_t)j * kAcc;
-            if (FLOW) {  // src/kernels.cu:191-207 (added for every pair)
-                atomicAdd(aj + 5, vxi);
-                atomicAdd(aj + 6, vyi);
-                if (DIM == 3) atomicAdd(aj + 7, vzi);
-            }
-            const double4_32a q = ld4(b.pred, j);
-            const FfRec rb = ld_rec(REC, j);
-            // wrappedDifference, src/kernels.cu:1094-1114 (FP64)
-            double dx = a.x - q.x, dy = a.y - q.y, dz = 0.0;
-            if (px) dx = min_image(dx, hx, Lx);
-            if (py) dy = min_image(dy, hy, Ly);
-            if (DIM == 3) {
-                dz = a.z - q.z;
-                if (pz) dz = min_image(dz, hz, Lz);
-            }
-            const ff X = ff_of(dx), Y = ff_of(dy), Z = ff_of(dz);
-            ff m = ff_add(ff_sqr(X), ff_sqr(Y));
-            if (DIM == 3) m = ff_add(m, ff_sqr(Z));
-            const ff R = ff_add(ra.r, rb.r);
-            const ff RR = ff_sqr(R);
-            const float dov = ff_diff_f(RR, m);
-            bool over = dov >= 0.f;
-            bool amb = fabsf(dov) <= kAmb * RR.h;
-            bool inside = false;
-            if (GAS) {
-                const float d1 = ff_diff_f(m, ra.rsq), d2 = ff_diff_f(m, rb.rsq);
-                inside = d1 < 0.f || d2 < 0.f;
-                amb |= fabsf(d1) <= kAmb * m.h || fabsf(d2) <= kAmb * m.h;
-            }
-            if (amb) {  // within 2^-38: the reference's FP64 tests decide
-                double m64 = dx * dx;
-                m64 = fma(dy, dy, m64);
-                if (DIM == 3) m64 = fma(dz, dz, m64);
-                const double r1 = DIM == 3 ? a.w : a.z, r2 = DIM == 3 ? q.w : q.z;
-                const double radii = r1 + r2;
-                over = nonneg_bits(fma(radii, radii, -m64));
-                if (GAS) {
-                    double r1sq, r2sq;
-                    if (DIM == 3) {
-                        r1sq = b.invr[2 * (size_t)i + 1];
-                        r2sq = b.invr[2 * (size_t)j + 1];
-                    } else {
-                        r1sq = r1 * r1;
-                        r2sq = r2 * r2;
-                    }
-                    inside = less_nonneg(m64, r1sq) || less_nonneg(m64, r2sq);
-                }
-            }
-            if (!over) continue;
-            // velocity f0 d (1/|d| - 1/(r1 + r2)), src/kernels.cu:218-233
-            const ff rs = ff_rsqrt(m);
-            const ff s = ff_mul(f0, ff_sub(rs, ff_rcp(R)));
-            const ff fx = ff_mul(X, s), fy = ff_mul(Y, s);
-            ax = ff_add(ax, fx);
-            ay = ff_add(ay, fy);
-            add_d(aj + 0, ff_neg(fx));
-            add_d(aj + 1, ff_neg(fy));
-            if (DIM == 3) {
-                const ff fz = ff_mul(Z, s);
-                az = ff_add(az, fz);
-                add_d(aj + 2, ff_neg(fz));
-            }
-            hit = true;
-            if (GAS) {  // pairwise gas exchange, src/kernels.cu:236-280
-                // chord: r2^2 - t^2 / m with t = (r2^2 - r1^2 + m) / 2, as
-                // r2^2 - w^2 / 4 with w = (r2^2 - r1^2 + m) / |d|; the
-                // overlap area in units of ov_unit (pi in 3D, 2 in 2D)
-                ff oa;
-                if (inside) {
-                    if (DIM == 3)
-                        oa = ff_less(ra.rsq, rb.rsq) ? ra.rsq : rb.rsq;
-                    else
-                        oa = ff_less(ra.r, rb.r) ? ra.r : rb.r;
-                } else {
-                    const ff w = ff_mul(ff_add(ff_sub(rb.rsq, ra.rsq), m), rs);
-                    const ff v = ff_abs(ff_sub(rb.rsq, ff_scale(ff_sqr(w), 0.25f)));
-                    oa = DIM == 3 ? v : ff_sqrt(v);
-                }
-                const ff gf = ff_mul(oa, ff_sub(rb.inv, ra.inv));
-                ag = ff_add(ag, gf);
-                ao = ff_add(ao, oa);
-                add_d(aj + 3, ff_neg(gf));
-                add_d(aj + 4, oa);
-                sAo = ff_add(sAo, oa);
-                sAor = ff_add(sAor, ff_mul(oa, ff_add(ra.inv, rb.inv)));
-            }
-            if (FLOW) {  // src/kernels.cu:298-307 (overlapping pairs only)
-                double *ai = b.acc + (size_t)i * kAcc;
-                atomicAdd(ai + 5, V0[j]);
-                atomicAdd(ai + 6, V1[j]);
-                if (DIM == 3) atomicAdd(ai + 7, V2[j]);
-            }
-        }
-        if (hit) flush(cur);
-    }
-    pairs_fold<DIM, RES>(b, vb, vg, ff_to_double(sAo), ff_to_double(sAor), smem, rx, rsm);
-}
-CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs_ff, (<DIM, GAS, FLOW>), __launch_bounds__(kBlock, 3))
+CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs, (<DIM, GAS, FLOW>), __launch_bounds__(kBlock, 4))
 
 
 // ---------------------------------------------------------------- correct
@@ -700,8 +549,8 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         if (gas || flow) a1 = reinterpret_cast<const double4_32a *>(acc)[1];
         double vpx = a0.x, vpy = a0.y, vpz = a0.z, vpr = a0.w;
         const double ov = a1.x;
-        const double4_32a p = ld4(b.pred, i);
-        const double xp = p.x, yp = p.y, zp = DIM == 3 ? p.z : 0.0, rp = DIM == 3 ? p.w : p.z;
+        const State p = ld_state<DIM>(b, i, k.fix_b);
+        const double xp = p.x, yp = p.y, zp = p.z, rp = p.r;
         if (flow | shear | k.any_wall) {
             const Vel3 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz, xp, yp, zp,
                                                   rp, a1.y, a1.z, a1.w, flow ? NN[i] : 0);
@@ -737,7 +586,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 inv = e.x;
                 area = 4.0 * e.y;
             } else {
-                inv = p.w;
+                inv = p.inv;
                 area = kPi * rp;
             }
             double vr = mfa - inv;
@@ -830,7 +679,7 @@ CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBloc
 // Attempts of a small foam inside one cooperative launch (see common.cuh).
 // Measured against the launch per phase, one GB300: see kRunCapacity
 // (context.cu).
-template <int DIM, bool GAS, bool FLOW, bool FF>
+template <int DIM, bool GAS, bool FLOW>
 __global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, const Bufs *foams,
                                                     const RunBlock *map, Ctrl *mirror,
                                                     long long n_steps, int threads) {
@@ -852,10 +701,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, const Bufs *foams,
         run_begin(&rx, attempts);
         k_predict_body<DIM, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
-        if (FF)
-            k_pairs_ff_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
-        else
-            k_pairs_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
+        k_pairs_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
         k_correct_body<DIM, true>(b, vb, vg, &rx, &rsm);
     } while (run_more(&rs, ++attempts));
@@ -875,35 +721,22 @@ __global__ void __launch_bounds__(kBlock) k_boot(Bufs b, int phase) {
                  *R = drow(b, c, RR);
     double *O0 = drow(b, c, RVO0), *O1 = drow(b, c, RVO1), *O2 = drow(b, c, RVO2),
            *O3 = drow(b, c, RVO3), *PATH = drow(b, c, RPATH);
-    double4_32a *P = reinterpret_cast<double4_32a *>(b.pred);
+    const int fixb = b.k->fix_b;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double *acc = b.acc + (size_t)i * kAcc;
         if (phase == 0) {
-            double4_32a p;
             const double r = R[i];
-            p.x = X[i];
-            p.y = Y[i];
             const double inv = 1.0 / r, rsq = r * r;
-            if (b.ffr) st_rec(b.ffr, i, r, inv, rsq);
-            if (DIM == 3) {
-                p.z = Z[i];
-                p.w = r;
-                reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
-            } else {
-                p.z = r;
-                p.w = inv;
-            }
-            P[i] = p;
+            if (DIM == 3) reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
+            st_state<DIM>(b, i, X[i], Y[i], DIM == 3 ? Z[i] : 0.0, r, inv, fixb);
             O0[i] = O1[i] = O2[i] = O3[i] = 0.0;
             PATH[i] = 0.0;
         } else {
             double4_32a a = reinterpret_cast<double4_32a *>(acc)[0];
             if (phase == 1) {
-                double4_32a p = P[i];
-                p.x += a.x * ts;
-                p.y += a.y * ts;
-                if (DIM == 3) p.z += a.z * ts;
-                P[i] = p;
+                const State p = ld_state<DIM>(b, i, fixb);
+                st_state<DIM>(b, i, p.x + a.x * ts, p.y + a.y * ts, p.z + a.z * ts, p.r,
+                                  p.inv, fixb);
             } else {
                 O0[i] = a.x;
                 O1[i] = a.y;
@@ -991,15 +824,10 @@ void launch_predict(const Launch &l, const Bufs &b, int dim) {
 }
 
 // mode bits: 1 = gas exchange, 2 = flow. mode 0 is the bootstrap form.
-void launch_pairs(const Launch &l, const Bufs &b, int dim, int mode, bool ff) {
+void launch_pairs(const Launch &l, const Bufs &b, int dim, int mode) {
     const bool gas = mode & 1, flow = mode & 2;
-#define CB_PAIRS(D, G, F)                                                                     \
-    do {                                                                                      \
-        if (ff)                                                                               \
-            CB_LAUNCH(l, k_pairs_ff, (<D, G, F>), wave_grid(k_pairs_ff<D, G, F>, l, l.pair_bps), b);      \
-        else                                                                                  \
-            CB_LAUNCH(l, k_pairs, (<D, G, F>), wave_grid(k_pairs<D, G, F>, l, l.pair_bps), b);            \
-    } while (0)
+#define CB_PAIRS(D, G, F) \
+    CB_LAUNCH(l, k_pairs, (<D, G, F>), wave_grid(k_pairs<D, G, F>, l, l.pair_bps), b)
     if (dim == 3) {
         if (gas && flow) CB_PAIRS(3, true, true);
         else if (gas) CB_PAIRS(3, true, false);
@@ -1021,27 +849,19 @@ void launch_correct(const Launch &l, const Bufs &b, int dim) {
         CB_LAUNCH(l, k_correct, (<2>), wave_grid(k_correct<2>, l, l.step_bps), b);
 }
 
-void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode, bool ff) {
+void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode) {
     const bool gas = mode & 1, flow = mode & 2;
-#define CB_RUN(D, G, F)                                  \
-    do {                                                 \
-        if (ff)                                          \
-            launch_coop(k_run<D, G, F, true>, r, b);     \
-        else                                             \
-            launch_coop(k_run<D, G, F, false>, r, b);    \
-    } while (0)
     if (dim == 3) {
-        if (gas && flow) CB_RUN(3, true, true);
-        else if (gas) CB_RUN(3, true, false);
-        else if (flow) CB_RUN(3, false, true);
-        else CB_RUN(3, false, false);
+        if (gas && flow) launch_coop(k_run<3, true, true>, r, b);
+        else if (gas) launch_coop(k_run<3, true, false>, r, b);
+        else if (flow) launch_coop(k_run<3, false, true>, r, b);
+        else launch_coop(k_run<3, false, false>, r, b);
     } else {
-        if (gas && flow) CB_RUN(2, true, true);
-        else if (gas) CB_RUN(2, true, false);
-        else if (flow) CB_RUN(2, false, true);
-        else CB_RUN(2, false, false);
+        if (gas && flow) launch_coop(k_run<2, true, true>, r, b);
+        else if (gas) launch_coop(k_run<2, true, false>, r, b);
+        else if (flow) launch_coop(k_run<2, false, true>, r, b);
+        else launch_coop(k_run<2, false, false>, r, b);
     }
-#undef CB_RUN
 }
 
 void launch_boot(const Launch &l, const Bufs &b, int dim, int phase) {

@@ -42,13 +42,15 @@ extern "C" {
 #define CB_ERR_NO_DEVICE 7        /* no CUDA device / extension unusable      */
 #define CB_ERR_STATE 8            /* call made in the wrong order             */
 
-#define CB_PRECISION_FP64 0  /* plain FP64 form (reference arithmetic)        */
+#define CB_PRECISION_FP64 0  /* FP64 form (pair terms in 64-bit fixed point, to
+                                within the rounding of FP64)                  */
 #define CB_PRECISION_MIXED 1 /* FP32 pair geometry on exact 64-bit fixed-point
                                 differences, FP64 positions/volume/error     */
-#define CB_PRECISION_FP64_FF 2 /* the FP64 form with its pair terms (distance,
-                                velocities, gas flux, overlap areas) in
-                                float-float (two FP32, ~2^-46 relative) on the
-                                FP32 pipe; FP64 state, update and sums       */
+#define CB_PRECISION_FP64_FF 2 /* FP64 state, update and sums with the pair terms
+                                off the FP64 pipe. Float-float (~2^-46) in
+                                earlier versions; the FP64 form's own pair
+                                terms are fixed point now, more exact and
+                                faster, and this form is the same           */
 
 /* ------------------------------------------------------------ constants */
 /* Mirrors `Constants` (src/data_definitions.h:183-225) plus the host-side
@@ -67,7 +69,10 @@ typedef struct cb_config {
     int32_t max_attempts;    /* reject-loop cap per step; 0 = 64           */
     int32_t precision;       /* CB_PRECISION_*                             */
     int32_t use_graph;       /* 1 = run cb_integrate as one CUDA graph with
-                                device-side conditional loops              */
+                                device-side conditional loops (contexts
+                                beyond 4 10^5 (3D) / 6 10^5 (2D) bubbles;
+                                smaller ones run their attempts inside one
+                                cooperative kernel either way)             */
     double lbb[3];           /* lower back bottom corner of the box        */
     double tfr[3];           /* top front right corner of the box          */
     double flow_lbb[3];
