@@ -163,8 +163,7 @@ struct Ctrl {
 // What a resident run's blocks (below) reduce into and wait on, in global
 // memory: zero between launches.
 struct RunAcc {
-    double sum[2];       // predict: area, area over radius
-    double osum[2];      // pairs: overlap area, overlap area over radius
+    double psum[4];      // overlap area, overlap area over radius; area, area over radius
     double csum[5];      // correct: volume; mixed form: the candidates' sums
     long long cmax[3];   // correct: error, radius, expansion (bits of doubles >= 0)
     int cnt[2];          // correct: deletions, non-finite values
@@ -527,93 +526,129 @@ __device__ __forceinline__ void set_cond(unsigned long long h, unsigned int v) {
     cudaGraphSetConditional((cudaGraphConditionalHandle)h, v);
 }
 
+// Reduced values of one attempt.
+struct AttemptResult {
+    double err, rad, exp, vol;
+    int del, bad;
+};
+
 // step(): accept / reject and the new dt (src/simulator.cu:239-246); on
 // accept, integrate()'s rotation and clock (src/simulator.cu:258-314) and the
-// delete / search decisions (:316-334). Run by one thread of the last block.
+// delete / search decisions (:316-334), in three parts that read nothing the
+// others write: what decides the next attempt, the clock, the buffer roles.
+struct AttemptFate {
+    int too_large, increase, accept;
+    double dt;  // of the next attempt
+};
+__device__ __forceinline__ AttemptFate attempt_fate(bool status_ok, bool no_accept,
+                                                    const DevConst &k, double dt,
+                                                    const AttemptResult &r) {
+    AttemptFate f;
+    f.too_large = r.err > k.tol;
+    f.increase = r.err < 0.45 * k.tol && dt < 10;
+    f.dt = f.too_large ? dt * 0.37 : (f.increase ? dt * 1.269 : dt);
+    f.accept = !f.too_large && !no_accept && status_ok && !(r.bad > 0 || isnan(r.err));
+    return f;
+}
+
 template <int DIM>
-__device__ void finish_attempt(Ctrl *c, const DevConst &k, double fErr, double fRad,
-                               double fExp, double fVol, double fDel, double fBad) {
-    const int gas = c->use_gas, path = c->inc_path;
-    const int n = c->n;
-    c->done[DC_CORRECT] = 0;
-    c->max_err = fErr;
-    c->max_rad = fRad;
-    c->max_exp = fExp;
-    c->vol_new = fVol;
-    c->ndel = gas ? (int)fDel : 0;
+__device__ __forceinline__ void attempt_decide(Ctrl *c, const DevConst &k, const AttemptResult &r,
+                                               const AttemptFate &f) {
+    const int gas = c->use_gas;
+    c->max_err = r.err;
+    c->max_rad = r.rad;
+    c->max_exp = r.exp;
+    c->vol_new = r.vol;
+    c->ndel = gas ? r.del : 0;
     c->attempts += 1;
     c->attempts_this_step += 1;
-    const double tol = k.tol;
-    const int too_large = fErr > tol;
-    const int increase = fErr < 0.45 * tol && c->dt < 10;
-    if (too_large)
-        c->dt *= 0.37;
-    else if (increase)
-        c->dt *= 1.269;
-    c->too_large = too_large;
+    c->dt = f.dt;
+    c->too_large = f.too_large;
     if (k.mixed) {  // speculative prediction of the next attempt (step_mixed.cu)
-        const int use = !too_large && !c->no_accept;
+        const int use = !f.too_large && !c->no_accept;
         c->pred_ready = use;
-        c->pred_slot = use ? (increase ? 2 : 1) : 0;
+        c->pred_slot = use ? (f.increase ? 2 : 1) : 0;
         if (use) {
-            c->sumA = c->cand_sumA[increase ? 1 : 0];
-            c->sumAr = c->cand_sumAr[increase ? 1 : 0];
+            c->sumA = c->cand_sumA[f.increase ? 1 : 0];
+            c->sumAr = c->cand_sumAr[f.increase ? 1 : 0];
         }
         c->cand_sumA[0] = c->cand_sumA[1] = c->cand_sumAr[0] = c->cand_sumAr[1] = 0.0;
     }
-    if (fBad > 0.0 || isnan(fErr)) c->status = CB_ERR_NONFINITE;
+    if (r.bad > 0 || isnan(r.err)) c->status = CB_ERR_NONFINITE;
     c->need_delete = 0;
     c->need_search = 0;
-    if (too_large && c->status == CB_OK) {
+    if (f.too_large && c->status == CB_OK) {
         if (c->attempts_this_step >= k.max_attempts) c->status = CB_ERR_MAX_ATTEMPTS;
-        if (c->dt < 1e-300) c->status = CB_ERR_DT_UNDERFLOW;
+        if (f.dt < 1e-300) c->status = CB_ERR_DT_UNDERFLOW;
     }
-    if (!too_large && !c->no_accept && c->status == CB_OK) {
-        int *r = c->drole;
-        for (int a = 0; a < DIM; a++) {
-            swap_role(r, RX + a, RXN + a);
-            const int old = r[RVO0 + a];
-            r[RVO0 + a] = r[RV0 + a];
-            r[RV0 + a] = r[RVP0 + a];
-            r[RVP0 + a] = old;
-        }
-        if (gas) {
-            swap_role(r, RR, RRN);
-            const int old = r[RVO3];
-            r[RVO3] = r[RV3];
-            r[RV3] = r[RVP3];
-            r[RVP3] = old;
-        }
-        if (path) swap_role(r, RPATH, RPATHN);
+    if (f.accept) {
         c->steps += 1;
-        c->bubble_steps += n;
+        c->bubble_steps += c->n;
         c->attempts_this_step = 0;
-        // time accumulator, src/simulator.cu:311-314 (adds the updated dt)
-        c->tfrac += c->dt;
-        c->tint += (unsigned long long)c->tfrac;
-        c->tfrac = c->tfrac - (double)(unsigned long long)c->tfrac;
-        c->dt_min = fmin(c->dt_min, c->dt);
-        c->dt_max = fmax(c->dt_max, c->dt);
-        c->dt_sum += c->dt;
         if (gas) {
-            c->max_bubble_radius = fRad;
+            c->max_bubble_radius = r.rad;
             c->need_delete = c->ndel > 0;
         }
-        c->need_search = fExp >= 0.5 * k.skin;
-        if (c->stop_on) {
-            const int left = n - (c->need_delete ? c->ndel : 0);
-            const int time_up = c->tint > c->stop_tint ||
-                                (c->tint == c->stop_tint && c->tfrac >= c->stop_tfrac);
-            c->stop_hit = time_up || left <= c->stop_nmin ||
-                          (gas && c->max_bubble_radius >= c->stop_rmax);
-        }
+        c->need_search = r.exp >= 0.5 * k.skin;
     }
+}
+
+// Time accumulator, src/simulator.cu:311-314 (adds the updated dt), the dt
+// statistics and the stop conditions.
+__device__ __forceinline__ void attempt_clock(Ctrl *c, const AttemptResult &r,
+                                              const AttemptFate &f) {
+    if (!f.accept) return;
+    double t = c->tfrac + f.dt;
+    const unsigned long long whole = (unsigned long long)t;
+    const unsigned long long ti = c->tint + whole;
+    t -= (double)whole;
+    c->tfrac = t;
+    c->tint = ti;
+    c->dt_min = fmin(c->dt_min, f.dt);
+    c->dt_max = fmax(c->dt_max, f.dt);
+    c->dt_sum += f.dt;
+    if (c->stop_on) {
+        const int left = c->n - (c->use_gas ? r.del : 0);
+        const int time_up = ti > c->stop_tint || (ti == c->stop_tint && t >= c->stop_tfrac);
+        c->stop_hit = time_up || left <= c->stop_nmin || (c->use_gas && r.rad >= c->stop_rmax);
+    }
+}
+
+template <int DIM>
+__device__ __forceinline__ void attempt_rotate(Ctrl *c, const AttemptFate &f) {
+    if (!f.accept) return;
+    int *r = c->drole;
+    for (int a = 0; a < DIM; a++) {
+        swap_role(r, RX + a, RXN + a);
+        const int old = r[RVO0 + a];
+        r[RVO0 + a] = r[RV0 + a];
+        r[RV0 + a] = r[RVP0 + a];
+        r[RVP0 + a] = old;
+    }
+    if (c->use_gas) {
+        swap_role(r, RR, RRN);
+        const int old = r[RVO3];
+        r[RVO3] = r[RV3];
+        r[RV3] = r[RVP3];
+        r[RVP3] = old;
+    }
+    if (c->inc_path) swap_role(r, RPATH, RPATHN);
+}
+
+// All of it by one thread of the last block, and the graph's conditions.
+template <int DIM>
+__device__ void finish_attempt(Ctrl *c, const DevConst &k, const AttemptResult &r) {
+    c->done[DC_CORRECT] = 0;
+    const AttemptFate f = attempt_fate(c->status == CB_OK, c->no_accept, k, c->dt, r);
+    attempt_decide<DIM>(c, k, r, f);
+    attempt_clock(c, r, f);
+    attempt_rotate<DIM>(c, f);
     if (c->graph_mode) {
         const int ok = c->status == CB_OK;
-        const int accepted = !too_large;
+        const int accepted = !f.too_large;
         set_cond(c->h_delete, ok && accepted && c->need_delete);
         set_cond(c->h_search, ok && accepted && c->need_search);
-        const int more = ok && (too_large || (c->steps < c->steps_target && !c->stop_hit));
+        const int more = ok && (f.too_large || (c->steps < c->steps_target && !c->stop_hit));
         set_cond(c->h_loop, more);
         // the last iteration's removal / search are decided above; clearing
         // the mode here spares the host a control-block write per launch
@@ -642,6 +677,9 @@ struct RunCtx {
     unsigned vg;
     int *failed;     // shared
     int threads;     // of the correct kernel in a launch per phase (mixed form)
+    // this thread's share of the prediction's sums, reduced with the pair
+    // phase's (FP64 form)
+    double sA, sAr;
 };
 constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: seconds in all
 constexpr int kRunMaxAttempts = 1 << 15;   // per launch (bounds the arrival counter)
@@ -675,8 +713,9 @@ __device__ __forceinline__ int first_item(int vb, int vg) {
                : (int)(vb * blockDim.x + threadIdx.x);
 }
 
-// The block's sums (FP64), maxima (bit patterns of doubles >= 0) and counts
-// into the run's global accumulators: warp by warp, across the warps through
+// The block's sums (of values >= 0; the mixed form's in FP32 inside a warp),
+// maxima (bit patterns of doubles >= 0) and counts into the run's global
+// accumulators: warp by warp, across the warps through
 // shared memory, then one reduction each. Read after the next run_barrier.
 // (Partials per block folded by every block after the barrier, in a fixed
 // order, took 1900-3900 cycles of latency there against ~700 for reading the
@@ -686,10 +725,31 @@ struct RunRed {
     long long m[3][kBlock / 32];
     int c[2][kBlock / 32];
 };
+static __device__ __noinline__ double warp_sum_slow(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// Sum over the warp of doubles >= 0 without FP64 arithmetic (five dependent
+// FP64 adds per warp keep the pipe busy for 16 cycles each, and every warp of
+// the SM queues for it): each value in units of 2^-57 of the largest one's
+// binade, exact to half a unit, summed in three slices of 19 bits. Infinities
+// and NaN take the FP64 sum.
 __device__ __forceinline__ double warp_sum(double v) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, (unsigned)__double2hiint(v)) >> 20;
+    if (m == 0u) return 0.0;  // zeros (subnormals count as such)
+    if (m >= 0x7feu || m < 64u) return warp_sum_slow(v);
+    const int B = 1079 - (int)m;  // v 2^B < 2^57
+    const unsigned long long q = (unsigned long long)fx_from_double(v, B);
+    const unsigned a = __reduce_add_sync(0xffffffffu, (unsigned)q & 0x7ffffu);
+    const unsigned b = __reduce_add_sync(0xffffffffu, (unsigned)(q >> 19) & 0x7ffffu);
+    const unsigned c = __reduce_add_sync(0xffffffffu, (unsigned)(q >> 38));
+    return fx_to_double(((unsigned long long)c << 38) + ((unsigned long long)b << 19) + a, -B);
+}
+__device__ __forceinline__ double warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
+    return (double)v;
 }
 // Maximum over the warp of bit patterns >= 0: the high words' maximum, then
 // the low words of the lanes that hold it (negative patterns lose against 0).
@@ -700,15 +760,20 @@ __device__ __forceinline__ long long warp_max_bits(long long v) {
     const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
     return (long long)(((unsigned long long)mh << 32) | ml);
 }
-template <int NS, int NM, int NC>
-__device__ __forceinline__ void run_reduce(const double *s, const long long *m, const int *c,
-                                           double *gs, long long *gm, int *gc, RunRed *sm) {
+// NS sums of type T and NF FP32 ones to gs[0 ... NS + NF), NM maxima, NC counts.
+template <int NS, int NM, int NC, int NF = 0, typename T>
+__device__ __forceinline__ void run_reduce(const T *s, const long long *m, const int *c,
+                                           double *gs, long long *gm, int *gc, RunRed *sm,
+                                           const float *sf = nullptr) {
+    constexpr int NA = NS + NF;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double ws[NS];
+    double ws[NA];
     long long wm[NM > 0 ? NM : 1];
     int wc[NC > 0 ? NC : 1];
 #pragma unroll
     for (int q = 0; q < NS; q++) ws[q] = warp_sum(s[q]);
+#pragma unroll
+    for (int q = 0; q < NF; q++) ws[NS + q] = warp_sum(sf[q]);
 #pragma unroll
     for (int q = 0; q < NM; q++) wm[q] = warp_max_bits(m[q]);
 #pragma unroll
@@ -716,7 +781,7 @@ __device__ __forceinline__ void run_reduce(const double *s, const long long *m, 
     __syncthreads();
     if (lane == 0) {
 #pragma unroll
-        for (int q = 0; q < NS; q++) sm->s[q][warp] = ws[q];
+        for (int q = 0; q < NA; q++) sm->s[q][warp] = ws[q];
 #pragma unroll
         for (int q = 0; q < NM; q++) sm->m[q][warp] = wm[q];
 #pragma unroll
@@ -724,7 +789,7 @@ __device__ __forceinline__ void run_reduce(const double *s, const long long *m, 
     }
     __syncthreads();
     const int t = threadIdx.x;
-    if (t < NS) {
+    if (t < NA) {
         double v[kBlock / 32];
 #pragma unroll
         for (int w = 0; w < kBlock / 32; w++) v[w] = w < nw ? sm->s[t][w] : 0.0;
@@ -732,15 +797,15 @@ __device__ __forceinline__ void run_reduce(const double *s, const long long *m, 
 #pragma unroll
             for (int w = 0; w < 4; w++) v[w] += v[w + 4];
         const double r = (v[0] + v[1]) + (v[2] + v[3]);
-        if (r != 0.0) atomicAdd(gs + t, r);
-    } else if (t < NS + NM) {
+        if (__double_as_longlong(r)) atomicAdd(gs + t, r);
+    } else if (t < NA + NM) {
         long long r = 0;
-        for (int w = 0; w < nw; w++) r = max(r, sm->m[t - NS][w]);
-        if (r) atomicMax(gm + (t - NS), r);
-    } else if (t < NS + NM + NC) {
+        for (int w = 0; w < nw; w++) r = max(r, sm->m[t - NA][w]);
+        if (r) atomicMax(gm + (t - NA), r);
+    } else if (t < NA + NM + NC) {
         int r = 0;
-        for (int w = 0; w < nw; w++) r += sm->c[t - NS - NM][w];
-        if (r) atomicAdd(gc + (t - NS - NM), r);
+        for (int w = 0; w < nw; w++) r += sm->c[t - NA - NM][w];
+        if (r) atomicAdd(gc + (t - NA - NM), r);
     }
 }
 
@@ -784,6 +849,34 @@ __device__ __forceinline__ void run_enter(RunShared *s, Bufs &b, long long n_ste
     b.ds = s->ds;
     b.is = s->is;
     b.ps = s->ps;
+}
+
+// After the correct phase's barrier: the attempt's reduced values and what
+// follows from them, by two threads of different warps (one after the other
+// in one thread they took 1700 cycles of ~27,000 of an attempt). dt is the
+// attempt's; the status is CB_OK and no_accept 0 in a run. `extra` runs in the
+// first thread before the decision.
+template <int DIM, typename F>
+__device__ __forceinline__ void run_finish(Ctrl *c, const DevConst &k, const RunAcc *g, double dt,
+                                           F extra) {
+    if (threadIdx.x == 0 || threadIdx.x == 32) {
+        AttemptResult r;
+        r.err = __longlong_as_double(__ldcg(&g->cmax[0]));
+        r.rad = __longlong_as_double(__ldcg(&g->cmax[1]));
+        r.exp = __longlong_as_double(__ldcg(&g->cmax[2]));
+        r.vol = __ldcg(&g->csum[0]);
+        r.del = __ldcg(&g->cnt[0]);
+        r.bad = __ldcg(&g->cnt[1]);
+        const AttemptFate f = attempt_fate(true, false, k, dt, r);
+        if (threadIdx.x == 0) {
+            extra();
+            attempt_decide<DIM>(c, k, r, f);
+        } else {
+            attempt_rotate<DIM>(c, f);
+            attempt_clock(c, r, f);
+        }
+    }
+    __syncthreads();
 }
 
 // Whether the next attempt runs in this launch (uniform over all blocks).

@@ -87,8 +87,18 @@ CB_HD double fx_to_double(uint64_t v, int e2, uint32_t sign = 0u) {
     const uint64_t b = ((uint64_t)(uint32_t)(1085 - lz + e2) << 52) + m;
     return ff_mkd((uint32_t)(b >> 32) | sign, (uint32_t)b);
 }
+// The same for values often below 2^32 (no call).
+CB_HD double fx_to_double_any(uint64_t v, int e2, uint32_t sign = 0u) {
+    if (v == 0) return 0.0;
+    const int lz = fx_clz(v);
+    const uint64_t n = v << lz;
+    const uint64_t m = (n >> 11) + ((n >> 10) & 1u);
+    const uint64_t b = ((uint64_t)(uint32_t)(1085 - lz + e2) << 52) + m;
+    return ff_mkd((uint32_t)(b >> 32) | sign, (uint32_t)b);
+}
 CB_HD double fx_to_double_signed(int64_t v, int e2) {
-    return v < 0 ? fx_to_double((uint64_t)-v, e2, 0x80000000u) : fx_to_double((uint64_t)v, e2);
+    return v < 0 ? fx_to_double_any((uint64_t)-v, e2, 0x80000000u)
+                 : fx_to_double_any((uint64_t)v, e2);
 }
 
 // The two halves of v': v' = h 2^32 + 2 l (+ its lowest bit), 0 <= l < 2^31.
@@ -102,6 +112,25 @@ CB_HD FxHalves fx_split(int64_t v) {
 CB_HD int64_t fx_square(int64_t v) {
     const FxHalves a = fx_split(v);
     return (int64_t)a.h * a.h + (((int64_t)a.h * a.l) >> 30);
+}
+
+CB_HD uint64_t fx_abs(int64_t v) { return (uint64_t)(v < 0 ? -v : v); }
+
+// |(x, y, z)| of integers in units 2^-B: squares normalised to the largest
+// component (2^-58), the root in float-float (~2^-46), no FP64 instruction.
+template <int DIM>
+CB_HD double fx_norm(int64_t x, int64_t y, int64_t z, int B) {
+    const uint64_t any = fx_abs(x) | fx_abs(y) | (DIM == 3 ? fx_abs(z) : 0u);
+    if (any == 0) return 0.0;
+    const int lz = fx_clz(any), s = lz > 2 ? lz - 2 : 0;  // components below 2^62
+    uint64_t M = (uint64_t)fx_square(x << s) + (uint64_t)fx_square(y << s);
+    if (DIM == 3) M += (uint64_t)fx_square(z << s);  // |v|^2 2^(2 s - 64), in [2^58, 2^62)
+    const int t = fx_clz(M) & ~1;  // to [2^62, 2^64): 48 bits keep 2^-47
+    M <<= t;
+    const float h = (float)(uint32_t)(M >> 40) * 0x1p24f,
+                l = (float)(((uint32_t)(M >> 16) & 0xffffffu) + ((uint32_t)(M >> 15) & 1u));
+    const double r = ff_to_double(ff_sqrt(fast_two_sum(h, l)));  // sqrt(M) / 2^8
+    return ff_mkd(ff_dhi(r) + ((uint32_t)(40 - s - t / 2 - B) << 20), ff_dlo(r));
 }
 
 // Two words of a 64-bit integer as FP32 (~2^-24 relative).

@@ -90,9 +90,9 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
     }
     if (DIM == 2) sAr = (double)na;
     constexpr double kArea = DIM == 3 ? 4.0 * kPi : 2.0 * kPi;
-    if (RES) {  // the sums are read after the pair phase
-        const double v[2] = {sA, sAr};
-        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->sum, nullptr, nullptr, rsm);
+    if (RES) {  // the sums are reduced with the pair phase's
+        rx->sA = sA;
+        rx->sAr = sAr;
         run_barrier(rx);
         return;
     }
@@ -156,19 +156,30 @@ __host__ __device__ constexpr double ov_unit(int dim) { return dim == 3 ? kPi : 
 template <int DIM, bool RES>
 __device__ __forceinline__ void pairs_fold(const Bufs &b, const int vb, const int vg, double sAo,
                                            double sAor, double *smem, RunCtx *rx, RunRed *rsm) {
-    double fAo, fAor;
+    double fAo = 0.0, fAor = 0.0;
     if (RES) {
-        const double v[2] = {sAo, sAor};
-        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->osum, nullptr, nullptr, rsm);
+        const double v[4] = {sAo, sAor, rx->sA, rx->sAr};
+        run_reduce<4, 0, 0>(v, nullptr, nullptr, rx->acc->psum, nullptr, nullptr, rsm);
         run_barrier(rx);
         run_clear_other(rx, vb);
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 || threadIdx.x == 32) {  // the two divisions in two warps
             constexpr double kArea = DIM == 3 ? 4.0 * kPi : 2.0 * kPi;
-            fAo = __ldcg(&rx->acc->osum[0]);
-            fAor = __ldcg(&rx->acc->osum[1]);
-            b.ctrl->sumA = kArea * __ldcg(&rx->acc->sum[0]);
-            b.ctrl->sumAr = kArea * __ldcg(&rx->acc->sum[1]);
+            Ctrl *cc = b.ctrl;
+            const double sumA = kArea * __ldcg(&rx->acc->psum[2]);
+            if (threadIdx.x == 32) {
+                cc->mfb = b.k->kappa * b.k->ain * (double)cc->n / sumA;
+            } else {
+                const double sumAr = kArea * __ldcg(&rx->acc->psum[3]);
+                const double sumAo = (2.0 * ov_unit(DIM)) * __ldcg(&rx->acc->psum[0]);
+                const double sumAor = ov_unit(DIM) * __ldcg(&rx->acc->psum[1]);
+                cc->mfa = (sumAr - sumAor) / (sumA - sumAo);
+                cc->sumA = sumA;
+                cc->sumAr = sumAr;
+                cc->sumAo = sumAo;
+                cc->sumAor = sumAor;
+            }
         }
+        return;
     } else {
         const double tAo = block_reduce(sAo, OpSum(), smem);
         const double tAor = block_reduce(sAor, OpSum(), smem);
@@ -491,19 +502,18 @@ static __device__ __noinline__ Vel3 boundary_velocity(const DevConst &k, int flo
     return {vpx, vpy, vpz};
 }
 
-// |(a, b, c)| of exact FP64 differences of nearby positions: squares, sum
-// and root in float-float (~2^-46), no FP64 instruction.
-static __device__ __noinline__ double norm_slow(double s) { return s > 0.0 ? sqrt(s) : 0.0; }
-template <int DIM>
-__device__ __forceinline__ double norm_ffd(double a, double b, double c) {
-    ff s = ff_add(ff_sqr(ff_of(a)), ff_sqr(ff_of(b)));
-    if (DIM == 3) s = ff_add(s, ff_sqr(ff_of(c)));
-    if (!(s.h > 0x1p-100f && s.h < 0x1p100f)) {
-        double d = a * a + b * b;
-        if (DIM == 3) d += c * c;
-        return norm_slow(d);
-    }
-    return ff_to_double(ff_sqrt(s));
+// FP64 issue and latency bound in its first forms (46 FP64 instructions a
+// bubble, 105 us at 3D, N = 10^6). The predictor-corrector error, the
+// expansion since the last search and the path increment are differences of
+// nearby positions: they are taken in the fixed point of the prediction
+// (exact; the corrected and saved positions are converted on the integer
+// pipe), which leaves the updates, the gas exchange and the volume to FP64:
+// 105 -> 92 us; with the row pointers in shared memory and every load ahead
+// of the first store 85 us (2D 105 -> 74). Three blocks per SM; two: 2D 82 us,
+// four: 90 us (200 bytes of spills).
+// 4 x for x > 0 well inside the range, on the exponent.
+__device__ __forceinline__ double times4(double x) {
+    return __hiloint2double(__double2hiint(x) + (2 << 20), __double2loint(x));
 }
 
 template <int DIM, bool RES = false>
@@ -518,18 +528,15 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     const double h = 0.5 * ts;
     const int gas = c->use_gas, path = c->inc_path;
     const int flow = c->use_flow && !k.shear_on, shear = c->use_flow && k.shear_on;
-    const double *X = drow(b, c, RX), *Y = drow(b, c, RY), *Z = drow(b, c, RZ),
-                 *R = drow(b, c, RR);
-    double *XN = drow(b, c, RXN), *YN = drow(b, c, RYN), *ZN = drow(b, c, RZN),
-           *RN = drow(b, c, RRN);
-    const double *V0 = drow(b, c, RV0), *V1 = drow(b, c, RV1), *V2 = drow(b, c, RV2),
-                 *V3 = drow(b, c, RV3);
-    double *P0 = drow(b, c, RVP0), *P1 = drow(b, c, RVP1), *P2 = drow(b, c, RVP2),
-           *P3 = drow(b, c, RVP3);
-    const double *S0 = drow(b, c, RS0), *S1 = drow(b, c, RS1), *S2 = drow(b, c, RS2),
-                 *S3 = drow(b, c, RS3);
-    const double *PATH = drow(b, c, RPATH);
-    double *PATHN = drow(b, c, RPATHN), *ERR = drow(b, c, RERR);
+    // row pointers from a table in shared memory (tab_ptr, common.cuh; a
+    // resident run has its tables there already): 128 -> 80 registers
+    __shared__ unsigned long long tab[RES ? 1 : ND_ROLES];
+    if (!RES) {
+        if (threadIdx.x < ND_ROLES)
+            tab[threadIdx.x] = reinterpret_cast<unsigned long long>(b.ds[c->drole[threadIdx.x]]);
+        __syncthreads();
+    }
+#define CB_D(r) (RES ? drow(b, c, r) : reinterpret_cast<double *>(tab_ptr(tab, r)))
     const int *NN = irow(b, c, INN);
     // mean-field factors, src/kernels.cu:399-408 (uniform over bubbles).
     // The overlap row ov and the pairwise rate are in units of ov_unit, and
@@ -538,6 +545,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     const double mfa = c->mfa, mfb = c->mfb;
     const double kq = DIM == 3 ? k.K * 0.25 : k.K * (1.0 / kPi);
     const double drag = 1.0 - k.wall_drag;
+    const int fixb = k.fix_b;
     long long merr = 0, mrad = 0, mexp = 0;
     double vol = 0.0;
     int ndel = 0, bad = 0;
@@ -549,54 +557,68 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         if (gas || flow) a1 = reinterpret_cast<const double4_32a *>(acc)[1];
         double vpx = a0.x, vpy = a0.y, vpz = a0.z, vpr = a0.w;
         const double ov = a1.x;
-        const State p = ld_state<DIM>(b, i, k.fix_b);
-        const double xp = p.x, yp = p.y, zp = p.z, rp = p.r;
+        const double4_32a p = ld4(b.pred, i);
+        // every input up front (a load cannot move across a store the
+        // compiler thinks may alias it)
+        const double err0 = CB_D(RERR)[i], path0 = path ? CB_D(RPATH)[i] : 0.0;
+        const double x0 = CB_D(RX)[i], y0 = CB_D(RY)[i], z0 = DIM == 3 ? CB_D(RZ)[i] : 0.0;
+        const double s0 = CB_D(RS0)[i], s1 = CB_D(RS1)[i], s2 = DIM == 3 ? CB_D(RS2)[i] : 0.0;
+        const double v0 = CB_D(RV0)[i], v1 = CB_D(RV1)[i], v2 = DIM == 3 ? CB_D(RV2)[i] : 0.0;
+        double v3 = 0.0, r0 = 0.0, s3 = 0.0;
+        double2 ri = make_double2(0.0, 0.0);  // (1/rp, rp^2) of k_predict
+        if (gas) {
+            v3 = CB_D(RV3)[i];
+            r0 = CB_D(RR)[i];
+            s3 = CB_D(RS3)[i];
+            if (DIM == 3) ri = reinterpret_cast<const double2 *>(b.invr)[i];
+        }
+        const long long qx = __double_as_longlong(p.x), qy = __double_as_longlong(p.y),
+                        qz = DIM == 3 ? __double_as_longlong(p.z) : 0,
+                        qr = __double_as_longlong(DIM == 3 ? p.w : p.z);
         if (flow | shear | k.any_wall) {
-            const Vel3 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz, xp, yp, zp,
-                                                  rp, a1.y, a1.z, a1.w, flow ? NN[i] : 0);
+            const State q = ld_state<DIM>(b, i, fixb);
+            const Vel3 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz, q.x, q.y,
+                                                  q.z, q.r, a1.y, a1.z, a1.w, flow ? NN[i] : 0);
             vpx = v.x;
             vpy = v.y;
             vpz = v.z;
         }
         // AM2 correct x + 0.5 ts (v + vp), src/kernels.cu:487-495 and :366-387
-        long long e = 0;
-        // inputs read after the first store below, loaded up front (a load
-        // cannot move across a store the compiler thinks may alias it)
-        const double err0 = ERR[i], path0 = path ? PATH[i] : 0.0;
-        const double x0 = X[i], y0 = Y[i];
-        const double cx = fma(h, V0[i] + vpx, x0);
-        e = max_bits(e, abs_bits(xp - cx));
-        const double cy = fma(h, V1[i] + vpy, y0);
-        e = max_bits(e, abs_bits(yp - cy));
-        double cz = 0.0, z0 = 0.0, sz = 0.0;
+        const double cx = fma(h, v0 + vpx, x0);
+        const double cy = fma(h, v1 + vpy, y0);
+        const long long fx = fx_from_double(cx, fixb), fy = fx_from_double(cy, fixb);
+        // the largest |predicted - corrected|, in units 2^-fixb
+        uint64_t em = max(fx_abs(qx - fx), fx_abs(qy - fy));
+        double cz = 0.0;
+        long long fz = 0, sz = 0;
         if (DIM == 3) {
-            z0 = Z[i];
-            cz = fma(h, V2[i] + vpz, z0);
-            e = max_bits(e, abs_bits(zp - cz));
-            sz = cz - S2[i];
+            cz = fma(h, v2 + vpz, z0);
+            fz = fx_from_double(cz, fixb);
+            em = max(em, fx_abs(qz - fz));
+            sz = fz - fx_from_double(s2, fixb);
         }
         // distance from the position of the last search; only its maximum
         // over the foam is used (the search trigger)
-        double dist = norm_ffd<DIM>(cx - S0[i], cy - S1[i], sz);
+        double dist = fx_norm<DIM>(fx - fx_from_double(s0, fixb), fy - fx_from_double(s1, fixb),
+                                   sz, fixb);
         int del = 0;
         if (gas) {  // mean-field gas exchange and radius, src/kernels.cu:390-431
             double inv, area;
-            if (DIM == 3) {  // (1/rp, rp^2) record of k_predict
-                const double2 e = reinterpret_cast<const double2 *>(b.invr)[i];
-                inv = e.x;
-                area = 4.0 * e.y;
+            if (DIM == 3) {
+                inv = ri.x;
+                area = times4(ri.y);
             } else {
-                inv = p.inv;
-                area = kPi * rp;
+                inv = p.w;
+                area = kPi * fx_to_double((unsigned long long)qr, -fixb);
             }
             double vr = mfa - inv;
             vr *= mfb * (area - ov);
             vr += vpr;
             vr *= DIM == 3 ? kq * (inv * inv) : kq * inv;
             vpr = vr;
-            const double cr = fma(h, V3[i] + vr, R[i]);
-            e = max_bits(e, abs_bits(rp - cr));
-            dist += cr - S3[i];
+            const double cr = fma(h, v3 + vr, r0);
+            em = max(em, fx_abs(qr - fx_from_double(cr, fixb)));
+            dist += cr - s3;
             if (__double_as_longlong(cr) > __double_as_longlong(k.min_rad)) {  // cr > minRad
                 vol = fma(DIM == 3 ? cr * cr : cr, cr, vol);
             } else {
@@ -604,23 +626,26 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 ndel++;
             }
             mrad = max_bits(mrad, cr);
-            RN[i] = cr;
-            P3[i] = vpr;
+            CB_D(RRN)[i] = cr;
+            CB_D(RVP3)[i] = vpr;
             bad |= !finite_bits(cr);
         }
         b.delflag[i] = del;
         mexp = max_bits(mexp, dist);
         if (path)  // src/kernels.cu:437-451; the increment to ~2^-46
-            PATHN[i] = path0 + norm_ffd<DIM>(x0 - cx, y0 - cy, z0 - cz);
-        ERR[i] = __longlong_as_double(max(e, __double_as_longlong(err0)));  // both >= 0
+            CB_D(RPATHN)[i] = path0 + fx_norm<DIM>(fx_from_double(x0, fixb) - fx,
+                                            fx_from_double(y0, fixb) - fy,
+                                            DIM == 3 ? fx_from_double(z0, fixb) - fz : 0, fixb);
+        const long long e = __double_as_longlong(fx_to_double_any(em, -fixb));
+        CB_D(RERR)[i] = __longlong_as_double(max(e, __double_as_longlong(err0)));  // both >= 0
         merr = max(merr, e);
-        XN[i] = cx;
-        YN[i] = cy;
-        P0[i] = vpx;
-        P1[i] = vpy;
+        CB_D(RXN)[i] = cx;
+        CB_D(RYN)[i] = cy;
+        CB_D(RVP0)[i] = vpx;
+        CB_D(RVP1)[i] = vpy;
         if (DIM == 3) {
-            ZN[i] = cz;
-            P2[i] = vpz;
+            CB_D(RZN)[i] = cz;
+            CB_D(RVP2)[i] = vpz;
         }
         bad |= !(finite_bits(cx) && finite_bits(cy) && finite_bits(cz));
         if (b.dbg_ov) b.dbg_ov[i] = ov_unit(DIM) * ov;
@@ -630,20 +655,13 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         reinterpret_cast<double4_32a *>(acc)[0] = zero;
         if (gas || flow) reinterpret_cast<double4_32a *>(acc)[1] = zero;
     }
+#undef CB_D
     if (RES) {
         const long long m[3] = {merr, mrad, mexp};
         const int cn[2] = {ndel, bad};
         run_reduce<1, 3, 2>(&vol, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
         run_barrier(rx);
-        if (threadIdx.x == 0) {
-            const RunAcc *g = rx->acc;
-            const double e = __longlong_as_double(__ldcg(&g->cmax[0])),
-                         r = __longlong_as_double(__ldcg(&g->cmax[1])),
-                         x = __longlong_as_double(__ldcg(&g->cmax[2])), v = __ldcg(&g->csum[0]);
-            const int nd = __ldcg(&g->cnt[0]), nb = __ldcg(&g->cnt[1]);
-            finish_attempt<DIM>(c, k, e, r, x, v, (double)nd, (double)nb);
-        }
-        __syncthreads();
+        run_finish<DIM>(c, k, rx->acc, ts, [] {});
         return;
     }
     long long *lsm = reinterpret_cast<long long *>(smem);
@@ -670,9 +688,9 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     const double fDel = fold_partials(b.part + 4 * G, G, false, smem);
     const double fBad = fold_partials(b.part + 5 * G, G, false, smem);
     if (threadIdx.x != 0) return;
-    finish_attempt<DIM>(c, k, fErr, fRad, fExp, fVol, fDel, fBad);
+    finish_attempt<DIM>(c, k, {fErr, fRad, fExp, fVol, (int)fDel, (int)fBad});
 }
-CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBlock))
+CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBlock, 3))
 
 
 // ----------------------------------------------------------- resident run
@@ -694,7 +712,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, const Bufs *foams,
         if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
     }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
     do {

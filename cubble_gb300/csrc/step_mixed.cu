@@ -271,9 +271,9 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
             }
         }
     }
-    if (RES) {  // the sums are read after the pair phase
-        const double v[2] = {(double)sA, (double)sAr};
-        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->sum, nullptr, nullptr, rsm);
+    if (RES) {  // read after the pair phase
+        const float v[2] = {sA, sAr};
+        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->psum + 2, nullptr, nullptr, rsm);
         run_barrier(rx);
         return;
     }
@@ -609,11 +609,11 @@ __device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, con
         if (hit) flush();
     }
     if (RES) {
-        const double v[2] = {(double)sAo, (double)sAor};
-        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->osum, nullptr, nullptr, rsm);
+        const float v[2] = {sAo, sAor};
+        run_reduce<2, 0, 0>(v, nullptr, nullptr, rx->acc->psum, nullptr, nullptr, rsm);
         run_barrier(rx);
         run_clear_other(rx, vb);
-        double fAo = __ldcg(&rx->acc->osum[0]), fAor = __ldcg(&rx->acc->osum[1]);
+        double fAo = __ldcg(&rx->acc->psum[0]), fAor = __ldcg(&rx->acc->psum[1]);
         if (GAS) {
             int2 *RC = recheck_list(AV, cap);
             if (__ldcg(&RC[0].x)) {  // the same for every block; rare
@@ -626,17 +626,28 @@ __device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, con
                 if (vb == 0 && threadIdx.x == 0) RC[0].x = 0;  // every block has read it
             }
         }
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 || threadIdx.x == 32) {  // the two divisions in two warps
             Ctrl *cc = b.ctrl;
-            if (!cc->pred_ready) {  // the prediction of this attempt's predict phase
-                cc->sumA = __ldcg(&rx->acc->sum[0]);
-                cc->sumAr = DIM == 3 ? __ldcg(&rx->acc->sum[1])
+            double sumA = cc->sumA, sumAr = cc->sumAr;
+            const bool fresh = !cc->pred_ready;  // from this attempt's predict phase
+            if (fresh) sumA = __ldcg(&rx->acc->psum[2]);
+            if (threadIdx.x == 32) {
+                cc->mfb = k.kappa * k.ain * (double)cc->n / sumA;
+            } else {
+                if (fresh)
+                    sumAr = DIM == 3 ? __ldcg(&rx->acc->psum[3])
                                      : area_over_radius_2d<false>(cc->n, rx->threads);
+                cc->mfa = (sumAr - fAor) / (sumA - 2.0 * fAo);
+                cc->sumAo = 2.0 * fAo;
+                cc->sumAor = fAor;
+                rx->sA = sumA;  // stored below: the other thread may still read
+                rx->sAr = sumAr;
             }
-            cc->sumAo = 2.0 * fAo;
-            cc->sumAor = fAor;
-            cc->mfa = (cc->sumAr - cc->sumAor) / (cc->sumA - cc->sumAo);
-            cc->mfb = k.kappa * k.ain * (double)cc->n / cc->sumA;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            b.ctrl->sumA = rx->sA;
+            b.ctrl->sumAr = rx->sAr;
         }
         return;
     }
@@ -944,29 +955,22 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
 #undef CB_D
 #undef CB_F
     if (RES) {
-        const double sv[5] = {vol, (double)cA0, (double)cA1, (double)cAr0, (double)cAr1};
+        const float sv[4] = {cA0, cA1, cAr0, cAr1};
         const long long m[3] = {merr, mrad, __double_as_longlong(double_from_float(mexp))};
         const int cn[2] = {ndel, bad};
-        run_reduce<!GAS ? 1 : (DIM == 2 ? 3 : 5), 3, 2>(sv, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
+        constexpr int kS = !GAS ? 0 : (DIM == 2 ? 2 : 4);  // 2D: area_over_radius_2d
+        run_reduce<1, 3, 2, kS>(&vol, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm, sv);
         run_barrier(rx);
-        if (threadIdx.x == 0) {
-            const RunAcc *g = rx->acc;
-            const double e = __longlong_as_double(__ldcg(&g->cmax[0])),
-                         r = __longlong_as_double(__ldcg(&g->cmax[1])),
-                         x = __longlong_as_double(__ldcg(&g->cmax[2])), v = __ldcg(&g->csum[0]);
-            const int nd = __ldcg(&g->cnt[0]), nx = __ldcg(&g->cnt[1]);
-            c->cand_sumA[0] = __ldcg(&g->csum[1]);
-            c->cand_sumA[1] = __ldcg(&g->csum[2]);
-            if (DIM == 3) {
-                c->cand_sumAr[0] = __ldcg(&g->csum[3]);
-                c->cand_sumAr[1] = __ldcg(&g->csum[4]);
-            } else {
-                c->cand_sumAr[0] = c->cand_sumAr[1] =
-                    area_over_radius_2d<true>(n, rx->threads);
-            }
-            finish_attempt<DIM>(c, k, e, r, x, v, (double)nd, (double)nx);
-        }
-        __syncthreads();
+        const RunAcc *g = rx->acc;
+        run_finish<DIM>(c, k, g, c->dt, [&] {
+            const double a0 = __ldcg(&g->csum[1]), a1 = __ldcg(&g->csum[2]);
+            double r0 = __ldcg(&g->csum[3]), r1 = __ldcg(&g->csum[4]);
+            if (DIM == 2) r0 = r1 = area_over_radius_2d<true>(n, rx->threads);
+            c->cand_sumA[0] = a0;
+            c->cand_sumA[1] = a1;
+            c->cand_sumAr[0] = r0;
+            c->cand_sumAr[1] = r1;
+        });
         return;
     }
     CorrRed v{merr, mrad, __double_as_longlong(double_from_float(mexp)), vol, ndel, bad,
@@ -996,7 +1000,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     const double fDel = (double)vc->acnt_del, fBad = (double)vc->acnt_bad;
     c->amax_err = c->amax_rad = c->amax_exp = 0;
     c->acnt_del = c->acnt_bad = 0;
-    finish_attempt<DIM>(c, k, fErr, fRad, fExp, fVol, fDel, fBad);
+    finish_attempt<DIM>(c, k, {fErr, fRad, fExp, fVol, (int)fDel, (int)fBad});
 }
 CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_mx, (<DIM, GAS, FLOW, WALLS>), __launch_bounds__(kBlock, 4))
 
@@ -1023,7 +1027,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_run_mx(Bufs b, const Bufs *foams,
     // threads of the launch per phase (area_over_radius_2d): the virtual grid
     // of a batched foam, else four resident blocks per SM
     RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed,
-              map ? b.ctrl->vgrid_a * kBlock : threads};
+              map ? b.ctrl->vgrid_a * kBlock : threads, 0.0, 0.0};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
     do {

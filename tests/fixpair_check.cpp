@@ -91,6 +91,20 @@ int main() {
     taken += cbg::fx_pair<3, true>(one53, 0, 0, 3 * one53, -one53, 53, t);  // a negative radius
     taken += cbg::fx_pair<2, true>(1 << 20, 0, 0, 1 << 20, 1 << 20, 53, t); // below the unit range
     printf("taken_outside %d\n", taken);
+    // norms of differences, from one unit to the whole range
+    ld worst = 0, mean = 0;
+    for (int it = 0; it < 600000; it++) {
+        const double span = std::exp2(61.0 - 61.0 * std::fabs(U(rng)));
+        int64_t v[3];
+        for (int64_t &a : v) a = (int64_t)(U(rng) * span);
+        if (it % 5 == 0) v[it % 3] = 0;
+        const ld want = sqrtl((ld)v[0] * v[0] + (ld)v[1] * v[1] + (ld)v[2] * v[2]);
+        const double got = cbg::fx_norm<3>(v[0], v[1], v[2], 53);
+        const ld er = want == 0 ? (got == 0 ? 0 : 1) : (got - ldexpl(want, -53)) / ldexpl(want, -53);
+        worst = std::max(worst, absl_(er));
+        mean += er;
+    }
+    printf("norm %.3Le\nnorm_bias %.3Le\n", worst, absl_(mean / 600000));
     // to fixed point and back: the nearest integer, and the same double
     double back = 0, near = 0;
     for (int it = 0; it < 400000; it++) {

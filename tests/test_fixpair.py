@@ -50,3 +50,10 @@ def test_range(found):
 def test_conversions(found):
     assert found["to_fixed"] <= 0.5
     assert found["round_trip"] == 0
+
+
+def test_norm(found):
+    """Norms of integer differences in float-float: 2^-45, as its root and
+    squares, and no bias beyond the last place of a double."""
+    assert found["norm"] <= 2.0 ** -45
+    assert found["norm_bias"] <= 2.0 ** -52
