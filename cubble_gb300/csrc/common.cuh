@@ -883,6 +883,7 @@ __device__ __forceinline__ void run_finish(Ctrl *c, const DevConst &k, const Run
 __device__ __forceinline__ bool run_more(const RunShared *s, int attempts) {
     const Ctrl &c = s->c;
     if (s->failed || c.status != CB_OK || attempts >= kRunMaxAttempts) return false;
+    if (attempts == 0) return c.steps < c.steps_target;  // what the last launch left is done
     if (c.too_large) return true;
     return !c.need_delete && !c.need_search && c.steps < c.steps_target && !c.stop_hit;
 }
@@ -1032,6 +1033,13 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, cudaStream_t stream, 
             launch_pdl(NAME CB_ID ARGS, (GRID), (l).stream, (b));                    \
         *(l).launches += 1;                                                          \
     } while (0)
+
+// Blocks of a grid-stride kernel of a single foam: one per `kBlock / per`
+// bubbles of its capacity, up to l.grid.
+inline int small_grid(const Launch &l, int per = 1) {
+    const long long g = (long long)l.cover * per;
+    return (int)(g < l.grid ? g : l.grid);
+}
 
 // One wave of resident blocks of `kernel` (a multiple of the SM count),
 // bounded by l.grid (the size of the per-block partial arrays).

@@ -146,6 +146,26 @@ __global__ void __launch_bounds__(kBlock) k_max_radius(const double *R, int n, C
                   (unsigned long long)m);
 }
 
+// Rows of a loaded state that the caller did not give, zeroed by one kernel
+// (a cudaMemsetAsync each, ~25 of them, took ~60 us of host time a load).
+struct ZeroRows {
+    int4 *row[ND_ROLES + NI_ROLES + 1];
+    unsigned quads[ND_ROLES + NI_ROLES + 1];  // 16-byte units
+    int rows = 0;
+    void add(void *p, size_t bytes) {  // rows are allocated in whole 16-byte units
+        row[rows] = static_cast<int4 *>(p);
+        quads[rows++] = (unsigned)((bytes + 15) / 16);
+    }
+};
+__global__ void __launch_bounds__(kBlock) k_zero_rows(ZeroRows z) {
+    for (int r = 0; r < z.rows; r++) {
+        int4 *p = z.row[r];
+        for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < z.quads[r];
+             i += gridDim.x * blockDim.x)
+            p[i] = make_int4(0, 0, 0, 0);
+    }
+}
+
 // The mixed form's FP32 rate rows to and from the host's FP64 rows, through
 // scratch rows on the device. Bound by its 12 bytes per element (3 10^6
 // bubbles, 8 rows: ~45 us); the same conversion on the host took 10 ms of a
@@ -198,11 +218,14 @@ int sync_status(cb_context *c) {
 
 // A state change from the host (new rows, pairs, dt, options, box) makes
 // the candidate predictions of the mixed form stale.
+void stale_prediction(cb_context *c) {  // in the host's mirror
+    c->hctrl->pred_ready = 0;
+    c->hctrl->pred_slot = 0;
+}
 int invalidate_prediction(cb_context *c) {
     int rc = c->pull();
     if (rc) return rc;
-    c->hctrl->pred_ready = 0;
-    c->hctrl->pred_slot = 0;
+    stale_prediction(c);
     return c->push();
 }
 
@@ -297,8 +320,9 @@ int integrate_resident(cb_context *c, int64_t n_steps) {
             if ((rc = c->check_launch())) return rc;
         }
         if (search && (rc = run_search(c))) return rc;
-        if ((del || search) && (rc = sync_status(c))) return rc;
-        if (h.stop_hit || h.steps >= target) return CB_OK;
+        // the next run follows on the stream (it does nothing if the search
+        // failed, and brings the status back)
+        if (h.stop_hit || h.steps >= target) return del || search ? sync_status(c) : CB_OK;
     }
 }
 
@@ -543,8 +567,8 @@ int cbg::create_context(const cb_config *cfg, cb_context **out, bool graph) {
     const size_t cap = (size_t)c->hk.cap, pcap = (size_t)c->hk.pcap, ccap = (size_t)c->hk.ccap;
     c->launch.grid = std::max(1, c->sms) * 8;
     c->launch.sms = std::max(1, c->sms);
-    c->launch.scan_grid = std::min(1024, std::max(1, c->sms) * 4);
     c->launch.cover = (int)((cap + kBlock - 1) / kBlock);
+    c->launch.scan_grid = std::min(std::min(1024, std::max(1, c->sms) * 4), c->launch.cover);
     c->launch.stream = c->stream;
     c->launch.launches = &c->launches;
     const int G = std::max(c->launch.grid, c->launch.cover);
@@ -684,6 +708,7 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
     drows[RS2] = s->saved_z;
     drows[RS3] = s->saved_r;
     RateRows rates;
+    ZeroRows zero;
     for (int r = 0; r < ND_ROLES; r++) {
         double *dst = c->dslot[h.drole[r]];
         const bool rate = r >= RV0 && r <= RVP3;
@@ -699,7 +724,7 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
             CB_CUDA(cudaMemcpyAsync(dst, c->dslot[h.drole[RX + (r - RS0)]], n * 8,
                                     cudaMemcpyDeviceToDevice, c->stream));
         } else {
-            CB_CUDA(cudaMemsetAsync(dst, 0, (size_t)c->hk.cap * 8, c->stream));
+            zero.add(dst, (size_t)c->hk.cap * 8);
         }
     }
     if (rates.rows && (rc = convert_rates(c, rates, n, false))) return rc;
@@ -719,9 +744,12 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
         if (irows[r] && n)
             CB_CUDA(cudaMemcpyAsync(dst, irows[r], n * 4, cudaMemcpyHostToDevice, c->stream));
         else
-            CB_CUDA(cudaMemsetAsync(dst, 0, (size_t)c->hk.cap * 4, c->stream));
+            zero.add(dst, (size_t)c->hk.cap * 4);
     }
-    CB_CUDA(cudaMemsetAsync(c->bufs.acc, 0, (size_t)kAcc * c->hk.cap * 8, c->stream));
+    zero.add(c->bufs.acc, (size_t)kAcc * c->hk.cap * 8);
+    k_zero_rows<<<std::min(c->launch.grid, c->launch.cover), kBlock, 0, c->stream>>>(zero);
+    c->launches += 1;
+    if ((rc = c->check_launch())) return rc;
     h.n = s->count;
     h.np = 0;
     h.ndel = 0;
@@ -805,15 +833,10 @@ int cb_get_state(cb_context *c, cb_state_view *s) {
 }
 
 int cb_set_options(cb_context *c, int32_t g, int32_t f, int32_t p) {
-    {
-        if (!c) return fail(CB_ERR_INVALID_ARGUMENT, "null context");
-        CB_CUDA(cudaSetDevice(c->dev));
-        const int rc0 = invalidate_prediction(c);
-        if (rc0) return rc0;
-    }
     CB_ENTER(c);
     int rc = c->pull();
     if (rc) return rc;
+    stale_prediction(c);
     c->hctrl->use_gas = g ? 1 : 0;
     c->hctrl->use_flow = f ? 1 : 0;
     c->hctrl->inc_path = p ? 1 : 0;
@@ -821,15 +844,10 @@ int cb_set_options(cb_context *c, int32_t g, int32_t f, int32_t p) {
 }
 
 int cb_set_time(cb_context *c, double dt, uint64_t ti, double tf) {
-    {
-        if (!c) return fail(CB_ERR_INVALID_ARGUMENT, "null context");
-        CB_CUDA(cudaSetDevice(c->dev));
-        const int rc0 = invalidate_prediction(c);
-        if (rc0) return rc0;
-    }
     CB_ENTER(c);
     int rc = c->pull();
     if (rc) return rc;
+    stale_prediction(c);
     c->hctrl->dt = dt;
     c->hctrl->tint = ti;
     c->hctrl->tfrac = tf;
@@ -915,12 +933,6 @@ int cb_get_pairs(cb_context *c, int32_t *i, int32_t *j, int32_t capacity, int32_
 }
 
 int cb_set_pairs(cb_context *c, const int32_t *i, const int32_t *j, int32_t count) {
-    {
-        if (!c) return fail(CB_ERR_INVALID_ARGUMENT, "null context");
-        CB_CUDA(cudaSetDevice(c->dev));
-        const int rc0 = invalidate_prediction(c);
-        if (rc0) return rc0;
-    }
     CB_ENTER(c);
     if (count < 0 || (count && (!i || !j))) return fail(CB_ERR_INVALID_ARGUMENT, "bad pairs");
     if (count > c->hk.pcap) return fail(CB_ERR_CAPACITY, "pair capacity exceeded");
@@ -943,6 +955,7 @@ int cb_set_pairs(cb_context *c, const int32_t *i, const int32_t *j, int32_t coun
     if (h.n)
         CB_CUDA(cudaMemcpyAsync(c->islot[h.irole[INN]], nn.data(), (size_t)h.n * 4,
                                 cudaMemcpyHostToDevice, c->stream));
+    stale_prediction(c);
     h.np = count;
     return c->push();
 }

@@ -71,8 +71,9 @@ struct cb_context {
     template <typename T>
     int alloc(T **p, size_t n) {
         void *q = nullptr;
-        CB_CUDA(cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)));
-        CB_CUDA(cudaMemsetAsync(q, 0, std::max<size_t>(n, 1) * sizeof(T), stream));
+        const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 15) / 16 * 16;  // k_zero_rows
+        CB_CUDA(cudaMalloc(&q, bytes));
+        CB_CUDA(cudaMemsetAsync(q, 0, bytes, stream));
         allocs.push_back(q);
         *p = static_cast<T *>(q);
         return CB_OK;
@@ -114,6 +115,7 @@ struct NvtxRange {
 };
 
 int sync_status(cb_context *c);
+void stale_prediction(cb_context *c);
 int invalidate_prediction(cb_context *c);
 void launch_attempt_kernels(const cb_context *c, const Launch &l, const Bufs &b, int which = 7);
 int capture_conditional(cudaStream_t stream, cudaGraphConditionalNodeType type,

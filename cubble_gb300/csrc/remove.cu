@@ -111,7 +111,7 @@ CB_KERNEL_PAIR((template <int DIM>), k_remove_c, (<DIM>), __launch_bounds__(kBlo
 }  // namespace
 
 void launch_remove(const Launch &l, const Bufs &b, int dim) {
-    const int G = l.grid;
+    const int G = small_grid(l, 4);  // bubbles, and a few pairs each
     launch_scan(l, b, SCAN_DEL);
     CB_LAUNCH(l, k_remove_a, (), G, b);
     if (dim == 3)

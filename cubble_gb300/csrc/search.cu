@@ -1055,7 +1055,9 @@ CB_KERNEL_PAIR((), k_degree, (), __launch_bounds__(kBlock))
 }  // namespace
 
 void launch_search(const Launch &l, const Bufs &b, int dim) {
-    const int G = l.grid;
+    // G: kernels with a thread per bubble; W: with a warp per cell (2D foams
+    // have a cell per ~3 bubbles)
+    const int G = small_grid(l), W = small_grid(l, 8);
     if (dim == 3) {
         CB_LAUNCH(l, k_wrap, (<3>), G, b);
         CB_LAUNCH(l, k_cell_count, (<3>), G, b);
@@ -1065,24 +1067,24 @@ void launch_search(const Launch &l, const Bufs &b, int dim) {
     }
     launch_scan(l, b, SCAN_CELLS);
     CB_LAUNCH(l, k_cell_fill, (), G, b);
-    CB_LAUNCH(l, k_cell_order, (), G, b);
+    CB_LAUNCH(l, k_cell_order, (), W, b);
     if (dim == 3) {
         CB_LAUNCH(l, k_permute, (<3>), G, b);
-        CB_LAUNCH(l, k_pair_cells, (<3, false>), G, b);
-        CB_LAUNCH(l, k_pair_tiles, (<3>), G, b);
+        CB_LAUNCH(l, k_pair_cells, (<3, false>), W, b);
+        CB_LAUNCH(l, k_pair_tiles, (<3>), W, b);
         CB_LAUNCH(l, k_pair_rows, (<3>), G, b);
     } else {
         CB_LAUNCH(l, k_permute, (<2>), G, b);
-        CB_LAUNCH(l, k_pair_cells, (<2, false>), G, b);
+        CB_LAUNCH(l, k_pair_cells, (<2, false>), W, b);
         CB_LAUNCH(l, k_pair_rows, (<2>), G, b);
     }
     launch_scan(l, b, SCAN_ROWS);
     if (dim == 3) {
         CB_LAUNCH(l, k_pair_compact, (<3>), G, b);
-        CB_LAUNCH(l, k_pair_cells, (<3, true>), G, b);
+        CB_LAUNCH(l, k_pair_cells, (<3, true>), W, b);
     } else {
         CB_LAUNCH(l, k_pair_compact, (<2>), G, b);
-        CB_LAUNCH(l, k_pair_cells, (<2, true>), G, b);
+        CB_LAUNCH(l, k_pair_cells, (<2, true>), W, b);
     }
     CB_LAUNCH(l, k_degree, (), G, b);
 }

@@ -715,14 +715,15 @@ __global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, const Bufs *foams,
     RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
-    do {
+    while (run_more(&rs, attempts)) {
         run_begin(&rx, attempts);
         k_predict_body<DIM, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
         k_pairs_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
         k_correct_body<DIM, true>(b, vb, vg, &rx, &rsm);
-    } while (run_more(&rs, ++attempts));
+        attempts++;
+    }
     run_exit(&rs, ctrl, mirror, &rx, vb);
 }
 
@@ -884,25 +885,25 @@ void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode) {
 
 void launch_boot(const Launch &l, const Bufs &b, int dim, int phase) {
     if (dim == 3)
-        k_boot<3><<<l.grid, kBlock, 0, l.stream>>>(b, phase);
+        k_boot<3><<<small_grid(l), kBlock, 0, l.stream>>>(b, phase);
     else
-        k_boot<2><<<l.grid, kBlock, 0, l.stream>>>(b, phase);
+        k_boot<2><<<small_grid(l), kBlock, 0, l.stream>>>(b, phase);
     *l.launches += 1;
 }
 
 void launch_energy(const Launch &l, const Bufs &b, int dim, int per_bubble) {
     if (dim == 3)
-        k_energy<3><<<l.grid, kBlock, 0, l.stream>>>(b, per_bubble);
+        k_energy<3><<<small_grid(l, 4), kBlock, 0, l.stream>>>(b, per_bubble);
     else
-        k_energy<2><<<l.grid, kBlock, 0, l.stream>>>(b, per_bubble);
+        k_energy<2><<<small_grid(l, 4), kBlock, 0, l.stream>>>(b, per_bubble);
     *l.launches += 1;
 }
 
 void launch_volume(const Launch &l, const Bufs &b, int dim) {
     if (dim == 3)
-        k_volume<3><<<l.grid, kBlock, 0, l.stream>>>(b);
+        k_volume<3><<<small_grid(l), kBlock, 0, l.stream>>>(b);
     else
-        k_volume<2><<<l.grid, kBlock, 0, l.stream>>>(b);
+        k_volume<2><<<small_grid(l), kBlock, 0, l.stream>>>(b);
     *l.launches += 1;
 }
 

@@ -1030,14 +1030,15 @@ __global__ void __launch_bounds__(kBlock, 2) k_run_mx(Bufs b, const Bufs *foams,
               map ? b.ctrl->vgrid_a * kBlock : threads, 0.0, 0.0};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
-    do {
+    while (run_more(&rs, attempts)) {
         run_begin(&rx, attempts);
         k_predict_mx_body<DIM, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
         k_pairs_mx_body<DIM, GAS, FLOW, 4, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
         k_correct_mx_body<DIM, GAS, FLOW, WALLS, true>(b, vb, vg, &rx, &rsm);
-    } while (run_more(&rs, ++attempts));
+        attempts++;
+    }
     run_exit(&rs, ctrl, mirror, &rx, vb);
 }
 
@@ -1172,9 +1173,9 @@ void launch_run_mx(const RunLaunch &r, const Bufs &b, int dim, int mode, bool wa
 
 void launch_boot_mx(const Launch &l, const Bufs &b, int dim, int phase) {
     if (dim == 3)
-        k_boot_mx<3><<<l.grid, kBlock, 0, l.stream>>>(b, phase);
+        k_boot_mx<3><<<small_grid(l), kBlock, 0, l.stream>>>(b, phase);
     else
-        k_boot_mx<2><<<l.grid, kBlock, 0, l.stream>>>(b, phase);
+        k_boot_mx<2><<<small_grid(l), kBlock, 0, l.stream>>>(b, phase);
     *l.launches += 1;
 }
 
