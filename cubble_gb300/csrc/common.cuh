@@ -117,7 +117,7 @@ struct Ctrl {
     long long steps, attempts, searches, deleted, bubble_steps;
     long long steps_target;
     long long delete_events;  // removeBubbles() calls
-    unsigned long long h_loop, h_delete, h_search;  // conditional handles
+    unsigned long long h_loop, h_any, h_delete, h_search;  // conditional handles
     int drole[ND_ROLES];
     int irole[NI_ROLES];
     int prole[NP_ROLES];
@@ -646,8 +646,13 @@ __device__ void finish_attempt(Ctrl *c, const DevConst &k, const AttemptResult &
     if (c->graph_mode) {
         const int ok = c->status == CB_OK;
         const int accepted = !f.too_large;
-        set_cond(c->h_delete, ok && accepted && c->need_delete);
-        set_cond(c->h_search, ok && accepted && c->need_search);
+        const int del = ok && accepted && c->need_delete;
+        const int search = ok && accepted && c->need_search;
+        set_cond(c->h_any, del || search);
+        if (del || search) {
+            set_cond(c->h_delete, del);
+            set_cond(c->h_search, search);
+        }
         const int more = ok && (f.too_large || (c->steps < c->steps_target && !c->stop_hit));
         set_cond(c->h_loop, more);
         // the last iteration's removal / search are decided above; clearing

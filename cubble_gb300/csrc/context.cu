@@ -386,8 +386,10 @@ int capture_conditional(cudaStream_t stream, cudaGraphConditionalNodeType type,
 namespace {
 
 // integrate(n) as one graph:
-//   WHILE(h_loop) { predict; pairs; correct; IF(h_delete) remove; IF(h_search) search }
-// k_correct's last block sets the three conditions on the device.
+//   WHILE(h_loop) { predict; pairs; correct;
+//                   IF(h_any) { IF(h_delete) remove; IF(h_search) search } }
+// k_correct's last block sets the four conditions on the device. The outer IF
+// leaves one condition node on the path of an ordinary attempt.
 int build_graph(cb_context *c) {
     const int key = c->mode() | (c->hk.dim << 4);
     if (c->gexec && c->graph_key == key) return CB_OK;
@@ -397,7 +399,7 @@ int build_graph(cb_context *c) {
     }
     cudaGraph_t g;
     CB_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle hloop, hdel, hsearch;
+    cudaGraphConditionalHandle hloop, hany, hdel, hsearch;
     CB_CUDA(cudaGraphConditionalHandleCreate(&hloop, g, 1, cudaGraphCondAssignDefault));
     cudaGraphNodeParams wp{};
     wp.type = cudaGraphNodeTypeConditional;
@@ -416,11 +418,17 @@ int build_graph(cb_context *c) {
     const int dim = c->hk.dim;
     launch_attempt_kernels(c, l, c->bufs);
     const long long n_attempt = dummy;
-    cudaGraph_t delbody, searchbody;
-    int rc = capture_conditional(s, cudaGraphCondTypeIf, &hdel, 0, &delbody);
-    if (!rc) rc = capture_conditional(s, cudaGraphCondTypeIf, &hsearch, 0, &searchbody);
+    cudaGraph_t anybody, delbody, searchbody;
+    int rc = capture_conditional(s, cudaGraphCondTypeIf, &hany, 0, &anybody);
     cudaGraph_t out;
     cudaError_t e = cudaStreamEndCapture(s, &out);
+    if (rc) return rc;
+    CB_CUDA(e);
+    CB_CUDA(cudaStreamBeginCaptureToGraph(s, anybody, nullptr, nullptr, 0,
+                                          cudaStreamCaptureModeThreadLocal));
+    rc = capture_conditional(s, cudaGraphCondTypeIf, &hdel, 0, &delbody);
+    if (!rc) rc = capture_conditional(s, cudaGraphCondTypeIf, &hsearch, 0, &searchbody);
+    e = cudaStreamEndCapture(s, &out);
     if (rc) return rc;
     CB_CUDA(e);
     CB_CUDA(cudaStreamBeginCaptureToGraph(s, delbody, nullptr, nullptr, 0,
@@ -443,6 +451,7 @@ int build_graph(cb_context *c) {
     int r2 = c->pull();
     if (r2) return r2;
     c->hctrl->h_loop = (unsigned long long)hloop;
+    c->hctrl->h_any = (unsigned long long)hany;
     c->hctrl->h_delete = (unsigned long long)hdel;
     c->hctrl->h_search = (unsigned long long)hsearch;
     return c->push();
