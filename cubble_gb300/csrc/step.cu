@@ -135,9 +135,9 @@ CB_KERNEL_PAIR((template <int DIM>), k_predict, (<DIM>), __launch_bounds__(kBloc
 //     instead of five (alone: 202 -> 177 us);
 //   * overlap areas are accumulated in units of ov_unit (pi in 3D, 2 in 2D);
 //     the unit is applied to the global sums and in the correct kernel.
-// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 125 us (2D 117 -> 86, 3D
-// without gas exchange 141 -> 99). Nothing is saturated now: issue 57 %, L1 59 %
-// of its wavefronts, FP64 29 %; three or four blocks per SM make no difference,
+// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 123 us (2D 117 -> 84, 3D
+// without gas exchange 141 -> 96). Nothing is saturated now: issue 59 %, L1 62 %
+// of its wavefronts, FP64 31 %; three or four blocks per SM make no difference,
 // record loads a chunk ahead (108 registers) cost 8 us.
 __device__ __forceinline__ void red_add(double *p, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v));
@@ -216,7 +216,9 @@ static __device__ __noinline__ bool overlap_exact(long long ex, long long ey, lo
 // The terms of a pair fx_pair does not take, in FP64: centres much closer
 // than the radii, a negative predicted radius. The force goes to rs[0],
 // rs[kT], ...; returns the overlap as FxTerms::oa.
-constexpr int kT = 33;  // row length of the transposed results (32 pairs)
+// Row length of the transposed results (32 pairs): the 8-byte loads of four
+// pairs' components fall on distinct banks, but for the fifth row.
+constexpr int kT = 36;
 template <int DIM>
 static __device__ __noinline__ double pair_slow(long long ex, long long ey, long long ez,
                                                 long long q1, long long q2, double unit,
@@ -244,9 +246,10 @@ static __device__ __noinline__ void scale_force(double f0, double *rs) {
     for (int a = 0; a < DIM; a++) rs[a * kT] *= f0;
 }
 
-// A fixed-point length as FP32, in units of 2^62.
+// A fixed-point length as FP32, in units of 2^32: the signed high word and the
+// low one (~2^-24 relative, 2^-24 units where they cancel).
 __device__ __forceinline__ float fix_len(long long v) {
-    return fx_float((unsigned long long)(v < 0 ? -v : v)) * 0x1p-62f;
+    return fmaf((float)(unsigned)v, 0x1p-32f, (float)(int)(v >> 32));
 }
 
 template <int DIM, bool GAS, bool FLOW, bool RES = false>
@@ -257,7 +260,7 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     // queue slots: the differences, both radii
     constexpr int kR1 = DIM, kSlots = kR1 + 2;
     __shared__ long long qd[kW][kSlots][kQueue];
-    __shared__ int qij[kW][2][kQueue];
+    __shared__ int2 qij[kW][kQueue];
     // the results of 32 pairs, component by component
     constexpr int kC = GAS ? DIM + 2 : DIM;
     __shared__ double res[kW][kC * kT];
@@ -276,27 +279,27 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     long long(*Q)[kQueue] = qd[w];
-    int *QI = qij[w][0], *QJ = qij[w][1];
+    int2 *QP = qij[w];
     double *RS = res[w];
     double sAo = 0.0, sAor = 0.0;
 
     // minimum image (wrappedDifference, src/kernels.cu:1094-1114), exact
     auto image = [](long long d, long long half, long long len) {
-        if (d > half) d -= len;
-        else if (d < -half) d += len;
+        if ((unsigned long long)(d + half) > 2ull * half) d -= d > 0 ? len : -len;
         return d;
     };
 
     // the force and gas-exchange terms of queued (overlapping) pair e
-    auto process = [&](int e) {
-        const int i = QI[e], j = QJ[e];
+    // (slot of the ring; its results go to column e)
+    auto process = [&](int slot, int e) {
+        const int i = QP[slot].x, j = QP[slot].y;
         double inv1 = 0.0, inv2 = 0.0;
         if (GAS) {  // 1/r of k_predict
             inv1 = DIM == 3 ? b.invr[2 * (size_t)i] : b.pred[4 * (size_t)i + 3];
             inv2 = DIM == 3 ? b.invr[2 * (size_t)j] : b.pred[4 * (size_t)j + 3];
         }
-        const long long ex = Q[0][e], ey = Q[1][e], ez = DIM == 3 ? Q[2][e] : 0;
-        const long long q1 = Q[kR1][e], q2 = Q[kR1 + 1][e];
+        const long long ex = Q[0][slot], ey = Q[1][slot], ez = DIM == 3 ? Q[2][slot] : 0;
+        const long long q1 = Q[kR1][slot], q2 = Q[kR1 + 1][slot];
         double oa;
         FxTerms t;
         if (fx_pair<DIM, GAS>(ex, ey, ez, q1, q2, fixb, t)) {
@@ -322,9 +325,9 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
             if (DIM == 3) red_add(ai + 7, V2[j]);
         }
     };
-    // adds the results of queued pairs 0..m-1 to both bubbles' rows: eight
-    // lanes a pair, a component each
-    auto scatter = [&](int m) {
+    // adds the results of the m queued pairs from `head` on to both bubbles'
+    // rows: eight lanes a pair, a component each
+    auto scatter = [&](int head, int m) {
         __syncwarp();
         const int q = lane & 7;
         const int slot = DIM == 2 && q >= 2 ? q + 1 : q;  // vx, vy, vz, vr, overlap
@@ -333,14 +336,16 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
             const int e = e0 + (lane >> 3);
             if (e < m && q < kC) {
                 const double v = RS[q * kT + e];
-                red_add(b.acc + (size_t)QI[e] * kAcc + slot, v);
-                red_add(b.acc + (size_t)QJ[e] * kAcc + slot, slot == 4 ? v : neg_bits(v));
+                const int2 ij = QP[(head + e) & (kQueue - 1)];
+                red_add(b.acc + (size_t)ij.x * kAcc + slot, v);
+                red_add(b.acc + (size_t)ij.y * kAcc + slot, slot == 4 ? v : neg_bits(v));
             }
         }
         __syncwarp();
     };
 
-    int cnt = 0;  // queued pairs of this warp (uniform over its lanes)
+    // queued pairs of this warp: cnt of them from `head` on in a ring of kQueue
+    int cnt = 0, head = 0;
     const int nch = (np + 31) >> 5;
     const int wb = RES ? blockDim.x >> 5 : kW;  // warps of this block
     int p = ((RES ? w * vg + vb : vb * kW + w) << 5) + lane;
@@ -393,9 +398,8 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         }
         const unsigned mask = __ballot_sync(0xffffffffu, over);
         if (over) {
-            const int e = cnt + __popc(mask & below);
-            QI[e] = i;
-            QJ[e] = j;
+            const int e = (head + cnt + __popc(mask & below)) & (kQueue - 1);
+            QP[e] = make_int2(i, j);
             Q[0][e] = ex;
             Q[1][e] = ey;
             if (DIM == 3) Q[2][e] = ez;
@@ -405,20 +409,14 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         cnt += __popc(mask);
         __syncwarp();
         if (cnt >= 32) {  // a full warp of overlapping pairs
-            process(lane);
-            scatter(32);
+            process((head + lane) & (kQueue - 1), lane);
+            scatter(head, 32);
+            head = (head + 32) & (kQueue - 1);
             cnt -= 32;
-            if (lane < cnt) {
-                QI[lane] = QI[32 + lane];
-                QJ[lane] = QJ[32 + lane];
-#pragma unroll
-                for (int t = 0; t < kSlots; t++) Q[t][lane] = Q[t][32 + lane];
-            }
-            __syncwarp();
         }
     }
-    if (lane < cnt) process(lane);
-    scatter(cnt);
+    if (lane < cnt) process((head + lane) & (kQueue - 1), lane);
+    scatter(head, cnt);
 
     pairs_fold<DIM, RES>(b, vb, vg, sAo, sAor, smem, rx, rsm);
 }
