@@ -262,9 +262,7 @@ int build_run_map(cb_batch *b) {
     return CB_OK;
 }
 
-// Every selected foam's resident run, and the decision on the next phases.
-void launch_batch_run(cb_batch *b) {
-    const cb_context *c = b->first();
+RunLaunch batch_run_launch(cb_batch *b) {
     RunLaunch r;
     r.grid = b->run_blocks;
     r.block = kBlock;
@@ -275,6 +273,13 @@ void launch_batch_run(cb_batch *b) {
     r.launches = &b->launches;
     r.foams = b->dbufs;
     r.map = b->drun;
+    return r;
+}
+
+// Every selected foam's resident run, and the decision on the next phases.
+void launch_batch_run(cb_batch *b) {
+    const cb_context *c = b->first();
+    const RunLaunch r = batch_run_launch(b);
     if (c->hk.mixed)
         launch_run_mx(r, c->bufs, c->hk.dim, c->mode(), c->hk.any_wall != 0);
     else
@@ -395,7 +400,13 @@ int batch_integrate(cb_batch *b, int64_t n_steps, cb_report *reports, double *ms
                 CB_CUDA(cudaGetLastError());
                 if ((rc = b->pull_bc())) return rc;
                 if (b->hbc->any_delete) launch_batch_remove(b, &b->launches);
-                if (b->hbc->any_search) launch_batch_search(b, &b->launches);
+                if (b->hbc->any_search) {
+                    if (run)
+                        launch_search_run(batch_run_launch(b), b->first()->bufs,
+                                          b->first()->hk.dim);
+                    else
+                        launch_batch_search(b, &b->launches);
+                }
                 CB_CUDA(cudaGetLastError());
                 if (!b->hbc->any_attempt) break;
             }

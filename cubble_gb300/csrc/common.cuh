@@ -170,6 +170,8 @@ struct RunAcc {
 };
 struct RunSync {
     RunAcc acc[2];  // of even and odd attempts
+    long long search_max;  // k_search_run: largest radius (bits), a row beyond its stash
+    int stash_over, pad0_;
     unsigned arrive, pad_[31], exits, pad2_[31];
 };
 
@@ -888,7 +890,9 @@ __device__ __forceinline__ void run_finish(Ctrl *c, const DevConst &k, const Run
 __device__ __forceinline__ bool run_more(const RunShared *s, int attempts) {
     const Ctrl &c = s->c;
     if (s->failed || c.status != CB_OK || attempts >= kRunMaxAttempts) return false;
-    if (attempts == 0) return c.steps < c.steps_target;  // what the last launch left is done
+    // a first attempt waits for a deletion or search that the last one asked for
+    if (attempts == 0)
+        return c.steps < c.steps_target && !c.need_delete && !c.need_search && !c.stop_hit;
     if (c.too_large) return true;
     return !c.need_delete && !c.need_search && c.steps < c.steps_target && !c.stop_hit;
 }
@@ -1105,6 +1109,7 @@ void launch_energy(const Launch &l, const Bufs &b, int dim, int per_bubble);
 void launch_volume(const Launch &l, const Bufs &b, int dim);
 // search.cu
 void launch_search(const Launch &l, const Bufs &b, int dim);
+void launch_search_run(const RunLaunch &r, const Bufs &b, int dim);  // r.steps: forced
 // remove.cu
 void launch_remove(const Launch &l, const Bufs &b, int dim);
 // scan.cu

@@ -247,17 +247,6 @@ void launch_attempt_kernels(const cb_context *c, const Launch &l, const Bufs &b,
 
 namespace {
 
-int run_attempt(cb_context *c) {
-    NvtxRange nv("Integration step");
-    launch_attempt_kernels(c, c->launch, c->bufs);
-    return c->check_launch();
-}
-
-int run_search(cb_context *c) {
-    launch_search(c->launch, c->bufs, c->hk.dim);
-    return c->check_launch();
-}
-
 // Contexts of up to this many bubbles run their attempts inside one
 // cooperative kernel (resident run, common.cuh); larger ones a launch per
 // phase. us per attempt on one GB300 (searches included), launches per phase
@@ -274,6 +263,37 @@ constexpr int kRunCapacity2 = 600000, kRunCapacity3 = 400000;
 
 bool resident(const cb_context *c) {
     return c->coop && c->hk.cap <= (c->hk.dim == 3 ? kRunCapacity3 : kRunCapacity2);
+}
+
+// Contexts of up to this many bubbles search in one cooperative launch
+// (k_search_run, search.cu). us per search, launches per phase -> one launch:
+// 2D N = 10^3 55 -> 41, 10^4 58 -> 46, 4 10^4 65 -> 53, 2 10^5 93 -> 97;
+// 3D 4 10^3 59 -> 44, 3 10^4 67 -> 56, 10^5 89 -> 87, 4 10^5 204 -> 220.
+constexpr int kSearchRunCapacity = 100000;
+
+RunLaunch search_launch(cb_context *c, bool force) {
+    RunLaunch r;
+    r.block = kBlock;
+    r.grid = std::min(2 * c->sms, 4 * c->launch.cover);
+    r.threads = 0;
+    r.stream = c->stream;
+    r.steps = force ? 1 : 0;
+    r.mirror = c->hctrl;
+    r.launches = &c->launches;
+    return r;
+}
+
+// A neighbour search of the context's foam on its stream.
+void enqueue_search(cb_context *c) {
+    if (c->coop && c->hk.cap <= kSearchRunCapacity)
+        launch_search_run(search_launch(c, true), c->bufs, c->hk.dim);
+    else
+        launch_search(c->launch, c->bufs, c->hk.dim);
+}
+
+int run_search(cb_context *c) {
+    enqueue_search(c);
+    return c->check_launch();
 }
 
 // Blocks and threads of a resident run: a warp per 32 items (the mixed form's
@@ -296,23 +316,38 @@ RunLaunch run_launch(cb_context *c, int64_t n_steps) {
     return r;
 }
 
+int run_attempt(cb_context *c) {
+    NvtxRange nv("Integration step");
+    launch_attempt_kernels(c, c->launch, c->bufs);
+    return c->check_launch();
+}
+
+
 // integrate() of a small foam: resident runs of attempts, each until a
 // deletion, a search or the end; the control block comes back with the run.
-// Expects hctrl to hold the device's control block.
+// Expects hctrl to hold the device's control block. A long stretch enqueues
+// several runs, each with the search it may end in (neither does anything
+// where it is not due), before it waits: ~33 attempts lie between searches.
 int integrate_resident(cb_context *c, int64_t n_steps) {
     const long long target = c->hctrl->steps + n_steps;
+    const bool mixed = c->hk.mixed != 0;
     for (;;) {
-        const RunLaunch r = run_launch(c, target - c->hctrl->steps);
-        if (c->hk.mixed)
-            launch_run_mx(r, c->bufs, c->hk.dim, c->mode(), c->hk.any_wall != 0);
-        else
-            launch_run(r, c->bufs, c->hk.dim, c->mode());
+        const long long left = target - c->hctrl->steps;
+        const int ahead = c->hk.cap <= kSearchRunCapacity && left >= 48
+                              ? (int)std::min<long long>(4, left / 24) : 1;
+        for (int q = 0; q < ahead; q++) {
+            const RunLaunch r = run_launch(c, q == 0 ? left : -1);  // then to the same target
+            if (mixed)
+                launch_run_mx(r, c->bufs, c->hk.dim, c->mode(), c->hk.any_wall != 0);
+            else
+                launch_run(r, c->bufs, c->hk.dim, c->mode());
+            if (ahead > 1) launch_search_run(search_launch(c, false), c->bufs, c->hk.dim);
+        }
         int rc = c->check_launch();
         if (rc) return rc;
         CB_CUDA(cudaStreamSynchronize(c->stream));
         const Ctrl &h = *c->hctrl;
         if (h.status != CB_OK) return fail(h.status, status_text(h.status));
-        if (h.too_large) continue;
         const bool del = h.need_delete, search = h.need_search;
         if (del) {
             NvtxRange nv("Removal");
@@ -322,7 +357,8 @@ int integrate_resident(cb_context *c, int64_t n_steps) {
         if (search && (rc = run_search(c))) return rc;
         // the next run follows on the stream (it does nothing if the search
         // failed, and brings the status back)
-        if (h.stop_hit || h.steps >= target) return del || search ? sync_status(c) : CB_OK;
+        if (!h.too_large && (h.stop_hit || h.steps >= target))
+            return del || search ? sync_status(c) : CB_OK;
     }
 }
 
@@ -603,7 +639,7 @@ int cbg::create_context(const cb_config *cfg, cb_context **out, bool graph) {
     if ((rc = c->alloc(&b.part, (size_t)kPartSlots * G))) return bail(rc);
     if ((rc = c->alloc(&b.delflag, cap + 1))) return bail(rc);
     if ((rc = c->alloc(&b.iscan, cap + 1))) return bail(rc);
-    if ((rc = c->alloc(&b.blocksums, (size_t)c->launch.scan_grid + 1))) return bail(rc);
+    if ((rc = c->alloc(&b.blocksums, (size_t)std::max(c->launch.scan_grid, 2 * c->sms) + 1))) return bail(rc);
     if ((rc = c->alloc(&b.cellOf, cap))) return bail(rc);
     if ((rc = c->alloc(&b.cellSorted, cap))) return bail(rc);
     if ((rc = c->alloc(&b.perm, cap))) return bail(rc);
@@ -1198,7 +1234,7 @@ int profile_searches(cb_context *c, int32_t reps, double *ms) {
     if ((rc = run_search(c))) return rc;
     CB_CUDA(cudaStreamSynchronize(c->stream));
     CB_CUDA(cudaEventRecord(c->ev0, c->stream));
-    for (int r = 0; r < reps; r++) launch_search(c->launch, c->bufs, c->hk.dim);
+    for (int r = 0; r < reps; r++) enqueue_search(c);
     CB_CUDA(cudaEventRecord(c->ev1, c->stream));
     CB_CUDA(cudaEventSynchronize(c->ev1));
     float t = 0.f;

@@ -111,8 +111,37 @@ static __device__ __noinline__ void wrap_one(double *xp, int *wp, double x, doub
     *wp -= mult;
 }
 
-template <int DIM>
-__device__ __forceinline__ void k_wrap_body(const Bufs &b, const int vb, const int vg) {
+// The cell grid and the search's other decisions from the largest radius.
+__device__ __forceinline__ void search_begin(Ctrl *c, const DevConst &k, double max_r) {
+    int cd[3];
+    cell_grid(k, max_r, cd);
+    c->cell_dims[0] = cd[0];
+    c->cell_dims[1] = cd[1];
+    c->cell_dims[2] = cd[2];
+    c->ncell = cd[0] * cd[1] * cd[2];
+    c->searches += 1;
+    c->stash_over = 0;
+    c->sparse_cells = (long long)c->n < 24LL * c->ncell;
+    c->search_maxr = __double2float_ru(max_r);
+    c->pred_ready = 0;  // the bubbles move to new slots
+    c->pred_slot = 0;
+}
+// And its end: the pair count, or the status where the list does not fit.
+__device__ __forceinline__ void search_end(Ctrl *c, int pcap) {
+    const int found = c->np_found;
+    if (found > pcap) {
+        c->status = CB_ERR_CAPACITY;
+        c->np = 0;
+    } else {
+        c->np = found;
+    }
+    c->need_search = 0;
+}
+
+// RES here and below: as a phase of the resident search (k_search_run).
+template <int DIM, bool RES = false>
+__device__ __forceinline__ void k_wrap_body(const Bufs &b, const int vb, const int vg,
+                                            RunCtx *rx = nullptr) {
     __shared__ double smem[32];
     Ctrl *c = b.ctrl;
     const DevConst &k = *b.k;
@@ -147,23 +176,20 @@ __device__ __forceinline__ void k_wrap_body(const Bufs &b, const int vb, const i
         const double r = R[i];
         if (!is_nan_bits(r)) mr = max(mr, __double_as_longlong(r));  // fmax over radii >= 0
     }
-    const double t = __longlong_as_double(block_max_bits(mr, reinterpret_cast<long long *>(smem)));
-    if (threadIdx.x == 0) b.part[7 * vg + vb] = t;
+    const long long bm = block_max_bits(mr, reinterpret_cast<long long *>(smem));
+    if (RES) {
+        if (threadIdx.x == 0) atomicMax(&rx->g->search_max, bm);
+        run_barrier(rx);
+        if (threadIdx.x == 0)
+            search_begin(c, k, __longlong_as_double(__ldcg(&rx->g->search_max)));
+        __syncthreads();
+        return;
+    }
+    if (threadIdx.x == 0) b.part[7 * vg + vb] = __longlong_as_double(bm);
     if (last_block(&c->done[DC_WRAP], vg)) {
         const double f = fold_partials(b.part + 7 * vg, vg, true, smem);
         if (threadIdx.x == 0) {
-            int cd[3];
-            cell_grid(k, f, cd);
-            c->cell_dims[0] = cd[0];
-            c->cell_dims[1] = cd[1];
-            c->cell_dims[2] = cd[2];
-            c->ncell = cd[0] * cd[1] * cd[2];
-            c->searches += 1;
-            c->stash_over = 0;
-            c->sparse_cells = (long long)c->n < 24LL * c->ncell;
-            c->search_maxr = __double2float_ru(f);
-            c->pred_ready = 0;  // the bubbles move to new slots
-            c->pred_slot = 0;
+            search_begin(c, k, f);
             c->done[DC_WRAP] = 0;
         }
     }
@@ -249,7 +275,7 @@ __device__ __forceinline__ bool tile_grid(const DevConst &k, const int cd[3], in
 // their spare slots, then swap the roles. One pass over the bubbles: every
 // row of a bubble is gathered in the same iteration (the permutation read
 // once, all loads of the bubble in flight together).
-template <int DIM>
+template <int DIM, bool RES = false>
 __device__ __forceinline__ void k_permute_body(const Bufs &b, const int vb, const int vg) {
     Ctrl *c = b.ctrl;
     const int n = c->n;
@@ -339,7 +365,8 @@ __device__ __forceinline__ void k_permute_body(const Bufs &b, const int vb, cons
             b.pos32r[q] = make_float4(o[0], o[1], o[2], (float)p[3]);
         }
     }
-    if (last_block(&c->done[DC_PERMUTE], vg) && threadIdx.x == 0) {
+    if (RES) __syncthreads();  // every block swaps the roles in its own copy
+    if ((RES || last_block(&c->done[DC_PERMUTE], vg)) && threadIdx.x == 0) {
         int *r = c->drole;
         for (int a = 0; a < 4; a++) {
             if (DIM == 2 && a == 2) continue;
@@ -408,6 +435,13 @@ __device__ __forceinline__ int warp_sort(int v) {
 
 constexpr int kWarpsPerBlock = kBlock / 32;
 
+// Where a counting pass says that a row outgrew its stash (a resident search's
+// control block is a copy per block).
+template <bool RES>
+__device__ __forceinline__ int *stash_over_of(Ctrl *c, RunCtx *rx) {
+    return RES ? &rx->g->stash_over : &c->stash_over;
+}
+
 // Is j a pair partner of i (comparePair, src/kernels.cu:619-623)? Decided in
 // FP32 unless the distance lies within the guard band `pre_margin` of the
 // cutoff; there the reference's exact FP64 test decides. That test is a
@@ -460,8 +494,9 @@ __device__ __forceinline__ bool pair_take(const DevConst &k, const float4 &pi, c
 // in `stash` (k_pair_compact then writes the list without a second
 // enumeration); WRITE = true, needed only when some row had more partners,
 // enumerates again and writes the rows at rowStart.
-template <int DIM, bool WRITE>
-__device__ __forceinline__ void k_pair_cells_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool WRITE, bool RES = false>
+__device__ __forceinline__ void k_pair_cells_body(const Bufs &b, const int vb, const int vg,
+                                                  RunCtx *rx = nullptr) {
     __shared__ float4 stage[kWarpsPerBlock][32];
     Ctrl *c = b.ctrl;
     if (WRITE && !c->stash_over) return;  // k_pair_compact wrote the list
@@ -534,18 +569,12 @@ __device__ __forceinline__ void k_pair_cells_body(const Bufs &b, const int vb, c
         }
     }
     if (!WRITE) {
-        if (__syncthreads_or(over) && threadIdx.x == 0) atomicOr(&c->stash_over, 1);
+        if (__syncthreads_or(over) && threadIdx.x == 0) atomicOr(stash_over_of<RES>(c, rx), 1);
         return;
     }
+    if (RES) return;
     if (last_block(&c->done[DC_MISC], vg) && threadIdx.x == 0) {
-        const int found = c->np_found;
-        if (found > pcap) {
-            c->status = CB_ERR_CAPACITY;
-            c->np = 0;
-        } else {
-            c->np = found;
-        }
-        c->need_search = 0;
+        search_end(c, pcap);
         c->done[DC_MISC] = 0;
     }
 }
@@ -558,8 +587,9 @@ CB_KERNEL_PAIR((template <int DIM, bool WRITE>), k_pair_cells, (<DIM, WRITE>), _
 // in them, so the rows and their order are those of the warp-per-cell pass,
 // with all lanes busy (a warp per cell of ~3 bubbles would leave 90 % of its
 // lanes idle).
-template <int DIM>
-__device__ __forceinline__ void k_pair_rows_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool RES = false>
+__device__ __forceinline__ void k_pair_rows_body(const Bufs &b, const int vb, const int vg,
+                                                 RunCtx *rx = nullptr) {
     Ctrl *c = b.ctrl;
     if (!c->sparse_cells) return;
     const DevConst &k = *b.k;
@@ -661,7 +691,7 @@ __device__ __forceinline__ void k_pair_rows_body(const Bufs &b, const int vb, co
         b.rowCount[i] = cnt;
         over |= cnt > M;
     }
-    if (__syncthreads_or(over) && threadIdx.x == 0) atomicOr(&c->stash_over, 1);
+    if (__syncthreads_or(over) && threadIdx.x == 0) atomicOr(stash_over_of<RES>(c, rx), 1);
 }
 CB_KERNEL_PAIR((template <int DIM>), k_pair_rows, (<DIM>), __launch_bounds__(kBlock))
 
@@ -681,13 +711,12 @@ CB_KERNEL_PAIR((template <int DIM>), k_pair_rows, (<DIM>), __launch_bounds__(kBl
 // (in candidate order) into chunks of 32. The home cell's bubbles are then
 // broadcast from shared memory one at a time and every lane tests its
 // candidate against the bubble; the warp's hit mask of each (bubble, chunk)
-// goes to shared memory, and after a window of up to kTileChunks tested
+// goes to shared memory, and after a window of up to 16 (kTileChunks) tested
 // chunks each lane walks the masks of its home bubble and appends the
 // partners to the bubble's row in candidate order, the order of the thread
 // pass, so stash, counts and pair list are the same. All lanes work on every
 // test, against a thread per bubble that walks its own cells with, in 3D,
 // less than half of its warp's lanes busy.
-constexpr int kTileChunks = 16;  // window: 16 tested chunks of 32
 
 // The tests of one chunk against home bubbles 0..nh-1 (home cell bubbles
 // among the candidates: CMP, the j > i order test): the warp's hit mask of
@@ -760,8 +789,12 @@ __device__ __forceinline__ void tile_rows(const unsigned (*hitmask)[32], const i
     __syncwarp();
 }
 
-template <int DIM>
-__device__ __forceinline__ void k_pair_tiles_body(const Bufs &b, const int vb, const int vg) {
+template <int DIM, bool RES = false>
+__device__ __forceinline__ void k_pair_tiles_body(const Bufs &b, const int vb, const int vg,
+                                                  RunCtx *rx = nullptr) {
+    // a shorter window in the resident search, whose phases share the
+    // block's shared memory
+    constexpr int kTileChunks = RES ? 8 : 16;
     __shared__ float4 home[kWarpsPerBlock][32];
     __shared__ unsigned hitmask[kWarpsPerBlock][kTileChunks][32];  // [chunk][home bubble]
     __shared__ int candj[kWarpsPerBlock][kTileChunks * 32];
@@ -973,7 +1006,7 @@ __device__ __forceinline__ void k_pair_tiles_body(const Bufs &b, const int vb, c
             }
         }
     }
-    if (__syncthreads_or(over) && threadIdx.x == 0) atomicOr(&c->stash_over, 1);
+    if (__syncthreads_or(over) && threadIdx.x == 0) atomicOr(stash_over_of<RES>(c, rx), 1);
 }
 CB_KERNEL_PAIR((template <int DIM>), k_pair_tiles, (<DIM>), __launch_bounds__(kBlock, 4))
 
@@ -981,7 +1014,7 @@ CB_KERNEL_PAIR((template <int DIM>), k_pair_tiles, (<DIM>), __launch_bounds__(kB
 // rowStart[i] .. rowStart[i] + rowCount[i] (pairs grouped by i, j ascending
 // inside a row as the enumeration found them). Skipped when a row
 // overflowed its stash (the WRITE pass then writes the list).
-template <int DIM>
+template <int DIM, bool RES = false>
 __device__ __forceinline__ void k_pair_compact_body(const Bufs &b, const int vb, const int vg) {
     Ctrl *c = b.ctrl;
     if (c->stash_over) return;
@@ -1023,15 +1056,9 @@ __device__ __forceinline__ void k_pair_compact_body(const Bufs &b, const int vb,
             }
         }
     }
+    if (RES) return;
     if (last_block(&c->done[DC_MISC], vg) && threadIdx.x == 0) {
-        const int found = c->np_found;
-        if (found > pcap) {
-            c->status = CB_ERR_CAPACITY;
-            c->np = 0;
-        } else {
-            c->np = found;
-        }
-        c->need_search = 0;
+        search_end(c, pcap);
         c->done[DC_MISC] = 0;
     }
 }
@@ -1052,7 +1079,130 @@ __device__ __forceinline__ void k_degree_body(const Bufs &b, const int vb, const
 CB_KERNEL_PAIR((), k_degree, (), __launch_bounds__(kBlock))
 
 
+// Exclusive scan of in[0 ... count) to out[0 ... count], all blocks of a
+// resident search: the blocks' sums, a barrier, and every block its own
+// offset from them. Returns the total; the caller's next barrier publishes out.
+__device__ __forceinline__ int run_scan(const int *in, int *out, int count, int *blocksums,
+                                        RunCtx *rx, int vb, int vg) {
+    __shared__ int smem[32];
+    __shared__ int carry_s, total_s;
+    const int chunk = (count + vg - 1) / vg;
+    const int s = min(vb * chunk, count), e = min(s + chunk, count);
+    int v = 0;
+    for (int i = s + threadIdx.x; i < e; i += blockDim.x) v += in[i];
+    v = block_reduce_int(v, smem);
+    if (threadIdx.x == 0) __stcg(blocksums + vb, v);
+    run_barrier(rx);
+    int before = 0, all = 0;
+    for (int q = threadIdx.x; q < vg; q += blockDim.x) {
+        const int t = __ldcg(blocksums + q);
+        all += t;
+        if (q < vb) before += t;
+    }
+    before = block_reduce_int(before, smem);
+    all = block_reduce_int(all, smem);
+    if (threadIdx.x == 0) {
+        carry_s = before;
+        total_s = all;
+        if (vb == vg - 1) out[count] = all;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int base = s; base < e; base += blockDim.x) {
+        const int i = base + threadIdx.x;
+        const int w = i < e ? in[i] : 0;
+        int x = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += t;
+        }
+        if (lane == 31) smem[warp] = x;
+        __syncthreads();
+        int off = carry_s, sum = 0;
+        for (int q = 0; q < (int)(blockDim.x >> 5); q++) {
+            if (q < warp) off += smem[q];
+            sum += smem[q];
+        }
+        if (i < e) out[i] = off + x - w;
+        __syncthreads();
+        if (threadIdx.x == 0) carry_s += sum;
+        __syncthreads();
+    }
+    return total_s;
+}
+
+// The whole search of a small foam in one cooperative launch (common.cuh,
+// resident runs): the phases above with a grid barrier between them, their
+// decisions taken by every block in its own copy of the control block. The
+// launch per phase takes ~57 us whatever the size of a small foam (17 launches
+// of ~3.3 us), this one 41-56 us up to 3 10^4 bubbles, bound by the latency of
+// its eleven phases (~0.8 us a barrier, 1-2 us a phase).
+// `force`: a search asked for by the caller; otherwise only where the last
+// attempt left need_search.
+template <int DIM>
+__global__ void __launch_bounds__(kBlock, 2) k_search_run(Bufs b, const Bufs *foams,
+                                                       const RunBlock *map, Ctrl *mirror,
+                                                       long long force, int) {
+    __shared__ RunShared rs;
+    int vb = blockIdx.x, vg = gridDim.x;
+    if (map) {
+        const RunBlock w = map[blockIdx.x];
+        b = foams[w.foam];
+        vb = w.vb;
+        vg = w.vg;
+        if (!(b.ctrl->bsel & SEL_SEARCH)) return;
+    } else if (!force &&
+               (!b.ctrl->need_search || b.ctrl->need_delete || b.ctrl->status != CB_OK)) {
+        return;
+    }
+    Ctrl *ctrl = b.ctrl;
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, 0, 0.0, 0.0};
+    run_enter(&rs, b, -1);
+    Ctrl *c = &rs.c;
+    k_wrap_body<DIM, true>(b, vb, vg, &rx);
+    k_cell_count_body<DIM>(b, vb, vg);
+    run_barrier(&rx);
+    run_scan(b.cellCount, b.cellStart, c->ncell, b.blocksums, &rx, vb, vg);
+    run_barrier(&rx);
+    k_cell_fill_body(b, vb, vg);
+    run_barrier(&rx);
+    k_cell_order_body(b, vb, vg);
+    run_barrier(&rx);
+    k_permute_body<DIM, true>(b, vb, vg);
+    run_barrier(&rx);
+    k_pair_cells_body<DIM, false, true>(b, vb, vg, &rx);
+    if (DIM == 3) k_pair_tiles_body<DIM, true>(b, vb, vg, &rx);
+    k_pair_rows_body<DIM, true>(b, vb, vg, &rx);
+    run_barrier(&rx);
+    const int found = run_scan(b.rowCount, b.rowStart, c->n, b.blocksums, &rx, vb, vg);
+    if (threadIdx.x == 0) {
+        c->np_found = found;
+        c->stash_over = __ldcg(&rx.g->stash_over);
+    }
+    run_barrier(&rx);
+    if (!c->stash_over) {
+        k_pair_compact_body<DIM, true>(b, vb, vg);
+    } else {  // a row outgrew its stash: enumerated again
+        k_pair_cells_body<DIM, true, true>(b, vb, vg, &rx);
+        run_barrier(&rx);
+        if (threadIdx.x == 0) search_end(c, b.k->pcap);
+        __syncthreads();
+        k_degree_body(b, vb, vg);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) search_end(c, b.k->pcap);
+    run_exit(&rs, ctrl, mirror, &rx, vb);
+}
+
 }  // namespace
+
+void launch_search_run(const RunLaunch &r, const Bufs &b, int dim) {
+    if (dim == 3)
+        launch_coop(k_search_run<3>, r, b);
+    else
+        launch_coop(k_search_run<2>, r, b);
+}
 
 void launch_search(const Launch &l, const Bufs &b, int dim) {
     // G: kernels with a thread per bubble; W: with a warp per cell (2D foams

@@ -8,6 +8,7 @@ and deletion counts, bubbles and pairs; FP64 forms within 1e-11 of each row's
 maximum over 30 steps (the sums of ~10 terms per bubble differ by ~1e-15 of
 the row, growing along the run; the trajectory bar against the oracle is
 1e-9), the mixed form within 1e-6 (FP32 reductions)."""
+import numpy as np
 import pytest
 
 import cubble_gb300 as cb
@@ -120,3 +121,73 @@ def test_resident_batch_matches_batched_launches(dim, options, kw, precision):
         assert_rows_close(states[0][f], states[1][f], ["x", "y", "z", "r", "dxdt", "drdt", "path"],
                           1e-6 if precision == 1 else 1e-11, "batch ",
                           floor=position_ulp(states[1][f]))
+
+
+def dense_cluster(n, dim, seed):
+    """A crowd in one corner of a wide box: more than 24 bubbles per occupied
+    cell, rows beyond the partner stash."""
+    cfg, st = workloads.foam(n, dim, 0.9 if dim == 2 else 0.8, seed=seed)
+    rng = np.random.default_rng(seed)
+    for k in "xyz"[:dim]:
+        st[k][: n // 2] = 2.0 + rng.uniform(0.0, 4.0, n // 2)
+    return cfg, st
+
+
+# one to a few cells per axis (box sides from ~4 to ~100 units), walls, wide
+# cells (24 and more bubbles each), rows that outgrow their stash, odd sizes
+@pytest.mark.parametrize("n,dim,kind", [
+    (1, 2, "plain"), (2, 3, "plain"), (40, 2, "plain"), (60, 3, "plain"), (200, 3, "plain"),
+    (700, 3, "walls"), (2501, 2, "walls"), (5000, 3, "plain"), (9999, 2, "plain"),
+    (4001, 3, "wide"), (3001, 2, "wide"), (900, 3, "cluster"), (800, 2, "cluster"),
+    (50001, 3, "plain"), (99991, 2, "plain")])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_resident_search_matches_launch_per_phase(n, dim, kind, precision):
+    """One cooperative launch against a launch per phase: every row, the pair
+    list and the neighbour counts bit for bit."""
+    got = []
+    for cap in (n, 100001):  # the smallest capacity with a launch per phase
+        if kind == "cluster":
+            cfg, st = dense_cluster(n, dim, 17)
+        else:
+            cfg, st = workloads.foam(n, dim, 0.9 if dim == 2 else 0.8, seed=50 + n,
+                                     rstd=0.15, rclip=(0.3, 2.5),
+                                     wall=(1, 0, 1) if kind == "walls" else (0, 0, 0))
+        rng = np.random.default_rng(n)
+        for k in ("dxdt", "drdto", "path", "error"):
+            st[k] = rng.uniform(0.0, 1.0, n).astype(np.float32).astype(np.float64)
+        cfg.capacity, cfg.precision, cfg.pair_capacity = cap, precision, 400 * n + 100
+        f = cb.GpuFoam(cfg)
+        f.load_state(st)
+        if kind == "wide":
+            f.set_tuning(cell_scale=3.5)
+        for _ in range(2):  # the second one starts from a searched state
+            f.search_neighbors()
+        got.append((f.report(), f.get_state(), f.pairs()))
+        f.close()
+    (ra, sa, pa), (rb, sb, pb) = got
+    assert ra["searches"] == rb["searches"] == 2 and ra["num_pairs"] == rb["num_pairs"]
+    if kind == "cluster":
+        assert np.bincount(pa[0], minlength=1).max() > (32 if dim == 3 else 16)
+    for k in sa:
+        assert np.array_equal(sa[k], sb[k]), k
+    assert np.array_equal(pa[0], pb[0]) and np.array_equal(pa[1], pb[1])
+
+
+def test_resident_search_reports_a_full_pair_list():
+    """A pair list too small stops the run at the search that finds it, with
+    runs enqueued behind it."""
+    cfg, st = workloads.foam(3000, 2, 0.9, seed=12, use_graph=1, pair_capacity=20000)
+    probe = cb.GpuFoam(cfg)
+    probe.load_state(st)
+    probe.search_neighbors()
+    first = probe.report()["num_pairs"]
+    probe.close()
+    cfg.pair_capacity = first + 5  # the foam relaxes into more listed pairs
+    f = cb.GpuFoam(cfg)
+    f.load_state(st)
+    workloads.prepare(f)
+    with pytest.raises(cb.CubbleError) as e:
+        f.integrate(3000)
+    assert e.value.code == 3
+    r = f.report()
+    assert r["status"] == 3 and 0 < r["steps"] < 3000
