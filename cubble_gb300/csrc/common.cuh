@@ -106,6 +106,10 @@ struct DevConst {
 // end of a graph launch (one small copy).
 struct Ctrl {
     int n, np, ndel, status;
+    // delflag holds marks of an attempt that were not consumed by a deletion:
+    // the next correct kernel writes every flag; otherwise the flags are all
+    // zero before it and it writes the marks only
+    int marks, pad_marks;
     int use_gas, use_flow, inc_path, graph_mode;
     double dt;
     double sumA, sumAr, sumAo, sumAor;
@@ -562,6 +566,7 @@ __device__ __forceinline__ void attempt_decide(Ctrl *c, const DevConst &k, const
     c->max_exp = r.exp;
     c->vol_new = r.vol;
     c->ndel = gas ? r.del : 0;
+    c->marks = c->ndel > 0;
     c->attempts += 1;
     c->attempts_this_step += 1;
     c->dt = f.dt;

@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(kBlock) k_max_radius(const double *R, int n, C
 // Rows of a loaded state that the caller did not give, zeroed by one kernel
 // (a cudaMemsetAsync each, ~25 of them, took ~60 us of host time a load).
 struct ZeroRows {
-    int4 *row[ND_ROLES + NI_ROLES + 1];
-    unsigned quads[ND_ROLES + NI_ROLES + 1];  // 16-byte units
+    int4 *row[ND_ROLES + NI_ROLES + 2];
+    unsigned quads[ND_ROLES + NI_ROLES + 2];  // 16-byte units
     int rows = 0;
     void add(void *p, size_t bytes) {  // rows are allocated in whole 16-byte units
         row[rows] = static_cast<int4 *>(p);
@@ -792,12 +792,14 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
             zero.add(dst, (size_t)c->hk.cap * 4);
     }
     zero.add(c->bufs.acc, (size_t)kAcc * c->hk.cap * 8);
+    zero.add(c->bufs.delflag, (size_t)c->hk.cap * 4);
     k_zero_rows<<<std::min(c->launch.grid, c->launch.cover), kBlock, 0, c->stream>>>(zero);
     c->launches += 1;
     if ((rc = c->check_launch())) return rc;
     h.n = s->count;
     h.np = 0;
     h.ndel = 0;
+    h.marks = 0;
     h.status = CB_OK;
     h.max_bubble_radius = 0.0;
     h.too_large = h.need_search = h.need_delete = h.attempts_this_step = 0;
@@ -1222,6 +1224,7 @@ int profile_attempts(cb_context *c, int32_t reps, double ms[3]) {
     const int status = c->hctrl->status;
     *c->hctrl = saved;
     c->hctrl->status = status;
+    c->hctrl->marks = 1;  // the attempts may have left deletion marks
     return c->push();
 }
 

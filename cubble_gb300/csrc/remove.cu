@@ -89,8 +89,10 @@ __device__ __forceinline__ void k_remove_c_body(const Bufs &b, const int vb, con
     volMul = DIM == 3 ? rcbrt(volMul) : rsqrt(volMul);
     volMul *= k.vol_mul_const;
     double *R = drow(b, c, RR);
-    for (int i = vb * blockDim.x + threadIdx.x; i < nNew; i += stride)
-        R[i] = R[i] * volMul;
+    for (int i = vb * blockDim.x + threadIdx.x; i < n; i += stride) {
+        if (i < nNew) R[i] = R[i] * volMul;
+        b.delflag[i] = 0;  // for the next correct kernel (Ctrl::marks)
+    }
     if (last_block(&c->done[DC_REMOVE], vg) && threadIdx.x == 0) {
         swap_role(c->prole, PI0, PI1);
         swap_role(c->prole, PJ0, PJ1);
@@ -99,6 +101,7 @@ __device__ __forceinline__ void k_remove_c_body(const Bufs &b, const int vb, con
         c->deleted += D;
         c->delete_events += 1;
         c->ndel = 0;
+        c->marks = 0;
         c->need_delete = 0;
         c->pred_ready = 0;  // bubbles moved and radii rescaled
         c->pred_slot = 0;

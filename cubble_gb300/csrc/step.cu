@@ -550,6 +550,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     const int fixb = k.fix_b;
     long long merr = 0, mrad = 0, mexp = 0;
     double vol = 0.0;
+    const int marks = c->marks;
     int ndel = 0, bad = 0;
     for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
         double *acc = b.acc + (size_t)i * kAcc;
@@ -632,7 +633,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
             CB_D(RVP3)[i] = vpr;
             bad |= !finite_bits(cr);
         }
-        b.delflag[i] = del;
+        if (del | marks) b.delflag[i] = del;
         mexp = max_bits(mexp, dist);
         if (path)  // src/kernels.cu:437-451; the increment to ~2^-46
             CB_D(RPATHN)[i] = path0 + fx_norm<DIM>(fx_from_double(x0, fixb) - fx,

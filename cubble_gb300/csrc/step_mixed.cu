@@ -157,9 +157,12 @@ __device__ __forceinline__ PredMx ld_pred(const double *base, int i) {
 }
 
 __device__ __forceinline__ void st_pred(double *base, int i, const PredMx &r) {
-    longlong2 *p = reinterpret_cast<longlong2 *>(base) + 2 * (size_t)i;
-    p[0] = make_longlong2(r.q[0], r.q[1]);
-    p[1] = make_longlong2(r.q[2], r.qr);
+    longlong4_32a v;  // one 32-byte store: two 16-byte ones took k_predict_mx 34 us
+    v.x = r.q[0];     // instead of 31 (3D, N = 10^6)
+    v.y = r.q[1];
+    v.z = r.q[2];
+    v.w = r.qr;
+    reinterpret_cast<longlong4_32a *>(base)[i] = v;
 }
 
 // The predicted radius as FP32 (one rounding of the fixed-point value, which
@@ -744,6 +747,8 @@ __device__ __forceinline__ CorrRed block_reduce_corr(CorrRed v, CorrRed *smem) {
     return v;
 }
 
+// Three blocks per SM in 3D (80 registers; four, with 64 and spills, take
+// 151 us instead of 143 at N = 3 10^6), four in 2D (49 against 51 us at 10^6).
 // Grid-stride over the bubbles (one wave of blocks). The maxima and counts go
 // to the control block with integer atomics (order-independent); only the
 // volume sum keeps per-block partials for its in-order FP64 fold.
@@ -782,6 +787,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     long long merr = 0, mrad = 0;
     float mexp = 0.f;
     double vol = 0.0;
+    const int marks = c->marks;
     int ndel = 0, bad = 0;
     for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
         const float4 a = AV[i];
@@ -899,7 +905,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
             CB_F(RVP3)[i] = vpr;
             bad |= !finite_bits(cr);
         }
-        b.delflag[i] = del;
+        if (del | marks) b.delflag[i] = del;
         mexp = fmaxf(mexp, dist);
         const double ed = double_from_float(h * e);
         merr = max(merr, __double_as_longlong(ed));
@@ -1002,7 +1008,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     c->acnt_del = c->acnt_bad = 0;
     finish_attempt<DIM>(c, k, {fErr, fRad, fExp, fVol, (int)fDel, (int)fBad});
 }
-CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_mx, (<DIM, GAS, FLOW, WALLS>), __launch_bounds__(kBlock, 4))
+CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_mx, (<DIM, GAS, FLOW, WALLS>), __launch_bounds__(kBlock, DIM == 3 ? 3 : 4))
 
 
 // ----------------------------------------------------------- resident run
