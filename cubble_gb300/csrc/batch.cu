@@ -151,6 +151,7 @@ struct cb_batch {
     int gmax = 1;  // blocks of every batched launch
     RunBlock *drun = nullptr;  // resident run: what each of its blocks works on
     int run_blocks = 0;
+    bool run_wide = false;  // its form; k_search_run has the narrow map only
     long long launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -224,13 +225,17 @@ void launch_batch_search(const cb_batch *b, long long *counter) {
 // deletions and searches of all foams that need one run batched. kRunTotal
 // bounds the bubbles of all foams together.
 // ms per 100 steps on one GB300, one graph of batched launches -> resident
-// runs (sizes 10^3 ... 3 10^4 on a logarithmic ladder):
-//   16 2D foams (1.4 10^5 bubbles)  mixed 10.8 -> 3.2, FP64 16.7 -> 6.3
-//   64 2D foams (5.5 10^5)          mixed 17.3 -> 9.3, FP64 28.6 -> 21.1
-//   100 2D foams (8.6 10^5)         mixed 18.9 -> 15.7, FP64 41.0 -> 36.1
-//   48 3D foams (4.2 10^5)          mixed 20.7 -> 10.7, FP64 41.7 -> 23.8
-//   100 3D foams (8.6 10^5)         mixed 27.4 -> 25.7, FP64 61.0 -> 58.4
-constexpr long long kRunTotal = 1000000;
+// runs (sizes on a logarithmic ladder from 10^3 to 3 10^4, the last from
+// 2.9 10^3 to 8.7 10^4):
+//   16 2D foams (1.4 10^5 bubbles)  mixed 10.2 -> 3.0, FP64 15.3 -> 4.9
+//   64 2D foams (5.5 10^5)          mixed 16.4 -> 6.4, FP64 27.2 -> 13.8
+//   100 2D foams (8.6 10^5)         mixed 18.6 -> 9.5, FP64 30.8 -> 21.2
+//   150 2D foams (1.3 10^6)         mixed 25.1 -> 14.6, FP64 42.1 -> 34.8
+//   48 3D foams (4.2 10^5)          mixed 20.9 -> 7.5, FP64 37.3 -> 14.0
+//   100 3D foams (8.6 10^5)         mixed 27.6 -> 15.6, FP64 45.1 -> 29.4
+//   150 3D foams (1.3 10^6)         mixed 36.1 -> 24.4, FP64 64.4 -> 49.4
+//   150 3D foams (3.7 10^6)         mixed 73.5 -> 71.5, FP64 132 -> 143
+constexpr long long kRunTotal = 2000000;
 
 // The blocks of the foams: a warp per 32 items, as a single foam's run
 // (context.cu), scaled down where they would not all be resident.
@@ -240,14 +245,14 @@ int build_run_map(cb_batch *b) {
     long long total = 0;
     for (const cb_context *c : b->foams) total += c->hk.cap;
     if (total > kRunTotal) return CB_OK;
-    const int most = 2 * c0->sms;
     std::vector<double> want;
     double sum = 0.0;
     for (const cb_context *c : b->foams) {
-        const double items = (c->hk.dim == 3 ? 4.7 : 2.4) * c->hk.cap / (c->hk.mixed ? 2 : 1);
-        want.push_back(std::max(1.0, items / kBlock));
+        want.push_back(std::max(1.0, run_items(c) / kBlock));
         sum += want.back();
     }
+    b->run_wide = wide_run(sum * kBlock, c0->hk.mixed != 0, c0->sms);
+    const int most = c0->sms * (!b->run_wide ? kRunNarrow : (c0->hk.mixed ? kRunWideMx : kRunWide));
     const double scale = std::min(1.0, (most - (double)b->foams.size()) / sum);
     std::vector<RunBlock> map;
     for (int f = 0; f < (int)b->foams.size(); f++) {
@@ -266,6 +271,7 @@ RunLaunch batch_run_launch(cb_batch *b) {
     RunLaunch r;
     r.grid = b->run_blocks;
     r.block = kBlock;
+    r.wide = b->run_wide;
     r.threads = 0;
     r.stream = b->stream;
     r.steps = -1;
@@ -401,7 +407,7 @@ int batch_integrate(cb_batch *b, int64_t n_steps, cb_report *reports, double *ms
                 if ((rc = b->pull_bc())) return rc;
                 if (b->hbc->any_delete) launch_batch_remove(b, &b->launches);
                 if (b->hbc->any_search) {
-                    if (run)
+                    if (run && !b->run_wide)
                         launch_search_run(batch_run_launch(b), b->first()->bufs,
                                           b->first()->hk.dim);
                     else

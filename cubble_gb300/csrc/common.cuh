@@ -1069,12 +1069,17 @@ inline int wave_grid(K kernel, const Launch &l, int want = 0) {
     return g < l.grid ? g : l.grid;
 }
 
+// Blocks per SM of the resident runs' two forms: the narrow one, and the wide
+// one of the FP64 and of the mixed kernel.
+constexpr int kRunNarrow = 2, kRunWide = 3, kRunWideMx = 4;
+
 // Launch of a resident run: `steps` accepted steps from the control block's
 // count (< 0: to its steps_target) on `grid` blocks of `block` threads; the
 // control block is also written to `mirror` (pinned host memory) if given.
 // Batched: `foams` and `map` (device) say what every block works on.
 struct RunLaunch {
     int grid, block;
+    bool wide = false;  // the form with more blocks per SM
     int threads;  // of the correct kernel in a launch per phase (mixed form)
     cudaStream_t stream;
     long long steps;

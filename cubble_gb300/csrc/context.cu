@@ -249,21 +249,22 @@ namespace {
 
 // Contexts of up to this many bubbles run their attempts inside one
 // cooperative kernel (resident run, common.cuh); larger ones a launch per
-// phase. us per attempt on one GB300 (searches included), launches per phase
-// -> resident run:
-//   2D FP64   N = 10^3 52 -> 20, 10^4 52 -> 20, 2 10^5 97 -> 65, 5 10^5 162 -> 133
-//   2D mixed  N = 10^4 34 -> 15, 2 10^5 45 -> 35, 5 10^5 68 -> 64, 10^6 105 -> 114
-//   3D FP64   N = 4 10^3 53 -> 19, 3 10^4 59 -> 30, 3 10^5 145 -> 124,
-//             5 10^5 203 -> 195, 10^6 351 -> 359
-//   3D mixed  N = 4 10^3 34 -> 14, 3 10^5 67 -> 59, 5 10^5 95 -> 91, 10^6 150 -> 166
-// (two blocks per SM, the registers of the largest phase, against the four
-// blocks of the pair kernels: past the latency-bound sizes that costs more
-// than the launches).
-constexpr int kRunCapacity2 = 600000, kRunCapacity3 = 400000;
+// phase inside a graph. us per attempt on one GB300 (searches included),
+// launches per phase -> resident run:
+//   FP64  2D  N = 10^3 52 -> 15, 10^4 52 -> 17, 2 10^5 97 -> 48,
+//             10^6 194 -> 171, 3 10^6 462 -> 449
+//         3D  4 10^3 53 -> 15, 3 10^4 59 -> 22, 3 10^5 145 -> 84,
+//             10^6 260 -> 235, 3 10^6 657 -> 643, 6 10^6 1254 -> 1257
+//   mixed 2D  10^4 34 -> 14, 2 10^5 45 -> 31, 10^6 103 -> 91, 3 10^6 246 -> 235
+//         3D  4 10^3 34 -> 14, 3 10^5 67 -> 55, 10^6 148 -> 138,
+//             3 10^6 364 -> 359, 6 10^6 690 -> 684
+// (the launches up to 3 10^5 with the kernels they had before). Each launch
+// costs ~7 us of ramp, block partials and last-block fold in which the SMs are
+// mostly idle (19 % of k_pairs_mx at 10^6), a grid barrier ~1 us; at 6 10^6
+// that is lost in the noise.
+constexpr int kRunCapacity = 5000000;
 
-bool resident(const cb_context *c) {
-    return c->coop && c->hk.cap <= (c->hk.dim == 3 ? kRunCapacity3 : kRunCapacity2);
-}
+bool resident(const cb_context *c) { return c->coop && c->hk.cap <= kRunCapacity; }
 
 // Contexts of up to this many bubbles search in one cooperative launch
 // (k_search_run, search.cu). us per search, launches per phase -> one launch:
@@ -296,18 +297,19 @@ int run_search(cb_context *c) {
     return c->check_launch();
 }
 
-// Blocks and threads of a resident run: a warp per 32 items (the mixed form's
-// threads take two pairs) over as many SMs as that fills, at most two blocks
-// per SM; blocks of four warps while they reach, so that the warps of a small
-// foam spread over the SMs (N = 10^4, 2D: 20.1 us per attempt with four, 22.3
-// with two, 20.5 with eight).
+// Blocks and threads of a resident run: a warp per 32 items over as many SMs
+// as that fills, up to the resident blocks per SM of the kernel's form; blocks
+// of four warps while they reach, so that the warps of a small foam spread
+// over the SMs (N = 10^4, 2D: 20.1 us per attempt with four, 22.3 with two,
+// 20.5 with eight).
 RunLaunch run_launch(cb_context *c, int64_t n_steps) {
-    const double per = c->hk.dim == 3 ? 4.7 : 2.4;  // listed pairs per bubble
-    const int items = (int)(per * c->hk.cap) / (c->hk.mixed ? 2 : 1);
-    const int warps = std::max(1, (items + 31) / 32);
+    const double items = cbg::run_items(c);
+    const long long warps = std::max(1LL, (long long)(items + 31) / 32);
     RunLaunch r;
+    r.wide = cbg::wide_run(items, c->hk.mixed != 0, c->sms);
+    const int bps = !r.wide ? kRunNarrow : (c->hk.mixed ? kRunWideMx : kRunWide);
     r.block = warps <= 4 * 2 * c->sms ? 128 : kBlock;
-    r.grid = std::min(2 * c->sms, (32 * warps + r.block - 1) / r.block);
+    r.grid = (int)std::min<long long>(bps * c->sms, (32 * warps + r.block - 1) / r.block);
     r.threads = 4 * c->sms * kBlock;
     r.stream = c->stream;
     r.steps = n_steps;
@@ -392,6 +394,20 @@ int integrate_eager(cb_context *c, int64_t n_steps) {
 }  // namespace
 
 namespace cbg {
+// Work items of a foam's largest phase: its listed pairs (the mixed form's
+// threads take runs of four, counted as two each: fewer, longer chains).
+double run_items(const cb_context *c) {
+    const double per = c->hk.dim == 3 ? 4.7 : 2.4;  // listed pairs per bubble
+    return per * c->hk.cap / (c->hk.mixed ? 2 : 1);
+}
+// The form of a resident run with more blocks per SM and fewer registers, for
+// foams with several rounds of items. us per attempt, narrow / wide: FP64 3D
+// N = 3 10^4 21.7 / 22.7, 10^5 40.5 / 38.8, 10^6 267 / 236; mixed 3D 3 10^4
+// 17.0 / 17.6, 10^5 29.3 / 30.5, 5 10^5 95 / 80, 10^6 167 / 138.
+bool wide_run(double items, bool mixed, int sms) {
+    return items > (mixed ? 6.0 : 2.5) * kRunNarrow * sms * kBlock;
+}
+
 // Adds a conditional node to the graph that `stream` is capturing into and
 // returns its body graph; the capture continues after the node.
 int capture_conditional(cudaStream_t stream, cudaGraphConditionalNodeType type,

@@ -124,4 +124,6 @@ int capture_conditional(cudaStream_t stream, cudaGraphConditionalNodeType type,
 void fill_report(const cb_context *c, cb_report *r);
 int create_context(const cb_config *cfg, cb_context **out, bool graph);
 int apply_tuning(cb_context *c, const cb_tuning &t);
+bool wide_run(double items, bool mixed, int sms);
+double run_items(const cb_context *c);
 }  // namespace cbg

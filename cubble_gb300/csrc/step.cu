@@ -697,11 +697,12 @@ CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBloc
 
 
 // ----------------------------------------------------------- resident run
-// Attempts of a small foam inside one cooperative launch (see common.cuh).
-// Measured against the launch per phase, one GB300: see kRunCapacity
-// (context.cu).
-template <int DIM, bool GAS, bool FLOW>
-__global__ void __launch_bounds__(kBlock, 2) k_run(Bufs b, const Bufs *foams,
+// Attempts of a foam inside one cooperative launch (see common.cuh; where it
+// is taken and what it measured: kRunCapacity, context.cu). BPS blocks per SM:
+// two (128 registers) have the lower latency, three (80, some spills) the
+// higher throughput.
+template <int DIM, bool GAS, bool FLOW, int BPS>
+__global__ void __launch_bounds__(kBlock, BPS) k_run(Bufs b, const Bufs *foams,
                                                     const RunBlock *map, Ctrl *mirror,
                                                     long long n_steps, int threads) {
     __shared__ RunShared rs;
@@ -889,19 +890,22 @@ void launch_correct(const Launch &l, const Bufs &b, int dim) {
         CB_LAUNCH(l, k_correct, (<2>), wave_grid(k_correct<2>, l, l.step_bps), b);
 }
 
-void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode) {
+namespace {
+template <int DIM, int BPS>
+void launch_run_t(const RunLaunch &r, const Bufs &b, int mode) {
     const bool gas = mode & 1, flow = mode & 2;
-    if (dim == 3) {
-        if (gas && flow) launch_coop(k_run<3, true, true>, r, b);
-        else if (gas) launch_coop(k_run<3, true, false>, r, b);
-        else if (flow) launch_coop(k_run<3, false, true>, r, b);
-        else launch_coop(k_run<3, false, false>, r, b);
-    } else {
-        if (gas && flow) launch_coop(k_run<2, true, true>, r, b);
-        else if (gas) launch_coop(k_run<2, true, false>, r, b);
-        else if (flow) launch_coop(k_run<2, false, true>, r, b);
-        else launch_coop(k_run<2, false, false>, r, b);
-    }
+    if (gas && flow) launch_coop(k_run<DIM, true, true, BPS>, r, b);
+    else if (gas) launch_coop(k_run<DIM, true, false, BPS>, r, b);
+    else if (flow) launch_coop(k_run<DIM, false, true, BPS>, r, b);
+    else launch_coop(k_run<DIM, false, false, BPS>, r, b);
+}
+}  // namespace
+
+void launch_run(const RunLaunch &r, const Bufs &b, int dim, int mode) {
+    if (dim == 3)
+        r.wide ? launch_run_t<3, kRunWide>(r, b, mode) : launch_run_t<3, kRunNarrow>(r, b, mode);
+    else
+        r.wide ? launch_run_t<2, kRunWide>(r, b, mode) : launch_run_t<2, kRunNarrow>(r, b, mode);
 }
 
 void launch_boot(const Launch &l, const Bufs &b, int dim, int phase) {

@@ -1012,11 +1012,11 @@ CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_
 
 
 // ----------------------------------------------------------- resident run
-// Attempts of a small foam inside one cooperative launch (see common.cuh);
-// after an accepted attempt the next prediction is ready (two barriers then,
-// three otherwise).
-template <int DIM, bool GAS, bool FLOW, bool WALLS>
-__global__ void __launch_bounds__(kBlock, 2) k_run_mx(Bufs b, const Bufs *foams,
+// Attempts of a foam inside one cooperative launch (see common.cuh); after an
+// accepted attempt the next prediction is ready (two barriers then, three
+// otherwise). BPS blocks per SM: two (120 registers) or four (64).
+template <int DIM, bool GAS, bool FLOW, bool WALLS, int BPS>
+__global__ void __launch_bounds__(kBlock, BPS) k_run_mx(Bufs b, const Bufs *foams,
                                                     const RunBlock *map, Ctrl *mirror,
                                                     long long n_steps, int threads) {
     __shared__ RunShared rs;
@@ -1154,27 +1154,28 @@ void launch_correct_mx(const Launch &l, const Bufs &b, int dim, int mode, bool w
     }
 }
 
-void launch_run_mx(const RunLaunch &r, const Bufs &b, int dim, int mode, bool walls) {
+namespace {
+template <int DIM, int BPS, bool WALLS>
+void launch_run_mx_t(const RunLaunch &r, const Bufs &b, int mode) {
     const bool gas = mode & 1, flow = mode & 2;
-#define CB_RUN(D, G, F)                                   \
-    do {                                                  \
-        if (walls)                                        \
-            launch_coop(k_run_mx<D, G, F, true>, r, b);   \
-        else                                              \
-            launch_coop(k_run_mx<D, G, F, false>, r, b);  \
-    } while (0)
-    if (dim == 3) {
-        if (gas && flow) CB_RUN(3, true, true);
-        else if (gas) CB_RUN(3, true, false);
-        else if (flow) CB_RUN(3, false, true);
-        else CB_RUN(3, false, false);
-    } else {
-        if (gas && flow) CB_RUN(2, true, true);
-        else if (gas) CB_RUN(2, true, false);
-        else if (flow) CB_RUN(2, false, true);
-        else CB_RUN(2, false, false);
-    }
-#undef CB_RUN
+    if (gas && flow) launch_coop(k_run_mx<DIM, true, true, WALLS, BPS>, r, b);
+    else if (gas) launch_coop(k_run_mx<DIM, true, false, WALLS, BPS>, r, b);
+    else if (flow) launch_coop(k_run_mx<DIM, false, true, WALLS, BPS>, r, b);
+    else launch_coop(k_run_mx<DIM, false, false, WALLS, BPS>, r, b);
+}
+template <int DIM, int BPS>
+void launch_run_mx_w(const RunLaunch &r, const Bufs &b, int mode, bool walls) {
+    walls ? launch_run_mx_t<DIM, BPS, true>(r, b, mode) : launch_run_mx_t<DIM, BPS, false>(r, b, mode);
+}
+}  // namespace
+
+void launch_run_mx(const RunLaunch &r, const Bufs &b, int dim, int mode, bool walls) {
+    if (dim == 3)
+        r.wide ? launch_run_mx_w<3, kRunWideMx>(r, b, mode, walls)
+               : launch_run_mx_w<3, kRunNarrow>(r, b, mode, walls);
+    else
+        r.wide ? launch_run_mx_w<2, kRunWideMx>(r, b, mode, walls)
+               : launch_run_mx_w<2, kRunNarrow>(r, b, mode, walls);
 }
 
 void launch_boot_mx(const Launch &l, const Bufs &b, int dim, int phase) {

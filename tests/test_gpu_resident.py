@@ -17,7 +17,7 @@ from helpers import assert_rows_close, by_index, position_ulp
 
 pytestmark = pytest.mark.gpu
 
-BEYOND = {2: 600001, 3: 400001}  # the smallest capacity with a launch per phase
+BEYOND = 5000001  # the smallest capacity with a launch per phase
 
 OPTIONS = {
     "gas": {},
@@ -31,8 +31,8 @@ OPTIONS = {
 
 def both(n, dim, precision, options, **kw):
     out = []
-    for cap in (n, BEYOND[dim]):
-        args = dict(seed=300 + n, capacity=cap, pair_capacity=16 * BEYOND[dim] if cap > n else 0,
+    for cap in (n, BEYOND):
+        args = dict(seed=300 + n, capacity=cap, pair_capacity=16 * n + 64 if cap > n else 0,
                     precision=precision, use_graph=1)
         args.update(OPTIONS[options])
         args.update(kw)
@@ -48,11 +48,13 @@ def both(n, dim, precision, options, **kw):
 
 
 # one bubble; less, exactly and more than a warp; more than a block's threads;
-# a ragged size; more bubbles and pairs than the resident threads (two rounds)
+# a ragged size; more bubbles and pairs than the resident threads (two rounds);
+# the sizes around the change to more blocks per SM
 @pytest.mark.parametrize("n,dim,options", [
     (1, 2, "gas"), (31, 2, "gas"), (32, 3, "gas"), (33, 2, "settle"), (257, 3, "settle"),
     (4099, 3, "gas"), (4097, 3, "walls"), (3001, 3, "flow"), (2999, 2, "flow"),
-    (5003, 3, "shear"), (5000, 2, "shear"), (100003, 2, "gas"), (90001, 3, "gas")])
+    (5003, 3, "shear"), (5000, 2, "shear"), (100003, 2, "gas"), (90001, 3, "gas"),
+    (200003, 3, "walls"), (210001, 3, "shear"), (400009, 2, "flow"), (300007, 3, "settle")])
 @pytest.mark.parametrize("precision", [0, 1, 2])
 def test_resident_matches_launch_per_phase(n, dim, options, precision):
     a, b = both(n, dim, precision, options)
@@ -86,10 +88,11 @@ def test_resident_deletions_and_stops(precision):
 
 
 @pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("sizes", [(1, 700, 5003, 2048, 12001), (100, 40009, 1, 90007, 30000)])
 @pytest.mark.parametrize("dim,options,kw", [
     (2, "gas", {}), (3, "walls", {}), (3, "flow", {}),
     (2, "gas", dict(rstd=0.3, rclip=(0.01, 2.0), min_rad=0.2))])
-def test_resident_batch_matches_batched_launches(dim, options, kw, precision):
+def test_resident_batch_matches_batched_launches(dim, options, kw, sizes, precision):
     """A batch of small foams (resident: every foam its own blocks and loop)
     against the same batch with one foam's capacity beyond the resident
     total (the batched launches): the foams search, delete and finish at
@@ -101,7 +104,7 @@ def test_resident_batch_matches_batched_launches(dim, options, kw, precision):
         for f, n in enumerate(sizes):
             args = dict(seed=900 + f, kappa=0.01 * (f + 1), precision=precision, use_graph=1)
             if beyond and f == 3:
-                args.update(capacity=1000001, pair_capacity=16 * n)
+                args.update(capacity=BEYOND, pair_capacity=16 * n)
             args.update(OPTIONS[options])
             args.update(kw)
             items.append(workloads.foam(n, dim, 0.9 if dim == 2 else 0.8, **args))
