@@ -692,6 +692,8 @@ struct RunCtx {
     // this thread's share of the prediction's sums, reduced with the pair
     // phase's (FP64 form)
     double sA, sAr;
+    // mixed form, 2D, first thread: area_over_radius_2d of both kernels
+    double ar[2];
 };
 constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: seconds in all
 constexpr int kRunMaxAttempts = 1 << 15;   // per launch (bounds the arrival counter)

@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(kBlock, BPS) k_run(Bufs b, const Bufs *foams,
         if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
     }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0, {0.0, 0.0}};
     run_enter(&rs, b, n_steps);
     int attempts = 0;
     while (run_more(&rs, attempts)) {
