@@ -79,6 +79,8 @@ struct DevConst {
     // FP64 form: predicted positions and radii in units 2^-fix_b (fixpair.cuh)
     // and the periodic box length and half of it in those units
     long long flq[3], fhq[3];
+    // the same of the walls (box corners) and of the imposed flow's box
+    long long wlq[3], whq[3], vlq[3], vhq[3];
     double fix_unit;  // 2^-fix_b
     int fix_b;
     int mixed;

@@ -4,6 +4,7 @@
 // src/simulator.cu:219-221) or as a single CUDA graph whose while/if
 // conditional nodes are driven by the device (no host round trip per step).
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -43,6 +44,16 @@ std::atomic<unsigned long long> g_calls{0};
 
 
 namespace {
+
+// A wall or face of the flow's box in units 2^-b, held to the range of the
+// integers; `none` (a face no bubble is inside of) for NaN.
+long long fix_bound(double x, int b, long long none) {
+    const double v = std::ldexp(x, b);
+    if (std::isnan(v)) return none;
+    if (v >= 0x1p63) return LLONG_MAX;
+    if (v <= -0x1p63) return LLONG_MIN;
+    return std::llround(v);
+}
 
 void fill_const(cb_context *c) {
     DevConst &k = c->hk;
@@ -99,6 +110,10 @@ void fill_const(cb_context *c) {
         for (int a = 0; a < 3; a++) {
             k.flq[a] = (long long)std::llround(std::ldexp(k.iv[a], k.fix_b));
             k.fhq[a] = k.flq[a] / 2;
+            k.wlq[a] = fix_bound(k.lbb[a], k.fix_b, LLONG_MAX);
+            k.whq[a] = fix_bound(k.tfr[a], k.fix_b, LLONG_MIN);
+            k.vlq[a] = fix_bound(k.flow_lbb[a], k.fix_b, LLONG_MAX);
+            k.vhq[a] = fix_bound(k.flow_tfr[a], k.fix_b, LLONG_MIN);
         }
     }
     // Guard band of the FP32 pair prefilters. An FP32 coordinate carries up

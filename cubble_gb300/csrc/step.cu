@@ -424,74 +424,90 @@ CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs, (<DIM, GAS, F
 
 
 // ---------------------------------------------------------------- correct
-// touchesWall, src/kernels.cu:553-566
-__device__ __forceinline__ bool touches_wall(double f0, double rad, double x, double low,
-                                             double high, double &velocity) {
-    double d1 = x - low;
-    double d2 = x - high;
-    d1 = d1 * d1 < d2 * d2 ? d1 : d2;
-    if (rad * rad >= d1 * d1) {
-        d2 = d1 < 0.0 ? -1.0 : 1.0;
-        d1 *= d2;
-        velocity = d2 * f0 * (1.0 - d1 / rad);
-        return true;
-    }
-    return false;
+// |a - b| of fixed-point positions (any two of them)
+__device__ __forceinline__ unsigned long long fix_gap(long long a, long long b) {
+    const unsigned long long ua = (unsigned long long)a, ub = (unsigned long long)b;
+    return a > b ? ua - ub : ub - ua;
 }
+
+// The velocity of a bubble that touches a wall (touchesWall,
+// src/kernels.cu:553-566): d from the wall, which lies below or above it.
+static __device__ __noinline__ double wall_velocity(double f0, long long qr, unsigned long long d,
+                                                    bool below, int fixb) {
+    const double v = f0 * (1.0 - fx_to_double_any(d, -fixb) / fx_to_double_signed(qr, -fixb));
+    return below ? v : -v;
+}
+
+// 1 / (a number of neighbours), 0 for none (src/kernels.cu:500-502)
+constexpr int kInvCounts = 32;
+static __device__ const double kInvCount[kInvCounts] = {
+    0.0,      1.0 / 1,  1.0 / 2,  1.0 / 3,  1.0 / 4,  1.0 / 5,  1.0 / 6,  1.0 / 7,
+    1.0 / 8,  1.0 / 9,  1.0 / 10, 1.0 / 11, 1.0 / 12, 1.0 / 13, 1.0 / 14, 1.0 / 15,
+    1.0 / 16, 1.0 / 17, 1.0 / 18, 1.0 / 19, 1.0 / 20, 1.0 / 21, 1.0 / 22, 1.0 / 23,
+    1.0 / 24, 1.0 / 25, 1.0 / 26, 1.0 / 27, 1.0 / 28, 1.0 / 29, 1.0 / 30, 1.0 / 31};
+static __device__ __noinline__ double inv_count(int n) { return n > 0 ? 1.0 / (double)n : 0.0; }
 
 // Flow, shear and wall terms of the velocity (addFlowVelocity,
 // addWallVelocity, src/kernels.cu:497-593) as a call taken only when one of
 // them is on: inlined, their FP64 arithmetic would be predicated into every
-// bubble's path and take FP64 issue slots.
+// bubble's path and take FP64 issue slots. The tests of the flow's box and of
+// the walls are comparisons of the fixed-point positions (exact), 1/neighbours
+// comes from a table and only bubbles that touch a wall divide: two or three
+// FP64 instructions instead of ~55 for a bubble in a flow between walls.
 struct Vel3 {
     double x, y, z;
 };
 template <int DIM>
 static __device__ __noinline__ Vel3 boundary_velocity(const DevConst &k, int flow, int shear,
                                                       double drag, double vpx, double vpy,
-                                                      double vpz, double xp, double yp, double zp,
-                                                      double rp, double f0, double f1, double f2,
-                                                      int nn) {
+                                                      double vpz, long long qx, long long qy,
+                                                      long long qz, long long qr, double f0,
+                                                      double f1, double f2, int nn) {
+    const unsigned long long rad = fx_abs(qr);
+    const int fixb = k.fix_b;
     if (flow) {  // addFlowVelocity, src/kernels.cu:497-544
-        double multiplier = nn;
-        multiplier = (multiplier > 0 ? 1.0 / multiplier : 0.0);
-        const double riSq = rp * rp;
-        int inside = (int)((xp < k.flow_tfr[0] && xp > k.flow_lbb[0]) ||
-                           ((k.flow_lbb[0] - xp) * (k.flow_lbb[0] - xp) <= riSq) ||
-                           ((k.flow_tfr[0] - xp) * (k.flow_tfr[0] - xp) <= riSq));
-        inside *= (int)((yp < k.flow_tfr[1] && yp > k.flow_lbb[1]) ||
-                        ((k.flow_lbb[1] - yp) * (k.flow_lbb[1] - yp) <= riSq) ||
-                        ((k.flow_tfr[1] - yp) * (k.flow_tfr[1] - yp) <= riSq));
-        if (DIM == 3) {
-            inside *= (int)((zp < k.flow_tfr[2] && zp > k.flow_lbb[2]) ||
-                            ((k.flow_lbb[2] - zp) * (k.flow_lbb[2] - zp) <= riSq) ||
-                            ((k.flow_tfr[2] - zp) * (k.flow_tfr[2] - zp) <= riSq));
-            vpz += !inside * multiplier * f2 + k.flow_vel[2] * inside;
+        auto in_flow = [&](int a, long long q) {  // between the faces or touching one
+            return (q < k.vhq[a] && q > k.vlq[a]) || fix_gap(k.vlq[a], q) <= rad ||
+                   fix_gap(k.vhq[a], q) <= rad;
+        };
+        if (in_flow(0, qx) && in_flow(1, qy) && (DIM == 2 || in_flow(2, qz))) {
+            vpx += k.flow_vel[0];
+            vpy += k.flow_vel[1];
+            if (DIM == 3) vpz += k.flow_vel[2];
+        } else {
+            const double inv = (unsigned)nn < (unsigned)kInvCounts ? kInvCount[nn] : inv_count(nn);
+            vpx = fma(inv, f0, vpx);
+            vpy = fma(inv, f1, vpy);
+            if (DIM == 3) vpz = fma(inv, f2, vpz);
         }
-        vpx += !inside * multiplier * f0 + k.flow_vel[0] * inside;
-        vpy += !inside * multiplier * f1 + k.flow_vel[1] * inside;
     }
     if (shear) {  // linear shear along x over the last axis (cb_config.shear_speed)
-        const double q = DIM == 3 ? zp : yp;
+        const double q = fx_to_double_signed(DIM == 3 ? qz : qy, -fixb);
         vpx += k.shear * ((q - k.lbb[DIM - 1]) * k.shear_il - 1.0);
     }
     if (k.any_wall) {  // addWallVelocity, src/kernels.cu:546-593
         double xDrag = 1.0, yDrag = 1.0, velocity = 0.0;
-        if (k.wall[0] && touches_wall(k.f0, rp, xp, k.lbb[0], k.tfr[0], velocity)) {
+        auto touches = [&](int a, long long q) {  // the nearer wall, the upper one of two
+            const unsigned long long dl = fix_gap(q, k.wlq[a]), dh = fix_gap(q, k.whq[a]);
+            const bool low = dl < dh;
+            const unsigned long long d = low ? dl : dh;
+            if (d > rad) return false;
+            velocity = wall_velocity(k.f0, qr, d, q >= (low ? k.wlq[a] : k.whq[a]), fixb);
+            return true;
+        };
+        if (k.wall[0] && touches(0, qx)) {
             vpx += velocity;
             vpy *= drag;
             vpz *= drag;
             xDrag = drag;
         }
-        velocity = 0.0;
-        if (k.wall[1] && touches_wall(k.f0, rp, yp, k.lbb[1], k.tfr[1], velocity)) {
+        if (k.wall[1] && touches(1, qy)) {
             vpx *= drag;
             vpy += velocity * xDrag;
             vpz *= drag;
             yDrag = drag;
         }
-        velocity = 0.0;
-        if (k.wall[2] && touches_wall(k.f0, rp, zp, k.lbb[2], k.tfr[2], velocity)) {
+        if (k.wall[2] && touches(2, qz)) {
             vpx *= drag;
             vpy *= drag;
             vpz += velocity * xDrag * yDrag;
@@ -579,9 +595,8 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                         qz = DIM == 3 ? __double_as_longlong(p.z) : 0,
                         qr = __double_as_longlong(DIM == 3 ? p.w : p.z);
         if (flow | shear | k.any_wall) {
-            const State q = ld_state<DIM>(b, i, fixb);
-            const Vel3 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz, q.x, q.y,
-                                                  q.z, q.r, a1.y, a1.z, a1.w, flow ? NN[i] : 0);
+            const Vel3 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz, qx, qy, qz,
+                                                  qr, a1.y, a1.z, a1.w, flow ? NN[i] : 0);
             vpx = v.x;
             vpy = v.y;
             vpz = v.z;
