@@ -188,7 +188,7 @@ def allreduce(x, op, world):
     return float(t.item())
 
 
-def algorithmic_bytes(dim, np_per_n, mixed=False, ff=False):
+def algorithmic_bytes(dim, np_per_n, mixed=False):
     """Algorithmic HBM bytes per bubble of each attempt kernel.
 
     FP64 form, 3D: predict reads x,y,z,r, v x4, v_old x4 (96) and writes the
@@ -200,15 +200,7 @@ def algorithmic_bytes(dim, np_per_n, mixed=False, ff=False):
     Mixed form (FP32 rates, 32-byte fixed-point prediction, 20-byte FP32
     accumulators), 3D: predict 64 + 32, pairs 8 P/N + 32 + 20, correct
     132 + 88; step 176 + 8 P/N (q FP64 r/w 64, f FP32 r/w 32, f_old 16,
-    saved 32, path 16, error 16). The float-float form (CB_PRECISION_FP64_FF)
-    adds its 32-byte per-bubble records: written by predict, read by pairs
-    (which reads them instead of the 16-byte (1/r, r^2) row in 3D); the
-    step's compulsory traffic is the FP64 form's."""
-    if ff:
-        b = algorithmic_bytes(dim, np_per_n)
-        b["predict"] += 32.0
-        b["pairs"] += 32.0 - (16.0 if dim == 3 else 0.0)
-        return b
+    saved 32, path 16, error 16)."""
     if mixed:
         if dim == 3:
             return {"predict": 96.0, "pairs": 52.0 + 8.0 * np_per_n, "correct": 220.0,
@@ -378,12 +370,12 @@ def measure_form(args, world, rank, precision, clocks_on=True):
                  "deleted": qa1["deleted"] - qa0["deleted"],
                  "steps_per_search": (na / sa) if sa else None,
                  "what": "%d accepted steps after the timed ones, searches and deletions "
-                         "included, one graph launch, CUDA events" % na}
+                         "included, one call, CUDA events" % na}
     search_ms = sim.profile_search(reps=3)
     names = ["predict", "pairs", "correct"]
     top = int(np.argmax(kms))
     mixed = precision == 1
-    ab = algorithmic_bytes(dim, np_per_n, mixed=mixed, ff=precision == 2)
+    ab = algorithmic_bytes(dim, np_per_n, mixed=mixed)
     n_now = r1["count"]
     hbm, src = peaks()
     achieved = ab[names[top]] * n_now / (kms[top] * 1e-3) / 1e9
@@ -395,8 +387,7 @@ def measure_form(args, world, rank, precision, clocks_on=True):
     walls = int(any(cfg.wall[:dim]))
     kcorr = ("k_correct_mx<%d, %d, %d, %d>" % (dim, gas, flow, walls) if mixed
              else "k_correct<%d>" % dim)
-    kpairs = "k_pairs%s<%d, %d, %d>" % (sfx if mixed else ("_ff" if precision == 2 else ""),
-                                        dim, gas, flow)
+    kpairs = "k_pairs%s<%d, %d, %d>" % (sfx, dim, gas, flow)
     if mixed:  # the mixed pair kernel's pairs per thread (a template argument)
         run = tuning["pair_run"] if (gas and not flow) else 4
         kpairs = "k_pairs_mx<%d, %d, %d, %d>" % (dim, gas, flow, run)
@@ -414,10 +405,9 @@ def measure_form(args, world, rank, precision, clocks_on=True):
             "algorithmic_bytes_per_bubble": ab,
             "step_achieved_gbs": step_gbs, "step_frac": step_gbs / hbm}
     fp64 = profiled_metric(kname, "FP64 pipe % active")
-    if fp64 and precision == 0:
-        # the FP64 form is bound by FP64 issue (2 FP64 thread-instructions per
-        # SM and cycle on GB300), not by HBM: the ncu pipe utilisation says how
-        # close the dominant kernel is to that bound
+    if fp64 and not mixed:
+        # 2 FP64 thread-instructions per SM and cycle on GB300: the ncu pipe
+        # utilisation says how close the dominant kernel is to that bound
         roof["fp64_issue_bound"] = {"pipe_active_frac": fp64[0] / 100.0,
                                     "source": "%s (ncu sm__pipe_fp64_cycles_active of %s)"
                                               % (fp64[1], kname)}
@@ -429,7 +419,7 @@ def measure_form(args, world, rank, precision, clocks_on=True):
 
 
 def form_errors(args, precision=1, steps=50):
-    """Per-quantity error of another form (mixed, or the float-float FP64
+    """Per-quantity error of another form (mixed, or the second FP64
     form) against the FP64 form (which matches the FP64 oracle within 1e-12
     per step) from the same prepared state: one attempt, then `steps`
     accepted steps."""
@@ -915,10 +905,8 @@ def run_gb300(args, world, rank, local):
                    "attempts": fx["r1"]["attempts"] - fx["r0"]["attempts"],
                    "searches": fx["r1"]["searches"] - fx["r0"]["searches"],
                    "roofline": fx["roofline"], "gpu_launches": fx["launches"],
-                   "dtype": "f64 state and update; pair terms in float-float (2 x f32)",
-                   "workload": "same foam, CB_PRECISION_FP64_FF: the FP64 form with the pair "
-                               "kernel's distance, velocities, gas flux and overlap areas in "
-                               "float-float (~2^-46 relative) on the FP32 pipe"}
+                   "dtype": "f64 (pair terms in 64-bit fixed point)",
+                   "workload": "same foam, CB_PRECISION_FP64_FF: the FP64 form's kernels"}
         if rank == 0:
             fp64_ff["error_vs_fp64"] = form_errors(args, 2)
 
@@ -949,7 +937,7 @@ def run_gb300(args, world, rank, local):
         "metric": METRIC, "value": value, "unit": "bubble-steps/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * el / args.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": {0: "f64", 1: "f64/f32 mixed", 2: "f64 + float-float (2 x f32) pair terms"}[
+        "dtype": {0: "f64", 1: "f64/f32 mixed", 2: "f64"}[
             args.precision],
         "data": "synthetic (seeded, uniform positions)",
         "config": {"workload": desc,
