@@ -671,16 +671,16 @@ __device__ void finish_attempt(Ctrl *c, const DevConst &k, const AttemptResult &
 }
 
 // ---------------------------------------------------------- resident runs
-// Small foams run their attempts inside one cooperative kernel (k_run in
-// step.cu, k_run_mx in step_mixed.cu): the three attempt bodies in a loop with
+// Foams (up to kRunCapacity bubbles, context.cu) run their attempts inside one
+// cooperative kernel (k_run in step.cu, k_run_mx in step_mixed.cu): the three attempt bodies in a loop with
 // a grid barrier after each, until a bubble has to be deleted, the neighbours
 // searched, or the steps are done. At N = 10^4 an attempt's arithmetic takes
 // about 2 us, its three launches (a wave of ~600-1200 blocks each, every one
 // with a fence and an atomic on the same counter) and the two condition nodes
 // 55 us. The control block, the constants and the row tables live in shared
-// memory, one identical copy per block: every block folds all partials in the
-// same order after the barrier and takes the same decisions, so no second
-// barrier publishes them; block 0 writes the control block back at the end.
+// memory, one identical copy per block: every block reads the same reduced
+// values after the barrier and takes the same decisions, so no second barrier
+// publishes them; block 0 writes the control block back at the end.
 //
 // The launch is cooperative (all blocks resident), so every arrival comes;
 // still each wait is bounded, and a block that gives up tells the others.

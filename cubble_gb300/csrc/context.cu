@@ -340,7 +340,7 @@ int run_attempt(cb_context *c) {
 }
 
 
-// integrate() of a small foam: resident runs of attempts, each until a
+// integrate() by resident runs of attempts, each until a
 // deletion, a search or the end; the control block comes back with the run.
 // Expects hctrl to hold the device's control block. A long stretch enqueues
 // several runs, each with the search it may end in (neither does anything

@@ -70,7 +70,7 @@ typedef struct cb_config {
     int32_t precision;       /* CB_PRECISION_*                             */
     int32_t use_graph;       /* 1 = run cb_integrate as one CUDA graph with
                                 device-side conditional loops (contexts
-                                beyond 4 10^5 (3D) / 6 10^5 (2D) bubbles;
+                                beyond 5 10^6 bubbles;
                                 smaller ones run their attempts inside one
                                 cooperative kernel either way)             */
     double lbb[3];           /* lower back bottom corner of the box        */
@@ -228,8 +228,8 @@ typedef struct cb_stop {
 } cb_stop;
 
 /* Up to max_steps accepted steps (integrate() calls), ending after the
- * first step that meets a condition of *stop; checked on the device, so a
- * graph context runs the whole stretch as one graph launch. The caller
+ * first step that meets a condition of *stop; checked on the device, so the
+ * whole stretch runs without the host. The caller
  * reads which condition held from the report (time, count, max_radius). */
 CB_API int cb_integrate_until(cb_context *ctx, int64_t max_steps, const cb_stop *stop,
                               cb_report *report);

@@ -1,4 +1,4 @@
-"""GPU: resident runs (small contexts: every attempt of a stretch inside one
+"""GPU: resident runs (every attempt of a stretch inside one
 cooperative kernel) against the launch per phase that larger contexts take.
 
 The same foam is run in a context of its own size (resident) and in one whose
