@@ -32,6 +32,7 @@ struct BatchCtl {
     int graph_mode;
     int any_attempt, any_delete, any_search;
     long long decides, any_delete_phases, any_search_phases;
+    RunRound round;  // of resident runs
 };
 
 // Block-wide exclusive scan of one int per thread (blockDim.x a multiple of
@@ -120,6 +121,10 @@ __global__ void __launch_bounds__(1024) k_batch_decide(const Bufs *bb, int count
         bc->any_attempt = act;
         bc->any_delete = del;
         bc->any_search = srch;
+        bc->round.stopped = 0;
+        bc->round.last = bc->round.longest;
+        bc->round.longest = 0;
+        bc->round.active = max(carry[0][0], 1);
         if (!init) {
             bc->decides += 1;
             bc->any_delete_phases += del;
@@ -151,6 +156,7 @@ struct cb_batch {
     int gmax = 1;  // blocks of every batched launch
     RunBlock *drun = nullptr;  // resident run: what each of its blocks works on
     int run_blocks = 0;
+    long long run_total = 0;  // bubbles of all foams
     bool run_wide = false;  // its form; k_search_run has the narrow map only
     long long launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -222,26 +228,39 @@ void launch_batch_search(const cb_batch *b, long long *counter) {
 // Batches of small foams advance by resident runs (common.cuh): one
 // cooperative launch in which every foam has its own blocks, barrier and loop
 // and runs its attempts until its own deletion, search or end; then the
-// deletions and searches of all foams that need one run batched. kRunTotal
-// bounds the bubbles of all foams together.
+// deletions and searches of all foams that need one run batched. A foam that
+// could go on leaves its run once the others have waited long enough
+// (RunWait, common.cuh). kRunTotal bounds the bubbles of all foams together.
 // ms per 100 steps on one GB300, one graph of batched launches -> resident
-// runs (sizes on a logarithmic ladder from 10^3 to 3 10^4, the last from
-// 2.9 10^3 to 8.7 10^4):
-//   16 2D foams (1.4 10^5 bubbles)  mixed 10.2 -> 3.0, FP64 15.3 -> 4.9
-//   64 2D foams (5.5 10^5)          mixed 16.4 -> 6.4, FP64 27.2 -> 13.8
-//   100 2D foams (8.6 10^5)         mixed 18.6 -> 9.5, FP64 30.8 -> 21.2
-//   150 2D foams (1.3 10^6)         mixed 25.1 -> 14.6, FP64 42.1 -> 34.8
-//   48 3D foams (4.2 10^5)          mixed 20.9 -> 7.5, FP64 37.3 -> 14.0
-//   100 3D foams (8.6 10^5)         mixed 27.6 -> 15.6, FP64 45.1 -> 29.4
-//   150 3D foams (1.3 10^6)         mixed 36.1 -> 24.4, FP64 64.4 -> 49.4
-//   150 3D foams (3.7 10^6)         mixed 73.5 -> 71.5, FP64 132 -> 143
+// runs (sizes on a logarithmic ladder):
+//   16 2D foams, 10^3 ... 3 10^4 (1.4 10^5 bubbles)   mixed 10.2 -> 2.9, FP64 15.3 -> 5.1
+//   100 2D foams, the same       (8.6 10^5)           mixed 18.6 -> 9.0, FP64 30.8 -> 19.9
+//   100 3D foams, the same                            mixed 27.6 -> 15.0, FP64 45.1 -> 28.1
+//   304 2D foams of 10^3         (3.0 10^5)           mixed 13.4 -> 3.9, FP64 19.3 -> 8.9
+//   256 3D foams, 3 10^3 ... 1.5 10^4 (1.9 10^6)      mixed 45.4 -> 32.9, FP64 75.9 -> 64.5
+//   64 3D foams, 1.2 10^4 ... 1.2 10^5 (3.0 10^6)     mixed 60.4 -> 48.1, FP64 105 -> 88
+//   300 3D foams of 8000         (2.4 10^6)           mixed 51.0 -> 39.0, FP64 84 -> 91
+// ms per 1000 steps while a foam deletes a bubble every ~10 of them, launches
+// -> runs that wait for the last foam -> runs left early: 100 2D foams mixed
+// 238 -> 237 -> 130, FP64 365 -> 495 -> 235; 100 3D mixed 452 -> 542 -> 380; 16 2D
+// mixed 131 -> 86 -> 60.
+//
+// Where even the longest run of a round is short, the waiting and the round cost
+// more than the launches: kApart attempts of all foams together follow then (in
+// batches large enough not to be bound by launches). 100 3D mixed foams of 1.8
+// 10^6 bubbles, ms per 1000 steps with 34 and 115 deletions a step: batched
+// launches 588 and 780, runs 642 and 872, with this switch
+// 580 and 790 (every 16).
+constexpr long long kApartTotal = 500000;
+constexpr int kApartLongest = 4, kApart = 64;
 constexpr long long kRunTotal = 2000000;
 
 // The blocks of the foams: a warp per 32 items, as a single foam's run
 // (context.cu), scaled down where they would not all be resident.
 int build_run_map(cb_batch *b) {
     const cb_context *c0 = b->first();
-    if (!c0->coop || (int)b->foams.size() > c0->sms) return CB_OK;
+    if (!c0->coop) return CB_OK;
+    const int foams = (int)b->foams.size();
     long long total = 0;
     for (const cb_context *c : b->foams) total += c->hk.cap;
     if (total > kRunTotal) return CB_OK;
@@ -251,19 +270,31 @@ int build_run_map(cb_batch *b) {
         want.push_back(std::max(1.0, run_items(c) / kBlock));
         sum += want.back();
     }
-    b->run_wide = wide_run(sum * kBlock, c0->hk.mixed != 0, c0->sms);
+    b->run_wide = foams > c0->sms || wide_run(sum * kBlock, c0->hk.mixed != 0, c0->sms);
     const int most = c0->sms * (!b->run_wide ? kRunNarrow : (c0->hk.mixed ? kRunWideMx : kRunWide));
-    const double scale = std::min(1.0, (most - (double)b->foams.size()) / sum);
+    if (foams > most - c0->sms) return CB_OK;
+    // the fewest rounds of items per thread that the resident blocks allow
+    auto blocks = [&](double rounds) {
+        long long n = 0;
+        for (double w : want) n += (long long)std::ceil(w / rounds);
+        return n;
+    };
+    double low = 1.0, rounds = std::max(1.0, sum);  // one block per foam at `sum`
+    if (blocks(low) <= most) rounds = low;
+    while (rounds - low > 1e-3 * low) {
+        const double mid = 0.5 * (low + rounds);
+        (blocks(mid) <= most ? rounds : low) = mid;
+    }
     std::vector<RunBlock> map;
-    for (int f = 0; f < (int)b->foams.size(); f++) {
-        const int vg = std::max(1, (int)std::ceil(want[f] * scale));
+    for (int f = 0; f < foams; f++) {
+        const int vg = (int)std::ceil(want[f] / rounds);
         for (int v = 0; v < vg; v++) map.push_back({f, v, vg});
     }
-    if ((int)map.size() > most) return CB_OK;
     CB_CUDA(cudaMalloc(&b->drun, sizeof(RunBlock) * map.size()));
     CB_CUDA(cudaMemcpy(b->drun, map.data(), sizeof(RunBlock) * map.size(),
                        cudaMemcpyHostToDevice));
     b->run_blocks = (int)map.size();
+    b->run_total = total;
     return CB_OK;
 }
 
@@ -279,6 +310,7 @@ RunLaunch batch_run_launch(cb_batch *b) {
     r.launches = &b->launches;
     r.foams = b->dbufs;
     r.map = b->drun;
+    r.round = &b->dbc->round;
     return r;
 }
 
@@ -398,13 +430,19 @@ int batch_integrate(cb_batch *b, int64_t n_steps, cb_report *reports, double *ms
         if (graph) {
             CB_CUDA(cudaGraphLaunch(b->gexec, b->stream));
         } else {
+            int apart = 0;  // attempts of all foams together before the next runs
             for (;;) {
-                if (run)
+                const bool runs = run && apart == 0;
+                if (runs)
                     launch_batch_run(b);
                 else
                     launch_batch_attempt(b, &b->launches);
                 CB_CUDA(cudaGetLastError());
                 if ((rc = b->pull_bc())) return rc;
+                if (!runs && apart > 0)
+                    apart--;
+                else if (runs && b->run_total > kApartTotal && b->hbc->round.last <= kApartLongest)
+                    apart = kApart;
                 if (b->hbc->any_delete) launch_batch_remove(b, &b->launches);
                 if (b->hbc->any_search) {
                     if (run && !b->run_wide)

@@ -173,6 +173,7 @@ struct RunAcc {
     double csum[5];      // correct: volume; mixed form: the candidates' sums
     long long cmax[3];   // correct: error, radius, expansion (bits of doubles >= 0)
     int cnt[2];          // correct: deletions, non-finite values
+    int leave, pad0_;    // batched run: end the run after this attempt
 };
 struct RunSync {
     RunAcc acc[2];  // of even and odd attempts
@@ -696,6 +697,7 @@ struct RunCtx {
     double sA, sAr;
     // mixed form, 2D, first thread: area_over_radius_2d of both kernels
     double ar[2];
+    int *leave;  // shared; batched runs only
 };
 constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: seconds in all
 constexpr int kRunMaxAttempts = 1 << 15;   // per launch (bounds the arrival counter)
@@ -837,8 +839,36 @@ struct RunShared {
     double *ds[ND_ROLES];
     int *is[NI_ROLES];
     int *ps[NP_ROLES];
-    int failed;
+    int failed, leave;
 };
+
+// A round of resident runs of a batch: the foams that have stopped (each at
+// its own deletion, search or end) of those that take part, and the attempts of
+// the longest run (of the round before: `last`).
+struct RunRound {
+    int stopped, active, longest, last;
+};
+// When a foam ends its run although it could go on, because others wait: once
+// the waiting adds up to about what a round costs beyond its attempts (the
+// decision and the batched deletions and searches, ~100 us). Kept by the first
+// thread of the foam's first block.
+struct RunWait {
+    float idle = 0.f;
+    long long last = 0;
+    int stopped = 0;
+};
+constexpr float kRoundCycles = 400000.f;
+__device__ __forceinline__ void run_wait_look(RunWait *w, const RunRound *round, int vb) {
+    if (round && vb == 0 && threadIdx.x == 0) w->stopped = __ldcg(&round->stopped);
+}
+__device__ __forceinline__ void run_wait_add(RunWait *w, const RunRound *round, int vb,
+                                             RunAcc *acc) {
+    if (!round || vb != 0 || threadIdx.x != 0) return;
+    const long long now = clock64();
+    if (w->last) w->idle += (float)(now - w->last) * (float)w->stopped;
+    w->last = now;
+    if (w->idle > kRoundCycles * (float)round->active) atomicAdd(&acc->leave, 1);
+}
 
 template <typename T>
 __device__ __forceinline__ void run_copy(T *dst, const T *src) {
@@ -856,6 +886,7 @@ __device__ __forceinline__ void run_enter(RunShared *s, Bufs &b, long long n_ste
     __syncthreads();
     if (threadIdx.x == 0) {
         s->failed = 0;
+        s->leave = 0;
         s->c.graph_mode = 0;
         if (n_steps >= 0) s->c.steps_target = s->c.steps + n_steps;
     }
@@ -874,7 +905,7 @@ __device__ __forceinline__ void run_enter(RunShared *s, Bufs &b, long long n_ste
 // first thread before the decision.
 template <int DIM, typename F>
 __device__ __forceinline__ void run_finish(Ctrl *c, const DevConst &k, const RunAcc *g, double dt,
-                                           F extra) {
+                                           int *leave, F extra) {
     if (threadIdx.x == 0 || threadIdx.x == 32) {
         AttemptResult r;
         r.err = __longlong_as_double(__ldcg(&g->cmax[0]));
@@ -885,6 +916,7 @@ __device__ __forceinline__ void run_finish(Ctrl *c, const DevConst &k, const Run
         r.bad = __ldcg(&g->cnt[1]);
         const AttemptFate f = attempt_fate(true, false, k, dt, r);
         if (threadIdx.x == 0) {
+            if (leave) *leave = __ldcg(&g->leave);
             extra();
             attempt_decide<DIM>(c, k, r, f);
         } else {
@@ -903,6 +935,7 @@ __device__ __forceinline__ bool run_more(const RunShared *s, int attempts) {
     if (attempts == 0)
         return c.steps < c.steps_target && !c.need_delete && !c.need_search && !c.stop_hit;
     if (c.too_large) return true;
+    if (s->leave) return false;
     return !c.need_delete && !c.need_search && c.steps < c.steps_target && !c.stop_hit;
 }
 
@@ -922,10 +955,14 @@ __device__ __forceinline__ void run_clear_other(RunCtx *rx, int vb) {
 // Block 0 writes the control block to `ctrl` and, if given, to the host's
 // mirror; the last block out clears the accumulators and the barrier.
 __device__ __forceinline__ void run_exit(RunShared *s, Ctrl *ctrl, Ctrl *mirror, RunCtx *rx,
-                                         int vb) {
+                                         int vb, RunRound *round = nullptr, int attempts = 0) {
     __shared__ bool last;
     __syncthreads();
     if (threadIdx.x == 0 && s->failed) s->c.status = CB_ERR_CUDA;
+    if (round && vb == 0 && threadIdx.x == 0) {
+        atomicAdd(&round->stopped, 1);
+        atomicMax(&round->longest, attempts);
+    }
     __syncthreads();
     if (vb == 0)
         for (int w = threadIdx.x; w < (int)(sizeof(Ctrl) / 4); w += blockDim.x) {
@@ -1091,6 +1128,7 @@ struct RunLaunch {
     long long *launches;
     const Bufs *foams = nullptr;
     const RunBlock *map = nullptr;
+    RunRound *round = nullptr;
 };
 template <typename K>
 inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
@@ -1103,7 +1141,7 @@ inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, b, r.foams, r.map, r.mirror, r.steps, r.threads);
+    cudaLaunchKernelEx(&cfg, kernel, b, r.foams, r.map, r.round, r.mirror, r.steps, r.threads);
     *r.launches += 1;
 }
 

@@ -1142,7 +1142,7 @@ __device__ __forceinline__ int run_scan(const int *in, int *out, int count, int 
 // attempt left need_search.
 template <int DIM>
 __global__ void __launch_bounds__(kBlock, 2) k_search_run(Bufs b, const Bufs *foams,
-                                                       const RunBlock *map, Ctrl *mirror,
+                                                       const RunBlock *map, RunRound *, Ctrl *mirror,
                                                        long long force, int) {
     __shared__ RunShared rs;
     int vb = blockIdx.x, vg = gridDim.x;

@@ -690,7 +690,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         const int cn[2] = {ndel, bad};
         run_reduce<1, 3, 2>(&vol, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm);
         run_barrier(rx);
-        run_finish<DIM>(c, k, rx->acc, ts, [] {});
+        run_finish<DIM>(c, k, rx->acc, ts, rx->leave, [] {});
         return;
     }
     long long *lsm = reinterpret_cast<long long *>(smem);
@@ -729,7 +729,7 @@ CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBloc
 // higher throughput.
 template <int DIM, bool GAS, bool FLOW, int BPS>
 __global__ void __launch_bounds__(kBlock, BPS) k_run(Bufs b, const Bufs *foams,
-                                                    const RunBlock *map, Ctrl *mirror,
+                                                    const RunBlock *map, RunRound *round, Ctrl *mirror,
                                                     long long n_steps, int threads) {
     __shared__ RunShared rs;
     __shared__ RunRed rsm;
@@ -742,19 +742,23 @@ __global__ void __launch_bounds__(kBlock, BPS) k_run(Bufs b, const Bufs *foams,
         if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
     }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0, {0.0, 0.0}};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0, {0.0, 0.0}, nullptr};
     run_enter(&rs, b, n_steps);
+    if (round) rx.leave = &rs.leave;
+    RunWait wait;
     int attempts = 0;
     while (run_more(&rs, attempts)) {
         run_begin(&rx, attempts);
         k_predict_body<DIM, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
+        run_wait_look(&wait, round, vb);
         k_pairs_body<DIM, GAS, FLOW, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
+        run_wait_add(&wait, round, vb, rx.acc);
         k_correct_body<DIM, true>(b, vb, vg, &rx, &rsm);
         attempts++;
     }
-    run_exit(&rs, ctrl, mirror, &rx, vb);
+    run_exit(&rs, ctrl, mirror, &rx, vb, round, attempts);
 }
 
 // --------------------------------------------------------------- bootstrap

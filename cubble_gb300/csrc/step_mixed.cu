@@ -968,7 +968,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
         run_reduce<1, 3, 2, kS>(&vol, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm, sv);
         run_barrier(rx);
         const RunAcc *g = rx->acc;
-        run_finish<DIM>(c, k, g, c->dt, [&] {
+        run_finish<DIM>(c, k, g, c->dt, rx->leave, [&] {
             const double a0 = __ldcg(&g->csum[1]), a1 = __ldcg(&g->csum[2]);
             double r0 = __ldcg(&g->csum[3]), r1 = __ldcg(&g->csum[4]);
             if (DIM == 2) r0 = r1 = rx->ar[1];
@@ -1017,7 +1017,7 @@ CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_
 // otherwise). BPS blocks per SM: two (120 registers) or four (64).
 template <int DIM, bool GAS, bool FLOW, bool WALLS, int BPS>
 __global__ void __launch_bounds__(kBlock, BPS) k_run_mx(Bufs b, const Bufs *foams,
-                                                    const RunBlock *map, Ctrl *mirror,
+                                                    const RunBlock *map, RunRound *round, Ctrl *mirror,
                                                     long long n_steps, int threads) {
     __shared__ RunShared rs;
     __shared__ RunRed rsm;
@@ -1033,23 +1033,27 @@ __global__ void __launch_bounds__(kBlock, BPS) k_run_mx(Bufs b, const Bufs *foam
     // threads of the launch per phase (area_over_radius_2d): the virtual grid
     // of a batched foam, else four resident blocks per SM
     RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed,
-              map ? b.ctrl->vgrid_a * kBlock : threads, 0.0, 0.0, {0.0, 0.0}};
+              map ? b.ctrl->vgrid_a * kBlock : threads, 0.0, 0.0, {0.0, 0.0}, nullptr};
     run_enter(&rs, b, n_steps);
     if (DIM == 2 && threadIdx.x == 0) {  // once: a run ends where bubbles are deleted
         rx.ar[0] = area_over_radius_2d<false>(rs.c.n, rx.threads);
         rx.ar[1] = area_over_radius_2d<true>(rs.c.n, rx.threads);
     }
+    if (round) rx.leave = &rs.leave;
+    RunWait wait;
     int attempts = 0;
     while (run_more(&rs, attempts)) {
         run_begin(&rx, attempts);
         k_predict_mx_body<DIM, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
+        run_wait_look(&wait, round, vb);
         k_pairs_mx_body<DIM, GAS, FLOW, 4, true>(b, vb, vg, &rx, &rsm);
         __syncthreads();
+        run_wait_add(&wait, round, vb, rx.acc);
         k_correct_mx_body<DIM, GAS, FLOW, WALLS, true>(b, vb, vg, &rx, &rsm);
         attempts++;
     }
-    run_exit(&rs, ctrl, mirror, &rx, vb);
+    run_exit(&rs, ctrl, mirror, &rx, vb, round, attempts);
 }
 
 // --------------------------------------------------------------- bootstrap

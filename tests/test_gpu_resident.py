@@ -104,7 +104,7 @@ def test_resident_batch_matches_batched_launches(dim, options, kw, sizes, precis
         for f, n in enumerate(sizes):
             args = dict(seed=900 + f, kappa=0.01 * (f + 1), precision=precision, use_graph=1)
             if beyond and f == 3:
-                args.update(capacity=BEYOND, pair_capacity=16 * n)
+                args.update(capacity=6000001, pair_capacity=16 * n)
             args.update(OPTIONS[options])
             args.update(kw)
             items.append(workloads.foam(n, dim, 0.9 if dim == 2 else 0.8, **args))
