@@ -91,22 +91,24 @@ def test_resident_deletions_and_stops(precision):
 @pytest.mark.parametrize("sizes", [(1, 700, 5003, 2048, 12001), (100, 40009, 1, 90007, 30000)])
 @pytest.mark.parametrize("dim,options,kw", [
     (2, "gas", {}), (3, "walls", {}), (3, "flow", {}),
-    (2, "gas", dict(rstd=0.3, rclip=(0.01, 2.0), min_rad=0.2))])
+    (2, "gas", dict(rstd=0.3, rclip=(0.01, 2.0), min_rad=0.2)),
+    (2, "gas", dict(rstd=0.3, rclip=(0.01, 2.0), min_rad=0.3, capacity=130000))])
 def test_resident_batch_matches_batched_launches(dim, options, kw, sizes, precision):
     """A batch of small foams (resident: every foam its own blocks and loop)
     against the same batch with one foam's capacity beyond the resident
     total (the batched launches): the foams search, delete and finish at
-    different attempts."""
-    sizes = (1, 700, 5003, 2048, 12001)
+    different attempts. The larger foams take the runs with more blocks per SM;
+    capacities above 5 10^5 in all let short rounds alternate with attempts of
+    all foams together."""
     reports, states, launches = [], [], []
     for beyond in (0, 1):
         items = []
         for f, n in enumerate(sizes):
             args = dict(seed=900 + f, kappa=0.01 * (f + 1), precision=precision, use_graph=1)
-            if beyond and f == 3:
-                args.update(capacity=6000001, pair_capacity=16 * n)
             args.update(OPTIONS[options])
             args.update(kw)
+            if beyond and f == 3:
+                args.update(capacity=6000001, pair_capacity=16 * n)
             items.append(workloads.foam(n, dim, 0.9 if dim == 2 else 0.8, **args))
         batch = cb.GpuFoamBatch([c for c, _ in items])
         for (_, st), f in zip(items, batch.foams):
