@@ -901,8 +901,9 @@ __device__ __forceinline__ void run_enter(RunShared *s, Bufs &b, long long n_ste
 // After the correct phase's barrier: the attempt's reduced values and what
 // follows from them, by two threads of different warps (one after the other
 // in one thread they took 1700 cycles of ~27,000 of an attempt). dt is the
-// attempt's; the status is CB_OK and no_accept 0 in a run. `extra` runs in the
-// first thread before the decision.
+// attempt's, read from the control block before the phase's barrier: here one
+// of the two threads writes the next one there. The status is CB_OK and
+// no_accept 0 in a run. `extra` runs in the first thread before the decision.
 template <int DIM, typename F>
 __device__ __forceinline__ void run_finish(Ctrl *c, const DevConst &k, const RunAcc *g, double dt,
                                            int *leave, F extra) {

@@ -767,7 +767,8 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     __syncthreads();
 #define CB_D(r) reinterpret_cast<double *>(tab_ptr(tab, r))
 #define CB_F(r) reinterpret_cast<float *>(tab_ptr(tab, r))
-    const float h = float_rn_from_double(0.5 * c->dt);
+    const double ts = c->dt;  // a run's decision changes c->dt (run_finish)
+    const float h = float_rn_from_double(0.5 * ts);
     const int path = c->inc_path;
     float4 *AV = acc_v(b);
     float *AO = acc_ov(b, cap);
@@ -782,7 +783,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     const long long minr = __double_as_longlong(k.min_rad);
     const bool shear = c->use_flow && k.shear_on;
     // the two dt the next attempt can have after an accept (finish_attempt)
-    const float hI = float_rn_from_double(0.5 * (c->dt * 1.269));
+    const float hI = float_rn_from_double(0.5 * (ts * 1.269));
     float cA0 = 0.f, cA1 = 0.f, cAr0 = 0.f, cAr1 = 0.f;
     long long merr = 0, mrad = 0;
     float mexp = 0.f;
@@ -968,7 +969,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
         run_reduce<1, 3, 2, kS>(&vol, m, cn, rx->acc->csum, rx->acc->cmax, rx->acc->cnt, rsm, sv);
         run_barrier(rx);
         const RunAcc *g = rx->acc;
-        run_finish<DIM>(c, k, g, c->dt, rx->leave, [&] {
+        run_finish<DIM>(c, k, g, ts, rx->leave, [&] {
             const double a0 = __ldcg(&g->csum[1]), a1 = __ldcg(&g->csum[2]);
             double r0 = __ldcg(&g->csum[3]), r1 = __ldcg(&g->csum[4]);
             if (DIM == 2) r0 = r1 = rx->ar[1];
