@@ -703,7 +703,12 @@ constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: second
 constexpr int kRunMaxAttempts = 1 << 15;   // per launch (bounds the arrival counter)
 constexpr unsigned kRunGaveUp = 1u << 28;  // added to the arrivals by a block that gave up
 
-__device__ __forceinline__ void run_barrier(RunCtx *rx) {
+// false (the same in every thread of a block) where a wait gave up: now, or at
+// an earlier barrier. The arrivals stay beyond every phase from then on, so
+// the blocks that still come to a barrier leave it at once. An attempt's phases
+// may go on regardless (they only read and write rows of the foam); what
+// follows an index that another block had to publish must not.
+__device__ __forceinline__ bool run_barrier(RunCtx *rx) {
     __syncthreads();
     if (threadIdx.x == 0) {
         rx->phase += rx->vg;
@@ -720,6 +725,7 @@ __device__ __forceinline__ void run_barrier(RunCtx *rx) {
         if (past < 0 || past >= (int)(kRunGaveUp / 2)) *rx->failed = 1;
     }
     __syncthreads();
+    return !*rx->failed;
 }
 
 // First item of this thread of block vb of vg (stride vg * blockDim.x). A
@@ -954,7 +960,8 @@ __device__ __forceinline__ void run_clear_other(RunCtx *rx, int vb) {
 }
 
 // Block 0 writes the control block to `ctrl` and, if given, to the host's
-// mirror; the last block out clears the accumulators and the barrier.
+// mirror; the last block out clears the accumulators and the barrier, and
+// reports a wait that gave up in a block that block 0 has not heard of.
 __device__ __forceinline__ void run_exit(RunShared *s, Ctrl *ctrl, Ctrl *mirror, RunCtx *rx,
                                          int vb, RunRound *round = nullptr, int attempts = 0) {
     __shared__ bool last;
@@ -976,9 +983,14 @@ __device__ __forceinline__ void run_exit(RunShared *s, Ctrl *ctrl, Ctrl *mirror,
         last = atomicAdd(&rx->g->exits, 1u) == rx->vg - 1;
     }
     __syncthreads();
-    if (last)
-        for (int w = threadIdx.x; w < (int)(sizeof(RunSync) / 4); w += blockDim.x)
-            reinterpret_cast<int *>(rx->g)[w] = 0;
+    if (!last) return;
+    if (threadIdx.x == 0 && __ldcg(&rx->g->arrive) >= kRunGaveUp) {  // any block did
+        ctrl->status = CB_ERR_CUDA;
+        if (mirror) mirror->status = CB_ERR_CUDA;
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < (int)(sizeof(RunSync) / 4); w += blockDim.x)
+        reinterpret_cast<int *>(rx->g)[w] = 0;
 }
 
 // ------------------------------------------------------ kernel launchers

@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(kBlock) k_max_radius(const double *R, int n, C
 // Rows of a loaded state that the caller did not give, zeroed by one kernel
 // (a cudaMemsetAsync each, ~25 of them, took ~60 us of host time a load).
 struct ZeroRows {
-    int4 *row[ND_ROLES + NI_ROLES + 2];
-    unsigned quads[ND_ROLES + NI_ROLES + 2];  // 16-byte units
+    int4 *row[ND_ROLES + NI_ROLES + 4];
+    unsigned quads[ND_ROLES + NI_ROLES + 4];  // 16-byte units
     int rows = 0;
     void add(void *p, size_t bytes) {  // rows are allocated in whole 16-byte units
         row[rows] = static_cast<int4 *>(p);
@@ -824,6 +824,10 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
     }
     zero.add(c->bufs.acc, (size_t)kAcc * c->hk.cap * 8);
     zero.add(c->bufs.delflag, (size_t)c->hk.cap * 4);
+    if (h.status == CB_ERR_CUDA) {  // a resident search that gave up leaves its counts
+        zero.add(c->bufs.cellCount, ((size_t)c->hk.ccap + 1) * 4);
+        zero.add(c->bufs.cellFill, ((size_t)c->hk.ccap + 1) * 4);
+    }
     k_zero_rows<<<std::min(c->launch.grid, c->launch.cover), kBlock, 0, c->stream>>>(zero);
     c->launches += 1;
     if ((rc = c->check_launch())) return rc;

@@ -139,8 +139,9 @@ __device__ __forceinline__ void search_end(Ctrl *c, int pcap) {
 }
 
 // RES here and below: as a phase of the resident search (k_search_run).
+// false: the resident search's barrier gave up.
 template <int DIM, bool RES = false>
-__device__ __forceinline__ void k_wrap_body(const Bufs &b, const int vb, const int vg,
+__device__ __forceinline__ bool k_wrap_body(const Bufs &b, const int vb, const int vg,
                                             RunCtx *rx = nullptr) {
     __shared__ double smem[32];
     Ctrl *c = b.ctrl;
@@ -179,11 +180,11 @@ __device__ __forceinline__ void k_wrap_body(const Bufs &b, const int vb, const i
     const long long bm = block_max_bits(mr, reinterpret_cast<long long *>(smem));
     if (RES) {
         if (threadIdx.x == 0) atomicMax(&rx->g->search_max, bm);
-        run_barrier(rx);
+        if (!run_barrier(rx)) return false;
         if (threadIdx.x == 0)
             search_begin(c, k, __longlong_as_double(__ldcg(&rx->g->search_max)));
         __syncthreads();
-        return;
+        return true;
     }
     if (threadIdx.x == 0) b.part[7 * vg + vb] = __longlong_as_double(bm);
     if (last_block(&c->done[DC_WRAP], vg)) {
@@ -193,6 +194,7 @@ __device__ __forceinline__ void k_wrap_body(const Bufs &b, const int vb, const i
             c->done[DC_WRAP] = 0;
         }
     }
+    return true;
 }
 CB_KERNEL_PAIR((template <int DIM>), k_wrap, (<DIM>), __launch_bounds__(kBlock))
 
@@ -1081,7 +1083,8 @@ CB_KERNEL_PAIR((), k_degree, (), __launch_bounds__(kBlock))
 
 // Exclusive scan of in[0 ... count) to out[0 ... count], all blocks of a
 // resident search: the blocks' sums, a barrier, and every block its own
-// offset from them. Returns the total; the caller's next barrier publishes out.
+// offset from them. Returns the total (-1: the barrier gave up); the caller's
+// next barrier publishes out.
 __device__ __forceinline__ int run_scan(const int *in, int *out, int count, int *blocksums,
                                         RunCtx *rx, int vb, int vg) {
     __shared__ int smem[32];
@@ -1092,7 +1095,7 @@ __device__ __forceinline__ int run_scan(const int *in, int *out, int count, int 
     for (int i = s + threadIdx.x; i < e; i += blockDim.x) v += in[i];
     v = block_reduce_int(v, smem);
     if (threadIdx.x == 0) __stcg(blocksums + vb, v);
-    run_barrier(rx);
+    if (!run_barrier(rx)) return -1;
     int before = 0, all = 0;
     for (int q = threadIdx.x; q < vg; q += blockDim.x) {
         const int t = __ldcg(blocksums + q);
@@ -1132,6 +1135,47 @@ __device__ __forceinline__ int run_scan(const int *in, int *out, int count, int 
     return total_s;
 }
 
+// The phases of the resident search. Each takes indexes that the blocks of the
+// one before it published, so a barrier that gave up ends the search here
+// (run_exit then reports it).
+template <int DIM>
+__device__ __forceinline__ void search_phases(const Bufs &b, int vb, int vg, RunCtx *rx) {
+    Ctrl *c = b.ctrl;
+    if (!k_wrap_body<DIM, true>(b, vb, vg, rx)) return;
+    k_cell_count_body<DIM>(b, vb, vg);
+    if (!run_barrier(rx)) return;
+    if (run_scan(b.cellCount, b.cellStart, c->ncell, b.blocksums, rx, vb, vg) < 0) return;
+    if (!run_barrier(rx)) return;
+    k_cell_fill_body(b, vb, vg);
+    if (!run_barrier(rx)) return;
+    k_cell_order_body(b, vb, vg);
+    if (!run_barrier(rx)) return;
+    k_permute_body<DIM, true>(b, vb, vg);
+    if (!run_barrier(rx)) return;
+    k_pair_cells_body<DIM, false, true>(b, vb, vg, rx);
+    if (DIM == 3) k_pair_tiles_body<DIM, true>(b, vb, vg, rx);
+    k_pair_rows_body<DIM, true>(b, vb, vg, rx);
+    if (!run_barrier(rx)) return;
+    const int found = run_scan(b.rowCount, b.rowStart, c->n, b.blocksums, rx, vb, vg);
+    if (found < 0) return;
+    if (threadIdx.x == 0) {
+        c->np_found = found;
+        c->stash_over = __ldcg(&rx->g->stash_over);
+    }
+    if (!run_barrier(rx)) return;
+    if (!c->stash_over) {
+        k_pair_compact_body<DIM, true>(b, vb, vg);
+    } else {  // a row outgrew its stash: enumerated again
+        k_pair_cells_body<DIM, true, true>(b, vb, vg, rx);
+        if (!run_barrier(rx)) return;
+        if (threadIdx.x == 0) search_end(c, b.k->pcap);
+        __syncthreads();
+        k_degree_body(b, vb, vg);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) search_end(c, b.k->pcap);
+}
+
 // The whole search of a small foam in one cooperative launch (common.cuh,
 // resident runs): the phases above with a grid barrier between them, their
 // decisions taken by every block in its own copy of the control block. The
@@ -1159,39 +1203,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_search_run(Bufs b, const Bufs *fo
     Ctrl *ctrl = b.ctrl;
     RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, 0, 0.0, 0.0};
     run_enter(&rs, b, -1);
-    Ctrl *c = &rs.c;
-    k_wrap_body<DIM, true>(b, vb, vg, &rx);
-    k_cell_count_body<DIM>(b, vb, vg);
-    run_barrier(&rx);
-    run_scan(b.cellCount, b.cellStart, c->ncell, b.blocksums, &rx, vb, vg);
-    run_barrier(&rx);
-    k_cell_fill_body(b, vb, vg);
-    run_barrier(&rx);
-    k_cell_order_body(b, vb, vg);
-    run_barrier(&rx);
-    k_permute_body<DIM, true>(b, vb, vg);
-    run_barrier(&rx);
-    k_pair_cells_body<DIM, false, true>(b, vb, vg, &rx);
-    if (DIM == 3) k_pair_tiles_body<DIM, true>(b, vb, vg, &rx);
-    k_pair_rows_body<DIM, true>(b, vb, vg, &rx);
-    run_barrier(&rx);
-    const int found = run_scan(b.rowCount, b.rowStart, c->n, b.blocksums, &rx, vb, vg);
-    if (threadIdx.x == 0) {
-        c->np_found = found;
-        c->stash_over = __ldcg(&rx.g->stash_over);
-    }
-    run_barrier(&rx);
-    if (!c->stash_over) {
-        k_pair_compact_body<DIM, true>(b, vb, vg);
-    } else {  // a row outgrew its stash: enumerated again
-        k_pair_cells_body<DIM, true, true>(b, vb, vg, &rx);
-        run_barrier(&rx);
-        if (threadIdx.x == 0) search_end(c, b.k->pcap);
-        __syncthreads();
-        k_degree_body(b, vb, vg);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) search_end(c, b.k->pcap);
+    search_phases<DIM>(b, vb, vg, &rx);
     run_exit(&rs, ctrl, mirror, &rx, vb);
 }
 
