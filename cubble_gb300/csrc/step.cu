@@ -638,7 +638,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 area = times4(ri.y);
             } else {
                 inv = p.w;
-                area = kPi * fx_to_double((unsigned long long)qr, -fixb);
+                area = kPi * fx_to_double_signed(qr, -fixb);
             }
             double vr = mfa - inv;
             vr *= mfb * (area - ov);
