@@ -3,9 +3,10 @@
 // GB300 issues FP64 at 1/64 of its FP32 rate; one FP64 instruction costs the
 // issue slots of about 64 others, a 64-bit integer product about ten. The
 // predicted positions and radii of the FP64 form are therefore kept as
-// integers q = x 2^B (|x| < 2P, P the power of two that bounds the box
-// corners, B = 62 - log2 P: never coarser than the doubles they come from
-// except below 2^-9 P, where the unit stays 2^-53 of P / 2^9). Differences are
+// integers q = x 2^B (|x| < P, P the power of two that bounds the box corners
+// with an eighth to spare, B = 62 - log2 P: never coarser than the doubles they
+// come from except below 2^-9 P, where the unit stays 2^-53 of P / 2^9; a
+// bubble beyond P is taken in FP64). Differences are
 // then exact, the minimum image an integer compare, and the distance, the
 // reciprocals and the products of a pair run in integers normalised to the
 // pair's own scale R = r1 + r2:
@@ -57,6 +58,17 @@ CB_HD int64_t fx_from_double(double x, int B) {
         q = sh <= 10 ? m << sh : 0x7fffffffffffffffull;
     else
         q = sh >= -53 ? ((m >> (-sh - 1)) + 1) >> 1 : 0;
+    return (hi & 0x80000000u) ? -(int64_t)q : (int64_t)q;
+}
+
+// The same for |x| < 2^(62 - B), where differences of two results fit too;
+// beyond (NaN too) `far` is set and the result means nothing.
+CB_HD int64_t fx_from_double(double x, int B, bool &far) {
+    const uint32_t hi = ff_dhi(x), lo = ff_dlo(x);
+    const int sh = (int)((hi >> 20) & 0x7ffu) - 1075 + B;
+    const uint64_t m = ((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+    far |= sh > 9;
+    const uint64_t q = sh >= 0 ? m << (sh & 63) : sh >= -53 ? ((m >> (-sh - 1)) + 1) >> 1 : 0;
     return (hi & 0x80000000u) ? -(int64_t)q : (int64_t)q;
 }
 

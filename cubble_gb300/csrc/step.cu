@@ -24,27 +24,51 @@ __device__ __forceinline__ double4_32a ld4(const double *p, int i) {
 }
 
 // The packed predicted state of bubble i (positions and radius as fixed point,
-// fixpair.cuh; 2D: 1/r beside them): written and read back. The way back is
-// exact: the integer has no more bits than the double it was rounded from.
-template <int DIM>
-__device__ __forceinline__ void st_state(const Bufs &b, int i, double x, double y, double z,
-                                         double r, double inv, int fixb) {
-    double4_32a p;
-    const double qr = __longlong_as_double(fx_from_double(r, fixb));
-    p.x = __longlong_as_double(fx_from_double(x, fixb));
-    p.y = __longlong_as_double(fx_from_double(y, fixb));
-    p.z = DIM == 3 ? __longlong_as_double(fx_from_double(z, fixb)) : qr;
-    p.w = DIM == 3 ? qr : inv;
-    reinterpret_cast<double4_32a *>(b.pred)[i] = p;
+// fixpair.cuh; 2D: 1/r beside them): written and read back. A bubble that the
+// fixed point does not hold (it lies beyond the range after a large dt or as it
+// was loaded, or is NaN) has a marked record, and its state in the rows of the
+// corrected state, which are free until the correct kernel writes them: its
+// terms are then evaluated in FP64 (pair_far, far_moves and RealPlace below).
+constexpr long long kFarRecord = (long long)0x8000000000000000ULL;
+__device__ __forceinline__ bool is_far(double4_32a p) {  // |q| < 2^62 in the others
+    return __double2hiint(p.x) == (int)0x80000000;
 }
 struct State {
-    double x, y, z, r, inv;  // inv in 2D only
+    double x, y, z, r;
 };
 template <int DIM>
-__device__ __forceinline__ State ld_state(const Bufs &b, int i, int fixb) {
-    const double4_32a p = ld4(b.pred, i);
+static __device__ __noinline__ void st_far(double *const *ds, const Ctrl *c, int i, double x,
+                                           double y, double z, double r) {
+    ds[c->drole[RXN]][i] = x;
+    ds[c->drole[RYN]][i] = y;
+    if (DIM == 3) ds[c->drole[RZN]][i] = z;
+    ds[c->drole[RRN]][i] = r;
+}
+template <int DIM>
+__device__ __forceinline__ void st_state(const Bufs &b, const Ctrl *c, int i, double x, double y,
+                                         double z, double r, double inv, int fixb) {
+    double4_32a p;
+    bool far = false;
+    const double qr = __longlong_as_double(fx_from_double(r, fixb, far));
+    p.x = __longlong_as_double(fx_from_double(x, fixb, far));
+    p.y = __longlong_as_double(fx_from_double(y, fixb, far));
+    p.z = DIM == 3 ? __longlong_as_double(fx_from_double(z, fixb, far)) : qr;
+    p.w = DIM == 3 ? qr : inv;
+    if (far) {
+        p.x = __longlong_as_double(kFarRecord);
+        st_far<DIM>(b.ds, c, i, x, y, z, r);
+    }
+    reinterpret_cast<double4_32a *>(b.pred)[i] = p;
+}
+template <int DIM>
+__device__ __forceinline__ State ld_state(const double *pred, double *const *ds, const Ctrl *c,
+                                          int i, int fixb) {
+    const double4_32a p = ld4(pred, i);
+    if (is_far(p))
+        return {ds[c->drole[RXN]][i], ds[c->drole[RYN]][i],
+                DIM == 3 ? ds[c->drole[RZN]][i] : 0.0, ds[c->drole[RRN]][i]};
     auto back = [&](double q) { return fx_to_double_signed(__double_as_longlong(q), -fixb); };
-    return {back(p.x), back(p.y), DIM == 3 ? back(p.z) : 0.0, back(DIM == 3 ? p.w : p.z), p.w};
+    return {back(p.x), back(p.y), DIM == 3 ? back(p.z) : 0.0, back(DIM == 3 ? p.w : p.z)};
 }
 
 // ---------------------------------------------------------------- predict
@@ -76,7 +100,7 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
         const double rsq = rp * rp;
         const double zp = DIM == 3 ? fma(h, fma(3.0, V2[i], -O2[i]), Z[i]) : 0.0;
         if (DIM == 3) reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
-        st_state<DIM>(b, i, xp, yp, zp, rp, inv, fixb);
+        st_state<DIM>(b, c, i, xp, yp, zp, rp, inv, fixb);
         if (gas) {  // area and area per radius, src/kernels.cu:103-112, with
                     // the constant factor (4 pi, 2 pi) applied to the block sums
             if (DIM == 3) {
@@ -238,6 +262,55 @@ static __device__ __noinline__ double pair_slow(long long ex, long long ey, long
     return fabs(fma(-0.25 * w, w, r2sq));
 }
 
+// A listed pair with a member that the fixed point does not hold, in FP64 from
+// the states to both bubbles' rows. Returns the overlap (in units of ov_unit)
+// and the overlap times the sum of 1/r.
+template <int DIM, bool GAS, bool FLOW>
+static __device__ __noinline__ double2 pair_far(const double *pred, const double *invr, double *acc,
+                                                double *const *ds, const Ctrl *c,
+                                                const DevConst *kp, int i, int j) {
+    const DevConst &k = *kp;
+    const State a = ld_state<DIM>(pred, ds, c, i, k.fix_b), q = ld_state<DIM>(pred, ds, c, j, k.fix_b);
+    double dx = a.x - q.x, dy = a.y - q.y, dz = DIM == 3 ? a.z - q.z : 0.0;
+    if (!k.wall[0]) dx = min_image(dx, k.half_iv[0], k.iv[0]);
+    if (!k.wall[1]) dy = min_image(dy, k.half_iv[1], k.iv[1]);
+    if (DIM == 3 && !k.wall[2]) dz = min_image(dz, k.half_iv[2], k.iv[2]);
+    const double m = DIM == 3 ? fma(dz, dz, fma(dy, dy, dx * dx)) : fma(dy, dy, dx * dx);
+    const double radii = a.r + q.r;
+    if (radii * radii < m) return make_double2(0.0, 0.0);  // NaN: counted in
+    const double y = rsqrt_d(m), s = (y - rcp_d(radii)) * k.f0;
+    double *ai = acc + (size_t)i * kAcc, *aj = acc + (size_t)j * kAcc;
+    const double f[3] = {dx * s, dy * s, dz * s};
+#pragma unroll
+    for (int t = 0; t < DIM; t++) {
+        red_add(ai + t, f[t]);
+        red_add(aj + t, neg_bits(f[t]));
+    }
+    if (FLOW) {
+        static constexpr int kV[3] = {RV0, RV1, RV2};
+#pragma unroll
+        for (int t = 0; t < DIM; t++) red_add(ai + 5 + t, ds[c->drole[kV[t]]][j]);
+    }
+    if (!GAS) return make_double2(0.0, 0.0);
+    const double inv1 = DIM == 3 ? invr[2 * (size_t)i] : pred[4 * (size_t)i + 3];
+    const double inv2 = DIM == 3 ? invr[2 * (size_t)j] : pred[4 * (size_t)j + 3];
+    const double r1sq = a.r * a.r, r2sq = q.r * q.r;
+    double oa;
+    if (m < r1sq || m < r2sq) {
+        oa = fmin(r1sq, r2sq);
+    } else {
+        const double w = (r2sq - r1sq + m) * y;
+        oa = fabs(fma(-0.25 * w, w, r2sq));
+    }
+    if (DIM == 2) oa = sqrt(oa);
+    const double g = oa * (inv2 - inv1);
+    red_add(ai + 3, g);
+    red_add(aj + 3, neg_bits(g));
+    red_add(ai + 4, oa);
+    red_add(aj + 4, oa);
+    return make_double2(oa, oa * (inv1 + inv2));
+}
+
 // The force times f0 where it is not 1 (a call: inlined, its FP64 products
 // are predicated into every pair).
 template <int DIM>
@@ -382,30 +455,36 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         }
         if (p < np) {
             const double4_32a a = ld4(b.pred, i), q = ld4(b.pred, j);
-            q1 = __double_as_longlong(DIM == 3 ? a.w : a.z);
-            q2 = __double_as_longlong(DIM == 3 ? q.w : q.z);
-            ex = __double_as_longlong(a.x) - __double_as_longlong(q.x);
-            ey = __double_as_longlong(a.y) - __double_as_longlong(q.y);
-            if (px) ex = image(ex, hx, Lx);
-            if (py) ey = image(ey, hy, Ly);
-            if (DIM == 3) {
-                ez = __double_as_longlong(a.z) - __double_as_longlong(q.z);
-                if (pz) ez = image(ez, hz, Lz);
+            if (is_far(a) || is_far(q)) {
+                const double2 t = pair_far<DIM, GAS, FLOW>(b.pred, b.invr, b.acc, b.ds, c, &k, i, j);
+                sAo += t.x;
+                sAor += t.y;
+            } else {
+                q1 = __double_as_longlong(DIM == 3 ? a.w : a.z);
+                q2 = __double_as_longlong(DIM == 3 ? q.w : q.z);
+                ex = __double_as_longlong(a.x) - __double_as_longlong(q.x);
+                ey = __double_as_longlong(a.y) - __double_as_longlong(q.y);
+                if (px) ex = image(ex, hx, Lx);
+                if (py) ey = image(ey, hy, Ly);
+                if (DIM == 3) {
+                    ez = __double_as_longlong(a.z) - __double_as_longlong(q.z);
+                    if (pz) ez = image(ez, hz, Lz);
+                }
+                // overlap test (r1 + r2)^2 >= d^2: in FP32 outside a 1e-5 guard
+                // band (the differences exact, ~2^-22 relative as FP32), else on
+                // the integers
+                const float fx = fix_len(ex), fy = fix_len(ey), fz = DIM == 3 ? fix_len(ez) : 0.f;
+                float m32 = fx * fx;
+                m32 = fmaf(fy, fy, m32);
+                if (DIM == 3) m32 = fmaf(fz, fz, m32);
+                const long long R = q1 + q2;
+                const float R32 = fix_len(R);
+                const float RR = R32 * R32;
+                if (m32 < RR * (1.f - 1e-5f))
+                    over = true;
+                else if (!(m32 > RR * (1.f + 1e-5f)))
+                    over = overlap_exact<DIM>(ex, ey, ez, llabs(R));
             }
-            // overlap test (r1 + r2)^2 >= d^2: in FP32 outside a 1e-5 guard
-            // band (the differences exact, ~2^-22 relative as FP32), else on
-            // the integers
-            const float fx = fix_len(ex), fy = fix_len(ey), fz = DIM == 3 ? fix_len(ez) : 0.f;
-            float m32 = fx * fx;
-            m32 = fmaf(fy, fy, m32);
-            if (DIM == 3) m32 = fmaf(fz, fz, m32);
-            const long long R = q1 + q2;
-            const float R32 = fix_len(R);
-            const float RR = R32 * R32;
-            if (m32 < RR * (1.f - 1e-5f))
-                over = true;
-            else if (!(m32 > RR * (1.f + 1e-5f)))
-                over = overlap_exact<DIM>(ex, ey, ez, llabs(R));
         }
         const unsigned mask = __ballot_sync(0xffffffffu, over);
         if (over) {
@@ -443,11 +522,51 @@ __device__ __forceinline__ unsigned long long fix_gap(long long a, long long b) 
 
 // The velocity of a bubble that touches a wall (touchesWall,
 // src/kernels.cu:553-566): d from the wall, which lies below or above it.
-static __device__ __noinline__ double wall_velocity(double f0, long long qr, unsigned long long d,
-                                                    bool below, int fixb) {
-    const double v = f0 * (1.0 - fx_to_double_any(d, -fixb) / fx_to_double_signed(qr, -fixb));
+static __device__ __noinline__ double wall_velocity(double f0, double r, double d, bool below) {
+    const double v = f0 * (1.0 - d / r);
     return below ? v : -v;
 }
+
+// A predicted position against the flow's box and the walls: as fixed point
+// (exact comparisons), and in FP64 for a bubble the fixed point does not hold.
+struct FixPlace {
+    long long q[3], r;
+    // addFlowVelocity, src/kernels.cu:497-544: between the faces or touching one
+    __device__ __forceinline__ bool in_flow(const DevConst &k, int a) const {
+        const unsigned long long rad = fx_abs(r);
+        return (q[a] < k.vhq[a] && q[a] > k.vlq[a]) || fix_gap(k.vlq[a], q[a]) <= rad ||
+               fix_gap(k.vhq[a], q[a]) <= rad;
+    }
+    // touches the nearer wall, the upper one of two
+    __device__ __forceinline__ bool touches(const DevConst &k, int a, double &velocity) const {
+        const unsigned long long dl = fix_gap(q[a], k.wlq[a]), dh = fix_gap(q[a], k.whq[a]);
+        const bool low = dl < dh;
+        const unsigned long long d = low ? dl : dh;
+        if (d > fx_abs(r)) return false;
+        velocity = wall_velocity(k.f0, fx_to_double_signed(r, -k.fix_b),
+                                 fx_to_double_any(d, -k.fix_b),
+                                 q[a] >= (low ? k.wlq[a] : k.whq[a]));
+        return true;
+    }
+    __device__ __forceinline__ double at(const DevConst &k, int a) const {
+        return fx_to_double_signed(q[a], -k.fix_b);
+    }
+};
+struct RealPlace {
+    double x[3], r;
+    __device__ __forceinline__ bool in_flow(const DevConst &k, int a) const {
+        const double lo = k.flow_lbb[a] - x[a], hi = k.flow_tfr[a] - x[a];
+        return (hi > 0.0 && lo < 0.0) || lo * lo <= r * r || hi * hi <= r * r;
+    }
+    __device__ __forceinline__ bool touches(const DevConst &k, int a, double &velocity) const {
+        const double lo = x[a] - k.lbb[a], hi = x[a] - k.tfr[a];
+        const double d = lo * lo < hi * hi ? lo : hi;
+        if (!(r * r >= d * d)) return false;
+        velocity = wall_velocity(k.f0, r, fabs(d), !(d < 0.0));
+        return true;
+    }
+    __device__ __forceinline__ double at(const DevConst &, int a) const { return x[a]; }
+};
 
 // 1 / (a number of neighbours), 0 for none (src/kernels.cu:500-502)
 constexpr int kInvCounts = 32;
@@ -468,20 +587,13 @@ static __device__ __noinline__ double inv_count(int n) { return n > 0 ? 1.0 / (d
 struct Vel3 {
     double x, y, z;
 };
-template <int DIM>
+template <int DIM, typename Place>
 static __device__ __noinline__ Vel3 boundary_velocity(const DevConst &k, int flow, int shear,
                                                       double drag, double vpx, double vpy,
-                                                      double vpz, long long qx, long long qy,
-                                                      long long qz, long long qr, double f0,
-                                                      double f1, double f2, int nn) {
-    const unsigned long long rad = fx_abs(qr);
-    const int fixb = k.fix_b;
+                                                      double vpz, Place at, double f0, double f1,
+                                                      double f2, int nn) {
     if (flow) {  // addFlowVelocity, src/kernels.cu:497-544
-        auto in_flow = [&](int a, long long q) {  // between the faces or touching one
-            return (q < k.vhq[a] && q > k.vlq[a]) || fix_gap(k.vlq[a], q) <= rad ||
-                   fix_gap(k.vhq[a], q) <= rad;
-        };
-        if (in_flow(0, qx) && in_flow(1, qy) && (DIM == 2 || in_flow(2, qz))) {
+        if (at.in_flow(k, 0) && at.in_flow(k, 1) && (DIM == 2 || at.in_flow(k, 2))) {
             vpx += k.flow_vel[0];
             vpy += k.flow_vel[1];
             if (DIM == 3) vpz += k.flow_vel[2];
@@ -492,39 +604,58 @@ static __device__ __noinline__ Vel3 boundary_velocity(const DevConst &k, int flo
             if (DIM == 3) vpz = fma(inv, f2, vpz);
         }
     }
-    if (shear) {  // linear shear along x over the last axis (cb_config.shear_speed)
-        const double q = fx_to_double_signed(DIM == 3 ? qz : qy, -fixb);
-        vpx += k.shear * ((q - k.lbb[DIM - 1]) * k.shear_il - 1.0);
-    }
+    if (shear)  // linear shear along x over the last axis (cb_config.shear_speed)
+        vpx += k.shear * ((at.at(k, DIM - 1) - k.lbb[DIM - 1]) * k.shear_il - 1.0);
     if (k.any_wall) {  // addWallVelocity, src/kernels.cu:546-593
         double xDrag = 1.0, yDrag = 1.0, velocity = 0.0;
-        auto touches = [&](int a, long long q) {  // the nearer wall, the upper one of two
-            const unsigned long long dl = fix_gap(q, k.wlq[a]), dh = fix_gap(q, k.whq[a]);
-            const bool low = dl < dh;
-            const unsigned long long d = low ? dl : dh;
-            if (d > rad) return false;
-            velocity = wall_velocity(k.f0, qr, d, q >= (low ? k.wlq[a] : k.whq[a]), fixb);
-            return true;
-        };
-        if (k.wall[0] && touches(0, qx)) {
+        if (k.wall[0] && at.touches(k, 0, velocity)) {
             vpx += velocity;
             vpy *= drag;
             vpz *= drag;
             xDrag = drag;
         }
-        if (k.wall[1] && touches(1, qy)) {
+        if (k.wall[1] && at.touches(k, 1, velocity)) {
             vpx *= drag;
             vpy += velocity * xDrag;
             vpz *= drag;
             yDrag = drag;
         }
-        if (k.wall[2] && touches(2, qz)) {
+        if (k.wall[2] && at.touches(k, 2, velocity)) {
             vpx *= drag;
             vpy *= drag;
             vpz += velocity * xDrag * yDrag;
         }
     }
     return {vpx, vpy, vpz};
+}
+
+// The step error of a bubble, its distance from where the last search saw it
+// and its path increment, in FP64: for one of whose positions the fixed point
+// does not hold.
+struct Moves {
+    double err, dist, inc;
+};
+static __device__ __forceinline__ double norm3(double x, double y, double z) {
+    const double s = fma(z, z, fma(y, y, x * x));
+    return s > 0.0 ? sqrt(s) : 0.0;
+}
+template <int DIM>
+static __device__ __noinline__ Moves far_moves(const double *pred, double *const *ds, const Ctrl *c,
+                                               int i, int fixb, double cx, double cy, double cz,
+                                               double cr) {
+    auto row = [&](int role) { return ds[c->drole[role]][i]; };
+    const State p = ld_state<DIM>(pred, ds, c, i, fixb);
+    Moves m;
+    long long e = 0;  // a NaN counts as the largest error
+    e = max_bits(e, abs_bits(p.x - cx));
+    e = max_bits(e, abs_bits(p.y - cy));
+    if (DIM == 3) e = max_bits(e, abs_bits(p.z - cz));
+    if (c->use_gas) e = max_bits(e, abs_bits(p.r - cr));
+    m.err = __longlong_as_double(e);
+    m.dist = norm3(cx - row(RS0), cy - row(RS1), DIM == 3 ? cz - row(RS2) : 0.0);
+    if (c->use_gas) m.dist += cr - row(RS3);
+    m.inc = norm3(row(RX) - cx, row(RY) - cy, DIM == 3 ? row(RZ) - cz : 0.0);
+    return m;
 }
 
 // FP64 issue and latency bound in its first forms (46 FP64 instructions a
@@ -605,9 +736,18 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         const long long qx = __double_as_longlong(p.x), qy = __double_as_longlong(p.y),
                         qz = DIM == 3 ? __double_as_longlong(p.z) : 0,
                         qr = __double_as_longlong(DIM == 3 ? p.w : p.z);
+        bool far = is_far(p);
         if (flow | shear | k.any_wall) {
-            const Vel3 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz, qx, qy, qz,
-                                                  qr, a1.y, a1.z, a1.w, flow ? NN[i] : 0);
+            const int nn = flow ? NN[i] : 0;
+            Vel3 v;
+            if (far) {
+                const State f = ld_state<DIM>(b.pred, b.ds, c, i, fixb);
+                v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz,
+                                           RealPlace{{f.x, f.y, f.z}, f.r}, a1.y, a1.z, a1.w, nn);
+            } else {
+                v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz,
+                                           FixPlace{{qx, qy, qz}, qr}, a1.y, a1.z, a1.w, nn);
+            }
             vpx = v.x;
             vpy = v.y;
             vpz = v.z;
@@ -615,22 +755,23 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         // AM2 correct x + 0.5 ts (v + vp), src/kernels.cu:487-495 and :366-387
         const double cx = fma(h, v0 + vpx, x0);
         const double cy = fma(h, v1 + vpy, y0);
-        const long long fx = fx_from_double(cx, fixb), fy = fx_from_double(cy, fixb);
+        const long long fx = fx_from_double(cx, fixb, far), fy = fx_from_double(cy, fixb, far);
         // the largest |predicted - corrected|, in units 2^-fixb
         uint64_t em = max(fx_abs(qx - fx), fx_abs(qy - fy));
         double cz = 0.0;
         long long fz = 0, sz = 0;
         if (DIM == 3) {
             cz = fma(h, v2 + vpz, z0);
-            fz = fx_from_double(cz, fixb);
+            fz = fx_from_double(cz, fixb, far);
             em = max(em, fx_abs(qz - fz));
-            sz = fz - fx_from_double(s2, fixb);
+            sz = fz - fx_from_double(s2, fixb, far);
         }
         // distance from the position of the last search; only its maximum
         // over the foam is used (the search trigger)
-        double dist = fx_norm<DIM>(fx - fx_from_double(s0, fixb), fy - fx_from_double(s1, fixb),
-                                   sz, fixb);
+        double dist = fx_norm<DIM>(fx - fx_from_double(s0, fixb, far),
+                                   fy - fx_from_double(s1, fixb, far), sz, fixb);
         int del = 0;
+        double cr = 0.0;
         if (gas) {  // mean-field gas exchange and radius, src/kernels.cu:390-431
             double inv, area;
             if (DIM == 3) {
@@ -638,15 +779,15 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 area = times4(ri.y);
             } else {
                 inv = p.w;
-                area = kPi * fx_to_double_signed(qr, -fixb);
+                area = kPi * (is_far(p) ? CB_D(RRN)[i] : fx_to_double_signed(qr, -fixb));
             }
             double vr = mfa - inv;
             vr *= mfb * (area - ov);
             vr += vpr;
             vr *= DIM == 3 ? kq * (inv * inv) : kq * inv;
             vpr = vr;
-            const double cr = fma(h, v3 + vr, r0);
-            em = max(em, fx_abs(qr - fx_from_double(cr, fixb)));
+            cr = fma(h, v3 + vr, r0);
+            em = max(em, fx_abs(qr - fx_from_double(cr, fixb, far)));
             dist += cr - s3;
             if (__double_as_longlong(cr) > __double_as_longlong(k.min_rad)) {  // cr > minRad
                 vol = fma(DIM == 3 ? cr * cr : cr, cr, vol);
@@ -655,17 +796,25 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 ndel++;
             }
             mrad = max_bits(mrad, cr);
-            CB_D(RRN)[i] = cr;
             CB_D(RVP3)[i] = vpr;
             bad |= !finite_bits(cr);
         }
         if (del | marks) b.delflag[i] = del;
-        mexp = max_bits(mexp, dist);
+        double inc = 0.0;
         if (path)  // src/kernels.cu:437-451; the increment to ~2^-46
-            CB_D(RPATHN)[i] = path0 + fx_norm<DIM>(fx_from_double(x0, fixb) - fx,
-                                            fx_from_double(y0, fixb) - fy,
-                                            DIM == 3 ? fx_from_double(z0, fixb) - fz : 0, fixb);
-        const long long e = __double_as_longlong(fx_to_double_any(em, -fixb));
+            inc = fx_norm<DIM>(fx_from_double(x0, fixb, far) - fx,
+                               fx_from_double(y0, fixb, far) - fy,
+                               DIM == 3 ? fx_from_double(z0, fixb, far) - fz : 0, fixb);
+        long long e = __double_as_longlong(fx_to_double_any(em, -fixb));
+        if (far) {
+            const Moves m = far_moves<DIM>(b.pred, b.ds, c, i, fixb, cx, cy, cz, cr);
+            e = __double_as_longlong(m.err);
+            dist = m.dist;
+            inc = m.inc;
+        }
+        mexp = max_bits(mexp, dist);
+        if (path) CB_D(RPATHN)[i] = path0 + inc;
+        if (gas) CB_D(RRN)[i] = cr;
         CB_D(RERR)[i] = __longlong_as_double(max(e, __double_as_longlong(err0)));  // both >= 0
         merr = max(merr, e);
         CB_D(RXN)[i] = cx;
@@ -781,15 +930,15 @@ __global__ void __launch_bounds__(kBlock) k_boot(Bufs b, int phase) {
             const double r = R[i];
             const double inv = 1.0 / r, rsq = r * r;
             if (DIM == 3) reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
-            st_state<DIM>(b, i, X[i], Y[i], DIM == 3 ? Z[i] : 0.0, r, inv, fixb);
+            st_state<DIM>(b, c, i, X[i], Y[i], DIM == 3 ? Z[i] : 0.0, r, inv, fixb);
             O0[i] = O1[i] = O2[i] = O3[i] = 0.0;
             PATH[i] = 0.0;
         } else {
             double4_32a a = reinterpret_cast<double4_32a *>(acc)[0];
             if (phase == 1) {
-                const State p = ld_state<DIM>(b, i, fixb);
-                st_state<DIM>(b, i, p.x + a.x * ts, p.y + a.y * ts, p.z + a.z * ts, p.r,
-                                  p.inv, fixb);
+                const State p = ld_state<DIM>(b.pred, b.ds, c, i, fixb);
+                st_state<DIM>(b, c, i, p.x + a.x * ts, p.y + a.y * ts, p.z + a.z * ts, p.r,
+                              b.pred[4 * (size_t)i + 3], fixb);
             } else {
                 O0[i] = a.x;
                 O1[i] = a.y;

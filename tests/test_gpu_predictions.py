@@ -5,7 +5,7 @@ import pytest
 
 import cubble_gb300 as cb
 from cubble_gb300 import workloads
-from helpers import assert_rows_close
+from helpers import assert_rows_close, by_index
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +54,92 @@ def test_a_predicted_radius_below_zero(oracle_mod, dim, precision):
     for k in ("total_area", "total_area_per_radius", "total_volume_new", "max_error"):
         assert a[k] == pytest.approx(b[k], rel=1e-13), k
     assert np.array_equal(a["delete_flags"], b["delete_flags"])
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("row", ["dxdto", "dydt", "drdto"])
+def test_a_nan_that_enters_through_the_prediction(row, dim, precision):
+    """A NaN in a previous rate reaches the prediction alone: non-finite, and
+    not a step error that rejects until the cap."""
+    cfg, st = lattice(dim, 18.0)
+    st[row] = np.zeros(len(st["r"]))
+    st[row][5] = np.nan
+    for single in (False, True):
+        g = cb.GpuFoam(workloads.sweep_config_as(cfg, precision=precision))
+        g.load_state(st)
+        g.search_neighbors()
+        with pytest.raises(cb.CubbleError) as e:
+            g.attempt() if single else g.integrate(1)
+        assert e.value.code == 5, e.value
+
+
+ROWS = ["xp", "yp", "rp", "dxdtp", "dydtp", "drdtp", "overlap"]
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("at", [3.0, -40.0, 1e9])
+def test_bubbles_far_beyond_a_wall(oracle_mod, at, dim, precision):
+    """Three bubbles lie many boxes beyond a wall, two of them overlapping, one
+    moving: its step error rejects the first attempts, the pair moves apart,
+    and the move since the search is seen."""
+    cfg, st = lattice(dim, 18.0, wall=(1, 0, 0), wall_drag=0.1)
+    n = len(st["r"])
+    st["x"][:3] = at * 18.0 + np.array([0.0, 1.5, 60.0])
+    for k in "yz"[:dim - 1]:
+        st[k][:3] = 5.0
+    st["dxdt"] = np.zeros(n)
+    st["dxdt"][2] = 0.9  # error ~ h v: 4.5e-5 at the first dt
+    g, o = both(oracle_mod, cfg, st, precision)
+    assert np.array_equal(g.get_state()["index"], o.get_state()["index"])
+    g.set_pairs(*o.pairs())  # the search's FP32 filter is for the box's surroundings
+    a, b = g.attempt(), o.attempt()
+    tol = max(1e-12, 8 * 2.0 ** -53 * abs(at) * 18.0)  # of rows of about 1
+    rows = ROWS + (["zp", "dzdtp"] if dim == 3 else [])
+    assert_rows_close(a, b, rows, tol, "far ")
+    assert b["max_error"] > 1e-5
+    place = 4 * np.spacing(abs(at) * 18.0 + 60.0)
+    for k in ("error", "path_new"):
+        assert np.max(np.abs(a[k] - b[k])) <= max(place, 1e-15), k
+    for k in ("max_error", "max_expansion"):
+        assert a[k] == pytest.approx(b[k], rel=1e-11, abs=place), k
+    if abs(at) > 1e6:
+        return  # the coordinates no longer resolve the tolerance
+    rg, ro = g.integrate(4), o.integrate(4)
+    for k in ("steps", "attempts", "searches", "count", "num_pairs"):
+        assert rg[k] == ro[k], k
+    sg, so = by_index(g.get_state()), by_index(o.get_state())
+    assert_rows_close(sg, so, ["x", "y", "r", "dxdt", "path"], 1e-10, "far ")
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("dim,options", [
+    (2, {}), (3, {}), (2, dict(wall=(1, 1, 0), wall_drag=0.2)),
+    (3, dict(use_flow=1, flow_lbb=(0.0,) * 3, flow_tfr=(8.0,) * 3, flow_vel=(0.02, 0.01, 0.03))),
+    (3, dict(use_flow=1, shear_speed=0.05, wall=(0, 0, 1), wall_drag=0.1))])
+@pytest.mark.parametrize("dt", [40.0, 200.0, 2e4])
+def test_a_step_far_too_large(oracle_mod, dt, dim, options, precision):
+    """dt so large that some or all predictions leave the box, by up to many
+    times its size: the attempt is that of the oracle, and rejected. Its
+    positions reach ~10^4, so the forces carry ~10^-12 / d: 1e-9 of each row."""
+    cfg, st = workloads.foam(1500, dim, 0.9 if dim == 2 else 0.8, seed=88, **options)
+    g = cb.GpuFoam(workloads.sweep_config_as(cfg, precision=precision))
+    o = oracle_mod.OracleFoam(cfg)
+    for f in (g, o):
+        f.load_state(st)
+        workloads.prepare(f)
+        f.integrate(3)
+    s = o.get_state()  # the same rows for both
+    g.load_state(s)
+    o.load_state(s)
+    for f in (g, o):
+        f.search_neighbors()
+        f.set_time(dt)
+    a, b = g.attempt(), o.attempt()
+    assert b["max_error"] > cfg.tfr[0] / 2
+    rows = ROWS + (["zp", "dzdtp"] if dim == 3 else [])
+    assert_rows_close(a, b, rows + ["error", "path_new"], 1e-9, "large step ")
+    for k in ("max_error", "max_expansion", "total_overlap_area", "total_area"):
+        assert a[k] == pytest.approx(b[k], rel=1e-9), k
+    assert g.report()["time_step"] == o.report()["time_step"] == dt * 0.37
