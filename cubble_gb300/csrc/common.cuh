@@ -76,8 +76,9 @@ struct DevConst {
     // step_mixed.cu); lq / hq are the periodic box length and half of it in
     // those units.
     long long lq[3], hq[3];
-    // FP64 form: predicted positions and radii in units 2^-fix_b (fixpair.cuh)
-    // and the periodic box length and half of it in those units
+    // FP64 form: predicted positions in units 2^-fix_b (fixpair.cuh; radii in
+    // units 2^Ctrl::rad_k finer) and the periodic box length and half of it in
+    // those units
     long long flq[3], fhq[3];
     // the same of the walls (box corners) and of the imposed flow's box
     long long wlq[3], whq[3], vlq[3], vhq[3];
@@ -146,6 +147,8 @@ struct Ctrl {
     int stash_over;    // a row of the last search exceeded kStash partners
     int sparse_cells;  // < 24 bubbles per cell: thread-per-bubble pair pass
     float search_maxr;  // the search's largest radius, rounded up to FP32
+    int rad_k;          // FP64 form: bits of the radii's unit beyond the positions'
+                        // (radius_shift at the last search; 0 before one)
     // Mixed form: the correct kernel also writes the next attempt's
     // prediction for both dt it can have after an accept (unchanged, x1.269)
     // with their area sums; pred_ready says the prediction for the coming
@@ -167,7 +170,7 @@ struct Ctrl {
 };
 
 // What a resident run's blocks (below) reduce into and wait on, in global
-// memory: zero between launches.
+// memory: zero between launches (`far` serves the launch per phase too).
 struct RunAcc {
     double psum[4];      // overlap area, overlap area over radius; area, area over radius
     double csum[5];      // correct: volume; mixed form: the candidates' sums
@@ -178,7 +181,8 @@ struct RunAcc {
 struct RunSync {
     RunAcc acc[2];  // of even and odd attempts
     long long search_max;  // k_search_run: largest radius (bits), a row beyond its stash
-    int stash_over, pad0_;
+    int stash_over;
+    int far;  // FP64 form: a prediction of this attempt has a marked record (step.cu)
     unsigned arrive, pad_[31], exits, pad2_[31];
 };
 
@@ -949,7 +953,7 @@ __device__ __forceinline__ bool run_more(const RunShared *s, int attempts) {
 // Attempt `attempt` uses the accumulators of its parity. The other ones are
 // free once every block has passed the first barrier of this attempt (each
 // has then read the last attempt's results): cleared by block 0 between its
-// last two barriers.
+// last two barriers, and with them the mark of this attempt's predictions.
 __device__ __forceinline__ void run_begin(RunCtx *rx, int attempt) {
     rx->acc = &rx->g->acc[attempt & 1];
 }
@@ -957,6 +961,7 @@ __device__ __forceinline__ void run_clear_other(RunCtx *rx, int vb) {
     if (vb != 0) return;
     int *o = reinterpret_cast<int *>(rx->acc == &rx->g->acc[0] ? &rx->g->acc[1] : &rx->g->acc[0]);
     if (threadIdx.x < sizeof(RunAcc) / 4) o[threadIdx.x] = 0;
+    if (threadIdx.x == 0) rx->g->far = 0;
 }
 
 // Block 0 writes the control block to `ctrl` and, if given, to the host's

@@ -835,6 +835,7 @@ int cb_load_state(cb_context *c, const cb_state_view *s) {
     h.np = 0;
     h.ndel = 0;
     h.marks = 0;
+    h.rad_k = 0;
     h.status = CB_OK;
     h.max_bubble_radius = 0.0;
     h.too_large = h.need_search = h.need_delete = h.attempts_this_step = 0;

@@ -3,10 +3,12 @@
 // GB300 issues FP64 at 1/64 of its FP32 rate; one FP64 instruction costs the
 // issue slots of about 64 others, a 64-bit integer product about ten. The
 // predicted positions and radii of the FP64 form are therefore kept as
-// integers q = x 2^B (|x| < P, P the power of two that bounds the box corners
-// with an eighth to spare, B = 62 - log2 P: never coarser than the doubles they
-// come from except below 2^-9 P, where the unit stays 2^-53 of P / 2^9; a
-// bubble beyond P is taken in FP64). Differences are
+// integers: positions q = x 2^B (|x| < P, P the power of two that bounds the
+// box corners with an eighth to spare, B = 62 - log2 P: never coarser than the
+// doubles they come from except below 2^-9 P, where the unit stays 2^-53 of
+// P / 2^9), radii in a unit 2^K finer, which the largest radius sets the same
+// way (radius_shift: exact down to 2^-8 of it). A bubble beyond either range is
+// taken in FP64. Differences are
 // then exact, the minimum image an integer compare, and the distance, the
 // reciprocals and the products of a pair run in integers normalised to the
 // pair's own scale R = r1 + r2:
@@ -190,19 +192,19 @@ struct FxTerms {
     double fx, fy, fz, oa;
     bool inside;
 };
-// From the exact differences e (minimum image) and the predicted radii q1,
-// q2, all in units 2^-B. false where the fixed-point range does not hold the
-// pair: centres closer than R/16 ... R/8 (a deeply swallowed bubble), a
-// negative predicted radius, or R below 2^32 units.
+// From the exact differences e (minimum image) in units 2^-B and the predicted
+// radii q1, q2 in units 2^-(B + K). false where the fixed-point range does not
+// hold the pair: centres closer than R/16 ... R/8 (a deeply swallowed bubble),
+// a negative predicted radius, or R below 2^(32 + K) units.
 template <int DIM, bool GAS>
 CB_HD bool fx_pair(int64_t ex, int64_t ey, int64_t ez, int64_t q1, int64_t q2, int B,
-                   FxTerms &out) {
+                   FxTerms &out, int K = 0) {
     const int64_t R0 = q1 + q2;
-    const int s = ff_clz((uint32_t)((uint64_t)R0 >> 32)) - 1;
-    if (s > 30 || (q1 | q2) < 0) return false;
+    const int s = ff_clz((uint32_t)((uint64_t)R0 >> 32)) - 1, u = s + K;
+    if (u > 30 || (q1 | q2) < 0) return false;
     const int64_t R = (int64_t)fx_shl((uint64_t)R0, s);
-    const int64_t vx = (int64_t)fx_shl((uint64_t)ex, s), vy = (int64_t)fx_shl((uint64_t)ey, s),
-                  vz = DIM == 3 ? (int64_t)fx_shl((uint64_t)ez, s) : 0;
+    const int64_t vx = (int64_t)fx_shl((uint64_t)ex, u), vy = (int64_t)fx_shl((uint64_t)ey, u),
+                  vz = DIM == 3 ? (int64_t)fx_shl((uint64_t)ez, u) : 0;
     const FxHalves x = fx_split(vx), y = fx_split(vy), z = fx_split(vz);
     int64_t A = (int64_t)x.h * x.h + (int64_t)y.h * y.h;
     int64_t C = (int64_t)x.h * x.l + (int64_t)y.h * y.l;
@@ -224,7 +226,7 @@ CB_HD bool fx_pair(int64_t ex, int64_t ey, int64_t ez, int64_t q1, int64_t q2, i
     if (GAS) {
         const int64_t D = (int64_t)fx_shl((uint64_t)(q1 < q2 ? q2 - q1 : q1 - q2), s);
         const int64_t big = (R >> 1) + (D >> 1);  // max(r1, r2)
-        const int sc = 62 - s - B;                // R = R' 2^sc
+        const int sc = 62 - u - B;                // R = R' 2^sc
         out.inside = M < fx_square(big);
         uint64_t w;  // units 2^-62
         if (out.inside) {

@@ -111,6 +111,14 @@ static __device__ __noinline__ void wrap_one(double *xp, int *wp, double x, doub
     *wp -= mult;
 }
 
+// How much finer than the positions' unit 2^-fix_b that of the radii can be: the
+// largest radius may double before the next search (beyond that a bubble is
+// evaluated in FP64, step.cu), and a pair keeps room for its own scale.
+__device__ __forceinline__ int radius_shift(const DevConst &k, double max_r) {
+    const int e = ((__double2hiint(max_r) >> 20) & 0x7ff) - 1023;  // max_r < 2^(e + 1)
+    return min(max(62 - (e + 2) - k.fix_b, 0), 20);
+}
+
 // The cell grid and the search's other decisions from the largest radius.
 __device__ __forceinline__ void search_begin(Ctrl *c, const DevConst &k, double max_r) {
     int cd[3];
@@ -123,6 +131,7 @@ __device__ __forceinline__ void search_begin(Ctrl *c, const DevConst &k, double 
     c->stash_over = 0;
     c->sparse_cells = (long long)c->n < 24LL * c->ncell;
     c->search_maxr = __double2float_ru(max_r);
+    c->rad_k = radius_shift(k, max_r);
     c->pred_ready = 0;  // the bubbles move to new slots
     c->pred_slot = 0;
 }

@@ -23,12 +23,15 @@ __device__ __forceinline__ double4_32a ld4(const double *p, int i) {
     return reinterpret_cast<const double4_32a *>(p)[i];
 }
 
-// The packed predicted state of bubble i (positions and radius as fixed point,
-// fixpair.cuh; 2D: 1/r beside them): written and read back. A bubble that the
-// fixed point does not hold (it lies beyond the range after a large dt or as it
-// was loaded, or is NaN) has a marked record, and its state in the rows of the
-// corrected state, which are free until the correct kernel writes them: its
-// terms are then evaluated in FP64 (pair_far, far_moves and RealPlace below).
+// The packed predicted state of bubble i (positions in units 2^-fixb and the
+// radius in units 2^-radb, fixpair.cuh; 2D: 1/r beside them): written and read
+// back. A bubble that the fixed point does not hold (it lies beyond the range
+// after a large dt or as it was loaded, its radius is negative or has outgrown
+// what the last search saw, or one of them is NaN) has a marked record, and its
+// state in spare rows that only a search uses: its terms are then evaluated in
+// FP64 (far_pairs, far_moves and RealPlace below).
+// The mark lies 2^62 units or more from every other bubble, and its radius is the
+// only one below zero: the loop over the pairs needs no test for it.
 constexpr long long kFarRecord = (long long)0x8000000000000000ULL;
 __device__ __forceinline__ bool is_far(double4_32a p) {  // |q| < 2^62 in the others
     return __double2hiint(p.x) == (int)0x80000000;
@@ -39,36 +42,41 @@ struct State {
 template <int DIM>
 static __device__ __noinline__ void st_far(double *const *ds, const Ctrl *c, int i, double x,
                                            double y, double z, double r) {
-    ds[c->drole[RXN]][i] = x;
-    ds[c->drole[RYN]][i] = y;
-    if (DIM == 3) ds[c->drole[RZN]][i] = z;
-    ds[c->drole[RRN]][i] = r;
+    ds[c->drole[RVQ0]][i] = x;
+    ds[c->drole[RVQ1]][i] = y;
+    if (DIM == 3) ds[c->drole[RVQ2]][i] = z;
+    ds[c->drole[RVQ3]][i] = r;
 }
 template <int DIM>
 __device__ __forceinline__ void st_state(const Bufs &b, const Ctrl *c, int i, double x, double y,
-                                         double z, double r, double inv, int fixb) {
+                                         double z, double r, double inv, int fixb, int radb) {
     double4_32a p;
-    bool far = false;
-    const double qr = __longlong_as_double(fx_from_double(r, fixb, far));
+    bool far = __double2hiint(r) < 0;
+    double qr = __longlong_as_double(fx_from_double(r, radb, far));
     p.x = __longlong_as_double(fx_from_double(x, fixb, far));
     p.y = __longlong_as_double(fx_from_double(y, fixb, far));
-    p.z = DIM == 3 ? __longlong_as_double(fx_from_double(z, fixb, far)) : qr;
-    p.w = DIM == 3 ? qr : inv;
+    p.z = DIM == 3 ? __longlong_as_double(fx_from_double(z, fixb, far)) : 0.0;
     if (far) {
         p.x = __longlong_as_double(kFarRecord);
+        p.y = p.z = 0.0;
+        qr = __longlong_as_double(-1LL);
+        b.run->far = 1;
         st_far<DIM>(b.ds, c, i, x, y, z, r);
     }
+    (DIM == 3 ? p.w : p.z) = qr;
+    if (DIM == 2) p.w = inv;
     reinterpret_cast<double4_32a *>(b.pred)[i] = p;
 }
 template <int DIM>
 __device__ __forceinline__ State ld_state(const double *pred, double *const *ds, const Ctrl *c,
-                                          int i, int fixb) {
+                                          int i, int fixb, int radb) {
     const double4_32a p = ld4(pred, i);
     if (is_far(p))
-        return {ds[c->drole[RXN]][i], ds[c->drole[RYN]][i],
-                DIM == 3 ? ds[c->drole[RZN]][i] : 0.0, ds[c->drole[RRN]][i]};
-    auto back = [&](double q) { return fx_to_double_signed(__double_as_longlong(q), -fixb); };
-    return {back(p.x), back(p.y), DIM == 3 ? back(p.z) : 0.0, back(DIM == 3 ? p.w : p.z)};
+        return {ds[c->drole[RVQ0]][i], ds[c->drole[RVQ1]][i],
+                DIM == 3 ? ds[c->drole[RVQ2]][i] : 0.0, ds[c->drole[RVQ3]][i]};
+    auto back = [](double q, int b) { return fx_to_double_signed(__double_as_longlong(q), -b); };
+    return {back(p.x, fixb), back(p.y, fixb), DIM == 3 ? back(p.z, fixb) : 0.0,
+            back(DIM == 3 ? p.w : p.z, radb)};
 }
 
 // ---------------------------------------------------------------- predict
@@ -87,7 +95,7 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
                  *V3 = drow(b, c, RV3);
     const double *O0 = drow(b, c, RVO0), *O1 = drow(b, c, RVO1), *O2 = drow(b, c, RVO2),
                  *O3 = drow(b, c, RVO3);
-    const int fixb = b.k->fix_b;
+    const int fixb = b.k->fix_b, radb = fixb + c->rad_k;
     double sA = 0.0, sAr = 0.0;
     int na = 0;
     for (int i = first_item<RES>(vb, vg); i < n; i += vg * blockDim.x) {
@@ -100,7 +108,7 @@ __device__ __forceinline__ void k_predict_body(const Bufs &b, const int vb, cons
         const double rsq = rp * rp;
         const double zp = DIM == 3 ? fma(h, fma(3.0, V2[i], -O2[i]), Z[i]) : 0.0;
         if (DIM == 3) reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
-        st_state<DIM>(b, c, i, xp, yp, zp, rp, inv, fixb);
+        st_state<DIM>(b, c, i, xp, yp, zp, rp, inv, fixb, radb);
         if (gas) {  // area and area per radius, src/kernels.cu:103-112, with
                     // the constant factor (4 pi, 2 pi) applied to the block sums
             if (DIM == 3) {
@@ -226,29 +234,37 @@ __device__ __forceinline__ void pairs_fold(const Bufs &b, const int vb, const in
 }
 
 // The overlap test for pairs in the FP32 guard band: (r1 + r2)^2 >= d^2 from
-// the exact integers (R >= 0, a unit of 2^-60 R^2).
+// the exact integers (R >= 0 in units 2^-K of the differences'; a unit of
+// 2^-60 R^2).
 template <int DIM>
 static __device__ __noinline__ bool overlap_exact(long long ex, long long ey, long long ez,
-                                                  long long R) {
-    if (llabs(ex) > R || llabs(ey) > R || (DIM == 3 && llabs(ez) > R)) return false;
-    const int s = fx_clz((unsigned long long)R | 1ull) - 1;
-    long long m = fx_square(ex << s) + fx_square(ey << s);
-    if (DIM == 3) m += fx_square(ez << s);
+                                                  long long R, int K) {
+    const long long cut = R >> K;
+    if (llabs(ex) > cut || llabs(ey) > cut || (DIM == 3 && llabs(ez) > cut)) return false;
+    const int s = fx_clz((unsigned long long)R | 1ull) - 1, u = min(s + K, 63);  // |e| 2^u <= R 2^s
+    long long m = fx_square(ex << u) + fx_square(ey << u);
+    if (DIM == 3) m += fx_square(ez << u);
     return fx_square(R << s) >= m;
 }
 
-// The terms of a pair fx_pair does not take, in FP64: centres much closer
-// than the radii, a negative predicted radius. The force goes to rs[0],
-// rs[kT], ...; returns the overlap as FxTerms::oa.
+// The terms of a pair fx_pair does not take, in FP64: centres much closer than
+// the radii. The force goes to rs[0], rs[kT], ...; returns the overlap as
+// FxTerms::oa. Nothing for a marked bubble, whose pairs far_pairs takes.
 // Row length of the transposed results (32 pairs): the 8-byte loads of four
 // pairs' components fall on distinct banks, but for the fifth row.
 constexpr int kT = 36;
 template <int DIM>
 static __device__ __noinline__ double pair_slow(long long ex, long long ey, long long ez,
-                                                long long q1, long long q2, double unit,
-                                                double f0, double *rs) {
+                                                long long q1, long long q2, int K,
+                                                const DevConst &k, double *rs) {
+    if ((q1 | q2) < 0) {
+#pragma unroll
+        for (int t = 0; t < DIM; t++) rs[t * kT] = 0.0;
+        return 0.0;
+    }
+    const double unit = k.fix_unit, runit = ldexp(unit, -K), f0 = k.f0;
     const double dx = (double)ex * unit, dy = (double)ey * unit, dz = (double)ez * unit;
-    const double r1 = (double)q1 * unit, r2 = (double)q2 * unit;
+    const double r1 = (double)q1 * runit, r2 = (double)q2 * runit;
     double m = dx * dx;
     m = fma(dy, dy, m);
     if (DIM == 3) m = fma(dz, dz, m);
@@ -270,7 +286,9 @@ static __device__ __noinline__ double2 pair_far(const double *pred, const double
                                                 double *const *ds, const Ctrl *c,
                                                 const DevConst *kp, int i, int j) {
     const DevConst &k = *kp;
-    const State a = ld_state<DIM>(pred, ds, c, i, k.fix_b), q = ld_state<DIM>(pred, ds, c, j, k.fix_b);
+    const int fixb = k.fix_b, radb = fixb + c->rad_k;
+    const State a = ld_state<DIM>(pred, ds, c, i, fixb, radb),
+                q = ld_state<DIM>(pred, ds, c, j, fixb, radb);
     double dx = a.x - q.x, dy = a.y - q.y, dz = DIM == 3 ? a.z - q.z : 0.0;
     if (!k.wall[0]) dx = min_image(dx, k.half_iv[0], k.iv[0]);
     if (!k.wall[1]) dy = min_image(dy, k.half_iv[1], k.iv[1]);
@@ -311,12 +329,39 @@ static __device__ __noinline__ double2 pair_far(const double *pred, const double
     return make_double2(oa, oa * (inv1 + inv2));
 }
 
+// This thread's pairs of that kind, where any bubble is (RunSync::far), in a
+// pass of their own and with this thread's share of the sums: the call in the
+// loop over all pairs cost an attempt 2 to 3 %.
+template <int DIM, bool GAS, bool FLOW, bool RES>
+static __device__ __noinline__ double2 far_pairs(const double *pred, const double *invr, double *acc,
+                                                 double *const *ds, int *const *ps, const Ctrl *c,
+                                                 const DevConst *k, int vb, int vg) {
+    double2 sum = make_double2(0.0, 0.0);
+    const int np = c->np;
+    const int *PI = ps[c->prole[PI0]], *PJ = ps[c->prole[PJ0]];
+    for (int p = first_item<RES>(vb, vg); p < np; p += vg * blockDim.x) {
+        const int i = PI[p], j = PJ[p];
+        if (!is_far(ld4(pred, i)) && !is_far(ld4(pred, j))) continue;
+        const double2 t = pair_far<DIM, GAS, FLOW>(pred, invr, acc, ds, c, k, i, j);
+        sum.x += t.x;
+        sum.y += t.y;
+    }
+    return sum;
+}
+
 // The force times f0 where it is not 1 (a call: inlined, its FP64 products
 // are predicated into every pair).
 template <int DIM>
 static __device__ __noinline__ void scale_force(double f0, double *rs) {
 #pragma unroll
     for (int a = 0; a < DIM; a++) rs[a * kT] *= f0;
+}
+
+// The difference of two fixed-point positions (modulo 2^64: one of them may be
+// the mark of a bubble beyond the range).
+__device__ __forceinline__ long long fix_diff(double a, double b) {
+    return (long long)((unsigned long long)__double_as_longlong(a) -
+                       (unsigned long long)__double_as_longlong(b));
 }
 
 // A fixed-point length as FP32, in units of 2^32: the signed high word and the
@@ -339,13 +384,16 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     __shared__ double res[kW][kC * kT];
     const Ctrl *c = b.ctrl;
     const DevConst &k = *b.k;
+    const int any_far = __ldcg(&b.run->far);
+    double sAo = 0.0, sAor = 0.0;
     const int np = c->np;
     const int *PI = b.ps[c->prole[PI0]];
     const int *PJ = b.ps[c->prole[PJ0]];
     const double *V0 = drow(b, c, RV0), *V1 = drow(b, c, RV1), *V2 = drow(b, c, RV2);
     const double f0 = k.f0;
     const bool scaled = __double_as_longlong(f0) != 0x3ff0000000000000LL;
-    const int fixb = k.fix_b;
+    const int fixb = k.fix_b, radk = c->rad_k;
+    const float rscale = __int_as_float((127 - radk) << 23);  // radii in the positions' unit
     const bool px = !k.wall[0], py = !k.wall[1], pz = DIM == 3 && !k.wall[2];
     const long long hx = k.fhq[0], hy = k.fhq[1], hz = k.fhq[2];
     const long long Lx = k.flq[0], Ly = k.flq[1], Lz = k.flq[2];
@@ -354,11 +402,10 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     long long(*Q)[kQueue] = qd[w];
     int2 *QP = qij[w];
     double *RS = res[w];
-    double sAo = 0.0, sAor = 0.0;
 
     // minimum image (wrappedDifference, src/kernels.cu:1094-1114), exact
     auto image = [](long long d, long long half, long long len) {
-        if ((unsigned long long)(d + half) > 2ull * half) d -= d > 0 ? len : -len;
+        if ((unsigned long long)d + half > 2ull * half) d -= d > 0 ? len : -len;
         return d;
     };
 
@@ -375,14 +422,17 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         const long long q1 = Q[kR1][slot], q2 = Q[kR1 + 1][slot];
         double oa;
         FxTerms t;
-        if (fx_pair<DIM, GAS>(ex, ey, ez, q1, q2, fixb, t)) {
+        bool on = true;
+        if (fx_pair<DIM, GAS>(ex, ey, ez, q1, q2, fixb, t, radk)) {
             RS[0 * kT + e] = t.fx;
             RS[1 * kT + e] = t.fy;
             if (DIM == 3) RS[2 * kT + e] = t.fz;
             oa = t.oa;
             if (scaled) scale_force<DIM>(f0, RS + e);
         } else {
-            oa = pair_slow<DIM>(ex, ey, ez, q1, q2, k.fix_unit, f0, RS + e);
+            oa = pair_slow<DIM>(ex, ey, ez, q1, q2, radk, k, RS + e);
+            on = (q1 | q2) >= 0;
+            if (GAS && !on) inv1 = inv2 = 0.0;
         }
         if (GAS) {  // pairwise gas exchange, src/kernels.cu:236-280; oa in units of ov_unit
             if (DIM == 2) oa = __double_as_longlong(oa) > 0 ? oa * rsqrt_d(oa) : 0.0;
@@ -391,7 +441,7 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
             sAo += oa;
             sAor = fma(oa, inv1 + inv2, sAor);
         }
-        if (FLOW) {  // src/kernels.cu:298-307 (overlapping pairs only)
+        if (FLOW && on) {  // src/kernels.cu:298-307 (overlapping pairs only)
             double *ai = b.acc + (size_t)i * kAcc;
             red_add(ai + 5, V0[j]);
             red_add(ai + 6, V1[j]);
@@ -428,6 +478,12 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         i1 = PI[p];
         j1 = PJ[p];
     }
+    if (any_far) {  // ahead of the loop: its registers are free
+        const double2 t = far_pairs<DIM, GAS, FLOW, RES>(b.pred, b.invr, b.acc, b.ds, b.ps, c, &k,
+                                                         vb, vg);
+        sAo = t.x;
+        sAor = t.y;
+    }
     for (; (p >> 5) < nch; p += step) {
         bool over = false;
         const int i = i1, j = j1;
@@ -455,36 +511,30 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         }
         if (p < np) {
             const double4_32a a = ld4(b.pred, i), q = ld4(b.pred, j);
-            if (is_far(a) || is_far(q)) {
-                const double2 t = pair_far<DIM, GAS, FLOW>(b.pred, b.invr, b.acc, b.ds, c, &k, i, j);
-                sAo += t.x;
-                sAor += t.y;
-            } else {
-                q1 = __double_as_longlong(DIM == 3 ? a.w : a.z);
-                q2 = __double_as_longlong(DIM == 3 ? q.w : q.z);
-                ex = __double_as_longlong(a.x) - __double_as_longlong(q.x);
-                ey = __double_as_longlong(a.y) - __double_as_longlong(q.y);
-                if (px) ex = image(ex, hx, Lx);
-                if (py) ey = image(ey, hy, Ly);
-                if (DIM == 3) {
-                    ez = __double_as_longlong(a.z) - __double_as_longlong(q.z);
-                    if (pz) ez = image(ez, hz, Lz);
-                }
-                // overlap test (r1 + r2)^2 >= d^2: in FP32 outside a 1e-5 guard
-                // band (the differences exact, ~2^-22 relative as FP32), else on
-                // the integers
-                const float fx = fix_len(ex), fy = fix_len(ey), fz = DIM == 3 ? fix_len(ez) : 0.f;
-                float m32 = fx * fx;
-                m32 = fmaf(fy, fy, m32);
-                if (DIM == 3) m32 = fmaf(fz, fz, m32);
-                const long long R = q1 + q2;
-                const float R32 = fix_len(R);
-                const float RR = R32 * R32;
-                if (m32 < RR * (1.f - 1e-5f))
-                    over = true;
-                else if (!(m32 > RR * (1.f + 1e-5f)))
-                    over = overlap_exact<DIM>(ex, ey, ez, llabs(R));
+            q1 = __double_as_longlong(DIM == 3 ? a.w : a.z);
+            q2 = __double_as_longlong(DIM == 3 ? q.w : q.z);
+            ex = fix_diff(a.x, q.x);
+            ey = fix_diff(a.y, q.y);
+            if (px) ex = image(ex, hx, Lx);
+            if (py) ey = image(ey, hy, Ly);
+            if (DIM == 3) {
+                ez = fix_diff(a.z, q.z);
+                if (pz) ez = image(ez, hz, Lz);
             }
+            // overlap test (r1 + r2)^2 >= d^2: in FP32 outside a 1e-5 guard
+            // band (the differences exact, ~2^-22 relative as FP32), else on
+            // the integers
+            const float fx = fix_len(ex), fy = fix_len(ey), fz = DIM == 3 ? fix_len(ez) : 0.f;
+            float m32 = fx * fx;
+            m32 = fmaf(fy, fy, m32);
+            if (DIM == 3) m32 = fmaf(fz, fz, m32);
+            const long long R = q1 + q2;
+            const float R32 = fix_len(R) * rscale;
+            const float RR = R32 * R32;
+            if (m32 < RR * (1.f - 1e-5f))
+                over = true;
+            else if (!(m32 > RR * (1.f + 1e-5f)))
+                over = overlap_exact<DIM>(ex, ey, ez, max(R, 0LL), radk);
         }
         const unsigned mask = __ballot_sync(0xffffffffu, over);
         if (over) {
@@ -507,7 +557,6 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
     }
     if (lane < cnt) process((head + lane) & (kQueue - 1), lane);
     scatter(head, cnt);
-
     pairs_fold<DIM, RES>(b, vb, vg, sAo, sAor, smem, rx, rsm);
 }
 CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW>), k_pairs, (<DIM, GAS, FLOW>), __launch_bounds__(kBlock, 4))
@@ -530,20 +579,23 @@ static __device__ __noinline__ double wall_velocity(double f0, double r, double 
 // A predicted position against the flow's box and the walls: as fixed point
 // (exact comparisons), and in FP64 for a bubble the fixed point does not hold.
 struct FixPlace {
-    long long q[3], r;
+    long long q[3];
+    long long r;  // in units 2^-(fix_b + rad_k)
+    int rad_k;
+    // in the positions' unit, rounded down: a distance d <= r where d <= rad
+    __device__ __forceinline__ unsigned long long rad() const { return fx_abs(r) >> rad_k; }
     // addFlowVelocity, src/kernels.cu:497-544: between the faces or touching one
     __device__ __forceinline__ bool in_flow(const DevConst &k, int a) const {
-        const unsigned long long rad = fx_abs(r);
-        return (q[a] < k.vhq[a] && q[a] > k.vlq[a]) || fix_gap(k.vlq[a], q[a]) <= rad ||
-               fix_gap(k.vhq[a], q[a]) <= rad;
+        return (q[a] < k.vhq[a] && q[a] > k.vlq[a]) || fix_gap(k.vlq[a], q[a]) <= rad() ||
+               fix_gap(k.vhq[a], q[a]) <= rad();
     }
     // touches the nearer wall, the upper one of two
     __device__ __forceinline__ bool touches(const DevConst &k, int a, double &velocity) const {
         const unsigned long long dl = fix_gap(q[a], k.wlq[a]), dh = fix_gap(q[a], k.whq[a]);
         const bool low = dl < dh;
         const unsigned long long d = low ? dl : dh;
-        if (d > fx_abs(r)) return false;
-        velocity = wall_velocity(k.f0, fx_to_double_signed(r, -k.fix_b),
+        if (d > rad()) return false;
+        velocity = wall_velocity(k.f0, fx_to_double_signed(r, -k.fix_b - rad_k),
                                  fx_to_double_any(d, -k.fix_b),
                                  q[a] >= (low ? k.wlq[a] : k.whq[a]));
         return true;
@@ -644,7 +696,7 @@ static __device__ __noinline__ Moves far_moves(const double *pred, double *const
                                                int i, int fixb, double cx, double cy, double cz,
                                                double cr) {
     auto row = [&](int role) { return ds[c->drole[role]][i]; };
-    const State p = ld_state<DIM>(pred, ds, c, i, fixb);
+    const State p = ld_state<DIM>(pred, ds, c, i, fixb, fixb + c->rad_k);
     Moves m;
     long long e = 0;  // a NaN counts as the largest error
     e = max_bits(e, abs_bits(p.x - cx));
@@ -705,7 +757,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     const double mfa = c->mfa, mfb = c->mfb;
     const double kq = DIM == 3 ? k.K * 0.25 : k.K * (1.0 / kPi);
     const double drag = 1.0 - k.wall_drag;
-    const int fixb = k.fix_b;
+    const int fixb = k.fix_b, radk = c->rad_k;
     long long merr = 0, mrad = 0, mexp = 0;
     double vol = 0.0;
     const int marks = c->marks;
@@ -741,12 +793,12 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
             const int nn = flow ? NN[i] : 0;
             Vel3 v;
             if (far) {
-                const State f = ld_state<DIM>(b.pred, b.ds, c, i, fixb);
+                const State f = ld_state<DIM>(b.pred, b.ds, c, i, fixb, fixb + radk);
                 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz,
                                            RealPlace{{f.x, f.y, f.z}, f.r}, a1.y, a1.z, a1.w, nn);
             } else {
                 v = boundary_velocity<DIM>(k, flow, shear, drag, vpx, vpy, vpz,
-                                           FixPlace{{qx, qy, qz}, qr}, a1.y, a1.z, a1.w, nn);
+                                           FixPlace{{qx, qy, qz}, qr, radk}, a1.y, a1.z, a1.w, nn);
             }
             vpx = v.x;
             vpy = v.y;
@@ -770,6 +822,8 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         // over the foam is used (the search trigger)
         double dist = fx_norm<DIM>(fx - fx_from_double(s0, fixb, far),
                                    fy - fx_from_double(s1, fixb, far), sz, fixb);
+        far |= em >> (63 - radk) != 0;
+        em <<= radk;  // in the radius's unit
         int del = 0;
         double cr = 0.0;
         if (gas) {  // mean-field gas exchange and radius, src/kernels.cu:390-431
@@ -779,7 +833,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 area = times4(ri.y);
             } else {
                 inv = p.w;
-                area = kPi * (is_far(p) ? CB_D(RRN)[i] : fx_to_double_signed(qr, -fixb));
+                area = kPi * (is_far(p) ? CB_D(RVQ3)[i] : fx_to_double_signed(qr, -(fixb + radk)));
             }
             double vr = mfa - inv;
             vr *= mfb * (area - ov);
@@ -787,7 +841,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
             vr *= DIM == 3 ? kq * (inv * inv) : kq * inv;
             vpr = vr;
             cr = fma(h, v3 + vr, r0);
-            em = max(em, fx_abs(qr - fx_from_double(cr, fixb, far)));
+            em = max(em, fx_abs(qr - fx_from_double(cr, fixb + radk, far)));
             dist += cr - s3;
             if (__double_as_longlong(cr) > __double_as_longlong(k.min_rad)) {  // cr > minRad
                 vol = fma(DIM == 3 ? cr * cr : cr, cr, vol);
@@ -796,6 +850,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 ndel++;
             }
             mrad = max_bits(mrad, cr);
+            CB_D(RRN)[i] = cr;
             CB_D(RVP3)[i] = vpr;
             bad |= !finite_bits(cr);
         }
@@ -805,7 +860,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
             inc = fx_norm<DIM>(fx_from_double(x0, fixb, far) - fx,
                                fx_from_double(y0, fixb, far) - fy,
                                DIM == 3 ? fx_from_double(z0, fixb, far) - fz : 0, fixb);
-        long long e = __double_as_longlong(fx_to_double_any(em, -fixb));
+        long long e = __double_as_longlong(fx_to_double_any(em, -(fixb + radk)));
         if (far) {
             const Moves m = far_moves<DIM>(b.pred, b.ds, c, i, fixb, cx, cy, cz, cr);
             e = __double_as_longlong(m.err);
@@ -814,7 +869,6 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
         }
         mexp = max_bits(mexp, dist);
         if (path) CB_D(RPATHN)[i] = path0 + inc;
-        if (gas) CB_D(RRN)[i] = cr;
         CB_D(RERR)[i] = __longlong_as_double(max(e, __double_as_longlong(err0)));  // both >= 0
         merr = max(merr, e);
         CB_D(RXN)[i] = cx;
@@ -866,6 +920,7 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
     const double fDel = fold_partials(b.part + 4 * G, G, false, smem);
     const double fBad = fold_partials(b.part + 5 * G, G, false, smem);
     if (threadIdx.x != 0) return;
+    b.run->far = 0;
     finish_attempt<DIM>(c, k, {fErr, fRad, fExp, fVol, (int)fDel, (int)fBad});
 }
 CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBlock, 3))
@@ -923,22 +978,22 @@ __global__ void __launch_bounds__(kBlock) k_boot(Bufs b, int phase) {
                  *R = drow(b, c, RR);
     double *O0 = drow(b, c, RVO0), *O1 = drow(b, c, RVO1), *O2 = drow(b, c, RVO2),
            *O3 = drow(b, c, RVO3), *PATH = drow(b, c, RPATH);
-    const int fixb = b.k->fix_b;
+    const int fixb = b.k->fix_b, radb = fixb + c->rad_k;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double *acc = b.acc + (size_t)i * kAcc;
         if (phase == 0) {
             const double r = R[i];
             const double inv = 1.0 / r, rsq = r * r;
             if (DIM == 3) reinterpret_cast<double2 *>(b.invr)[i] = make_double2(inv, rsq);
-            st_state<DIM>(b, c, i, X[i], Y[i], DIM == 3 ? Z[i] : 0.0, r, inv, fixb);
+            st_state<DIM>(b, c, i, X[i], Y[i], DIM == 3 ? Z[i] : 0.0, r, inv, fixb, radb);
             O0[i] = O1[i] = O2[i] = O3[i] = 0.0;
             PATH[i] = 0.0;
         } else {
             double4_32a a = reinterpret_cast<double4_32a *>(acc)[0];
             if (phase == 1) {
-                const State p = ld_state<DIM>(b.pred, b.ds, c, i, fixb);
+                const State p = ld_state<DIM>(b.pred, b.ds, c, i, fixb, radb);
                 st_state<DIM>(b, c, i, p.x + a.x * ts, p.y + a.y * ts, p.z + a.z * ts, p.r,
-                              b.pred[4 * (size_t)i + 3], fixb);
+                              b.pred[4 * (size_t)i + 3], fixb, radb);
             } else {
                 O0[i] = a.x;
                 O1[i] = a.y;

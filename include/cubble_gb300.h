@@ -42,8 +42,13 @@ extern "C" {
 #define CB_ERR_NO_DEVICE 7        /* no CUDA device / extension unusable      */
 #define CB_ERR_STATE 8            /* call made in the wrong order             */
 
-#define CB_PRECISION_FP64 0  /* FP64 form (pair terms in 64-bit fixed point, to
-                                within the rounding of FP64)                  */
+#define CB_PRECISION_FP64 0  /* FP64 form. Pair terms in 64-bit fixed point, to
+                                within the rounding of FP64 on the predicted
+                                positions and radii, which keep the bits of
+                                their doubles down to 2^-9 of the largest box
+                                corner and 2^-8 of the largest radius (below
+                                that, absolute units of 2^-62 of twice and four
+                                times these)                                 */
 #define CB_PRECISION_MIXED 1 /* FP32 pair geometry on exact 64-bit fixed-point
                                 differences, FP64 positions/volume/error     */
 #define CB_PRECISION_FP64_FF 2 /* FP64 state, update and sums with the pair terms

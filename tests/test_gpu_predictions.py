@@ -143,3 +143,59 @@ def test_a_step_far_too_large(oracle_mod, dt, dim, options, precision):
     for k in ("max_error", "max_expansion", "total_overlap_area", "total_area"):
         assert a[k] == pytest.approx(b[k], rel=1e-9), k
     assert g.report()["time_step"] == o.report()["time_step"] == dt * 0.37
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("options", [{}, dict(wall=(1, 0, 0), wall_drag=0.1)])
+def test_radii_in_a_wide_box(oracle_mod, dim, options, precision):
+    """A radius keeps the bits of its double in a box 2^20 of it wide, where the
+    unit of the positions is 2^-41: positions that are multiples of 2^-20 leave
+    the radii as the only source of rounding. Bar: the oracle's own, ~1e-15 of
+    each term (6e-16 R^2 for the overlap), ten times that through the mean-field
+    difference of nearly equal 1/r."""
+    cfg, st = lattice(dim, 18.0, **options)
+    side = 2.0 ** 20
+    cfg.tfr = cb._abi.D3(side, side, side if dim == 3 else 0.0)
+    rng = np.random.default_rng(5)
+    n = len(st["r"])
+    for k in "xyz"[:dim]:
+        st[k] = np.round(st[k] * 2.0 ** 20) / 2.0 ** 20
+    for k in "yz"[:dim - 1]:
+        st[k] = st[k] + 2.0 ** 18
+    st["x"] = st["x"] + (0.0 if options else 2.0 ** 18)
+    st["r"] = rng.uniform(0.9, 1.1, n)
+    g, o = both(oracle_mod, cfg, st, precision)
+    g.set_pairs(*o.pairs())
+    a, b = g.attempt(), o.attempt()
+    assert np.count_nonzero(b["overlap"]) > n / 2
+    rows = ["dxdtp", "drdtp", "rp", "overlap"]
+    assert_rows_close(a, b, rows, 2e-14, "wide box ")
+    for k in ("total_overlap_area", "total_overlap_area_per_radius", "total_area"):
+        assert a[k] == pytest.approx(b[k], rel=2e-14), k
+    # the radius error |predicted - corrected|, beside no motion along y
+    i = np.argmax(b["error"])
+    assert abs(a["error"][i] - b["error"][i]) <= 2 * np.spacing(2.0 ** 18)
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("options", [{}, dict(wall=(1, 1, 0), wall_drag=0.1, use_flow=1,
+                                              flow_lbb=(0.0,) * 3, flow_tfr=(9.0,) * 3,
+                                              flow_vel=(0.02, 0.01, 0.0))])
+def test_a_radius_beyond_what_the_search_saw(oracle_mod, dim, options, precision):
+    """A bubble that grows to ten times the largest radius of the last search in
+    one prediction leaves the radii's range, which that search sets. Bar: its
+    own overlaps and area, of ~10^2, dominate the sums: 1e-13 of each row."""
+    cfg, st = lattice(dim, 18.0, **options)
+    n = len(st["r"])
+    st["drdt"] = np.zeros(n)
+    st["drdt"][4] = 6e4
+    g, o = both(oracle_mod, cfg, st, precision)
+    a, b = g.attempt(), o.attempt()
+    i = int(np.flatnonzero(o.get_state()["index"] == 4)[0])
+    assert b["error"][i] > 3.0 and b["overlap"][i] > 0.0
+    rows = ["dxdtp", "dydtp", "drdtp", "rp", "overlap", "error"]
+    assert_rows_close(a, b, rows, 1e-13, "grown ")
+    for k in ("total_overlap_area", "total_area", "max_error", "total_volume_new"):
+        assert a[k] == pytest.approx(b[k], rel=1e-13), k
