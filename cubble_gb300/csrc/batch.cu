@@ -303,7 +303,6 @@ RunLaunch batch_run_launch(cb_batch *b) {
     r.grid = b->run_blocks;
     r.block = kBlock;
     r.wide = b->run_wide;
-    r.threads = 0;
     r.stream = b->stream;
     r.steps = -1;
     r.mirror = nullptr;

@@ -695,12 +695,9 @@ struct RunCtx {
     unsigned phase;  // arrivals that complete the next barrier
     unsigned vg;
     int *failed;     // shared
-    int threads;     // of the correct kernel in a launch per phase (mixed form)
     // this thread's share of the prediction's sums, reduced with the pair
     // phase's (FP64 form)
     double sA, sAr;
-    // mixed form, 2D, first thread: area_over_radius_2d of both kernels
-    double ar[2];
     int *leave;  // shared; batched runs only
 };
 constexpr int kRunPolls = 1 << 22;         // a poll is an L2 round trip: seconds in all
@@ -1139,7 +1136,6 @@ constexpr int kRunNarrow = 2, kRunWide = 3, kRunWideMx = 4;
 struct RunLaunch {
     int grid, block;
     bool wide = false;  // the form with more blocks per SM
-    int threads;  // of the correct kernel in a launch per phase (mixed form)
     cudaStream_t stream;
     long long steps;
     Ctrl *mirror;
@@ -1159,7 +1155,7 @@ inline void launch_coop(K kernel, const RunLaunch &r, const Bufs &b) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, b, r.foams, r.map, r.round, r.mirror, r.steps, r.threads);
+    cudaLaunchKernelEx(&cfg, kernel, b, r.foams, r.map, r.round, r.mirror, r.steps);
     *r.launches += 1;
 }
 

@@ -291,7 +291,6 @@ RunLaunch search_launch(cb_context *c, bool force) {
     RunLaunch r;
     r.block = kBlock;
     r.grid = std::min(2 * c->sms, 4 * c->launch.cover);
-    r.threads = 0;
     r.stream = c->stream;
     r.steps = force ? 1 : 0;
     r.mirror = c->hctrl;
@@ -325,7 +324,6 @@ RunLaunch run_launch(cb_context *c, int64_t n_steps) {
     const int bps = !r.wide ? kRunNarrow : (c->hk.mixed ? kRunWideMx : kRunWide);
     r.block = warps <= 4 * 2 * c->sms ? 128 : kBlock;
     r.grid = (int)std::min<long long>(bps * c->sms, (32 * warps + r.block - 1) / r.block);
-    r.threads = 4 * c->sms * kBlock;
     r.stream = c->stream;
     r.steps = n_steps;
     r.mirror = c->hctrl;

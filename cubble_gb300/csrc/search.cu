@@ -1196,7 +1196,7 @@ __device__ __forceinline__ void search_phases(const Bufs &b, int vb, int vg, Run
 template <int DIM>
 __global__ void __launch_bounds__(kBlock, 2) k_search_run(Bufs b, const Bufs *foams,
                                                        const RunBlock *map, RunRound *, Ctrl *mirror,
-                                                       long long force, int) {
+                                                       long long force) {
     __shared__ RunShared rs;
     int vb = blockIdx.x, vg = gridDim.x;
     if (map) {
@@ -1210,7 +1210,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_search_run(Bufs b, const Bufs *fo
         return;
     }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, 0, 0.0, 0.0};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, 0.0, 0.0, nullptr};
     run_enter(&rs, b, -1);
     search_phases<DIM>(b, vb, vg, &rx);
     run_exit(&rs, ctrl, mirror, &rx, vb);

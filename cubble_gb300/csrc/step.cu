@@ -934,7 +934,7 @@ CB_KERNEL_PAIR((template <int DIM>), k_correct, (<DIM>), __launch_bounds__(kBloc
 template <int DIM, bool GAS, bool FLOW, int BPS>
 __global__ void __launch_bounds__(kBlock, BPS) k_run(Bufs b, const Bufs *foams,
                                                     const RunBlock *map, RunRound *round, Ctrl *mirror,
-                                                    long long n_steps, int threads) {
+                                                    long long n_steps) {
     __shared__ RunShared rs;
     __shared__ RunRed rsm;
     int vb = blockIdx.x, vg = gridDim.x;
@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(kBlock, BPS) k_run(Bufs b, const Bufs *foams,
         if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
     }
     Ctrl *ctrl = b.ctrl;
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, threads, 0.0, 0.0, {0.0, 0.0}, nullptr};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, 0.0, 0.0, nullptr};
     run_enter(&rs, b, n_steps);
     if (round) rx.leave = &rs.leave;
     RunWait wait;

@@ -188,32 +188,11 @@ __device__ __forceinline__ T ld_row(const T *p) {
     return RES ? *p : __ldg(p);
 }
 
-// The sum of area over radius in 2D, 2 pi for every bubble, with the FP32
-// rounding of the kernels launched per phase: each of their `threads` sums
-// its bubbles' constants, and in the correct kernel (BLOCK) a block its eight
-// warps' sums. That rounding (up to 10^-7 of the sum) shifts every bubble's gas
-// flux alike and shows in the total volume at 10^-9 over 300 steps, so a
-// resident run uses the same value: a foam must not depend on the path that
-// runs it. Computed once per run: at the end of every attempt its integer
-// divisions took 0.6 us (N = 10^4: 14.6 -> 14.0 us per attempt).
-template <bool BLOCK>
-__device__ __forceinline__ double area_over_radius_2d(int n, int threads) {
-    constexpr float c = 2.f * (float)kPi;
-    const int each = n / threads, more = n - each * threads;
-    float s = 0.f;
-    for (int q = 0; q < each; q++) s += c;
-    const float s1 = s + c;
-    if (!BLOCK) return (double)s * (threads - more) + (double)s1 * more;
-    float b = 0.f, b1 = 0.f;  // blocks whose threads all sum s, s1
-    for (int w = 0; w < kBlock / 32; w++) {
-        b += 32.f * s;
-        b1 += 32.f * s1;
-    }
-    const int full1 = more / kBlock, part = more - full1 * kBlock;
-    const int full = threads / kBlock - full1 - (part ? 1 : 0);
-    double t = (double)b * full + (double)b1 * full1;
-    if (part) t += (double)s1 * part + (double)s * (kBlock - part);
-    return t;
+// The sum of area over radius in 2D: the constant of the bubbles' areas (2 pi as
+// FP32, as in every bubble's gas-exchange term, whose balance it enters) for
+// each of n bubbles, exact.
+__device__ __forceinline__ double area_over_radius_2d(int n) {
+    return (double)(2.f * (float)kPi) * (double)n;
 }
 
 // ---------------------------------------------------------------- predict
@@ -271,7 +250,7 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
             if (gas) {
                 const float apr = DIM == 3 ? (4.f * (float)kPi) * rp : 2.f * (float)kPi;
                 sA = fmaf(apr, rp, sA);
-                if (!(RES && DIM == 2)) sAr += apr;  // 2D: area_over_radius_2d
+                if (DIM == 3) sAr += apr;  // 2D: area_over_radius_2d
             }
         }
     }
@@ -292,7 +271,7 @@ __device__ __forceinline__ void k_predict_mx_body(const Bufs &b, const int vb, c
         const double fAr = fold_partials(b.part + 1 * vg, vg, false, smem);
         if (threadIdx.x == 0) {
             b.ctrl->sumA = fA;
-            b.ctrl->sumAr = fAr;
+            b.ctrl->sumAr = DIM == 2 && gas ? area_over_radius_2d(n) : fAr;
             b.ctrl->done[DC_PREDICT] = 0;
         }
     }
@@ -639,7 +618,8 @@ __device__ __forceinline__ void k_pairs_mx_body(const Bufs &b, const int vb, con
                 cc->mfb = k.kappa * k.ain * (double)cc->n / sumA;
             } else {
                 if (fresh)
-                    sumAr = DIM == 3 ? __ldcg(&rx->acc->psum[3]) : rx->ar[0];
+                    sumAr = DIM == 2 && GAS ? area_over_radius_2d(cc->n)
+                                            : __ldcg(&rx->acc->psum[3]);
                 cc->mfa = (sumAr - fAor) / (sumA - 2.0 * fAo);
                 cc->sumAo = 2.0 * fAo;
                 cc->sumAor = fAor;
@@ -946,10 +926,10 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
                     const float apr = DIM == 3 ? (4.f * (float)kPi) * rp1 : 2.f * (float)kPi;
                     if (u) {
                         cA1 = fmaf(apr, rp1, cA1);
-                        if (!(RES && DIM == 2)) cAr1 += apr;  // area_over_radius_2d
+                        if (DIM == 3) cAr1 += apr;  // 2D: area_over_radius_2d
                     } else {
                         cA0 = fmaf(apr, rp1, cA0);
-                        if (!(RES && DIM == 2)) cAr0 += apr;
+                        if (DIM == 3) cAr0 += apr;
                     }
                 }
             }
@@ -972,7 +952,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
         run_finish<DIM>(c, k, g, ts, rx->leave, [&] {
             const double a0 = __ldcg(&g->csum[1]), a1 = __ldcg(&g->csum[2]);
             double r0 = __ldcg(&g->csum[3]), r1 = __ldcg(&g->csum[4]);
-            if (DIM == 2) r0 = r1 = rx->ar[1];
+            if (DIM == 2) r0 = r1 = area_over_radius_2d(n);
             c->cand_sumA[0] = a0;
             c->cand_sumA[1] = a1;
             c->cand_sumAr[0] = r0;
@@ -987,8 +967,10 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
         if (GAS) {
             atomicAdd(&c->cand_sumA[0], (double)v.cA[0]);
             atomicAdd(&c->cand_sumA[1], (double)v.cA[1]);
-            atomicAdd(&c->cand_sumAr[0], (double)v.cAr[0]);
-            atomicAdd(&c->cand_sumAr[1], (double)v.cAr[1]);
+            if (DIM == 3) {
+                atomicAdd(&c->cand_sumAr[0], (double)v.cAr[0]);
+                atomicAdd(&c->cand_sumAr[1], (double)v.cAr[1]);
+            }
         }
         atomicMax(&c->amax_err, v.err);
         atomicMax(&c->amax_rad, v.rad);
@@ -1007,6 +989,7 @@ __device__ __forceinline__ void k_correct_mx_body(const Bufs &b, const int vb, c
     const double fDel = (double)vc->acnt_del, fBad = (double)vc->acnt_bad;
     c->amax_err = c->amax_rad = c->amax_exp = 0;
     c->acnt_del = c->acnt_bad = 0;
+    if (GAS && DIM == 2) c->cand_sumAr[0] = c->cand_sumAr[1] = area_over_radius_2d(n);
     finish_attempt<DIM>(c, k, {fErr, fRad, fExp, fVol, (int)fDel, (int)fBad});
 }
 CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_mx, (<DIM, GAS, FLOW, WALLS>), __launch_bounds__(kBlock, DIM == 3 ? 3 : 4))
@@ -1019,7 +1002,7 @@ CB_KERNEL_PAIR((template <int DIM, bool GAS, bool FLOW, bool WALLS>), k_correct_
 template <int DIM, bool GAS, bool FLOW, bool WALLS, int BPS>
 __global__ void __launch_bounds__(kBlock, BPS) k_run_mx(Bufs b, const Bufs *foams,
                                                     const RunBlock *map, RunRound *round, Ctrl *mirror,
-                                                    long long n_steps, int threads) {
+                                                    long long n_steps) {
     __shared__ RunShared rs;
     __shared__ RunRed rsm;
     int vb = blockIdx.x, vg = gridDim.x;
@@ -1031,15 +1014,8 @@ __global__ void __launch_bounds__(kBlock, BPS) k_run_mx(Bufs b, const Bufs *foam
         if (!(b.ctrl->bsel & SEL_ATTEMPT)) return;
     }
     Ctrl *ctrl = b.ctrl;
-    // threads of the launch per phase (area_over_radius_2d): the virtual grid
-    // of a batched foam, else four resident blocks per SM
-    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed,
-              map ? b.ctrl->vgrid_a * kBlock : threads, 0.0, 0.0, {0.0, 0.0}, nullptr};
+    RunCtx rx{b.run, nullptr, 0u, (unsigned)vg, &rs.failed, 0.0, 0.0, nullptr};
     run_enter(&rs, b, n_steps);
-    if (DIM == 2 && threadIdx.x == 0) {  // once: a run ends where bubbles are deleted
-        rx.ar[0] = area_over_radius_2d<false>(rs.c.n, rx.threads);
-        rx.ar[1] = area_over_radius_2d<true>(rs.c.n, rx.threads);
-    }
     if (round) rx.leave = &rs.leave;
     RunWait wait;
     int attempts = 0;

@@ -74,7 +74,6 @@ extern "C" __attribute__((visibility("default"))) int give_up(const cb_config *c
     RunLaunch r;
     r.grid = blocks;
     r.block = kBlock;
-    r.threads = 0;
     r.stream = c->stream;
     r.steps = 1;
     r.mirror = nullptr;
