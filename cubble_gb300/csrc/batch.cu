@@ -622,7 +622,12 @@ int cb_batch_autotune(cb_batch *b, int32_t steps, int32_t *tile_out) {
     };
     double best = -1.0, rate = 0.0;
     int best_tile = b->tile;
+    // resident runs use neither tile nor pair_run: the same number of trials goes
+    // to the cell edge, each candidate's fastest counts
+    const bool launched = b->run_blocks == 0, mixed = b->first()->hk.mixed;
+    const double scales[] = {1.0, 1.15, 1.3};
     for (int t : {512, 1024, 2048, 4096, 8192}) {
+        if (!launched) break;
         b->tile = t;
         int rc = trial(&rate);
         if (rc) return rc;
@@ -636,9 +641,10 @@ int cb_batch_autotune(cb_batch *b, int32_t steps, int32_t *tile_out) {
     cb_tuning bt = b->first()->tune;
     const cb_tuning keep0 = bt;
     best = -1.0;
-    for (double cs : {1.0, 1.15, 1.3}) {
+    const int trials = launched ? 3 : 5 + 3 + (mixed ? 3 : 0);
+    for (int n = 0; n < trials; n++) {
         cb_tuning q = keep0;
-        q.cell_scale = cs;
+        q.cell_scale = scales[n % 3];
         int rc = cb_batch_set_tuning(b, &q);
         if (!rc) rc = trial(&rate);
         if (rc) return rc;
@@ -647,7 +653,7 @@ int cb_batch_autotune(cb_batch *b, int32_t steps, int32_t *tile_out) {
             bt = q;
         }
     }
-    if (b->first()->hk.mixed) {
+    if (launched && mixed) {
         const cb_tuning keep1 = bt;
         best = -1.0;
         for (int run : {2, 4, 8}) {

@@ -1359,7 +1359,9 @@ int cb_autotune(cb_context *c, int32_t reps, cb_tuning *best) {
     const int blocks[] = {0, 2, 3};
     double best_pairs = 1e300;
     cb_tuning bt = t;
-    for (int r = 0; r < nruns; r++)
+    // resident runs launch neither kernel: those knobs stay as they are there
+    const bool launched = !resident(c);
+    for (int r = 0; launched && r < nruns; r++)
         for (int bl : blocks) {
             cb_tuning q = t;
             q.pair_run = runs[r];
@@ -1374,6 +1376,7 @@ int cb_autotune(cb_context *c, int32_t reps, cb_tuning *best) {
     // predict + correct: resident blocks per SM
     double best_step = 1e300;
     for (int bl : {0, 1, 2, 3}) {
+        if (!launched) break;
         cb_tuning q = bt;
         q.step_blocks = bl;
         if ((rc = apply_tuning(c, q)) || (rc = profile_attempts(c, reps, ms))) return rc;

@@ -299,8 +299,10 @@ CB_API int cb_profile_search(cb_context *ctx, int32_t reps, double *ms);
  * Launch and search knobs of a context. None changes the pair set or the
  * arithmetic of a pair; they change how work is cut into threads, blocks and
  * cells (so the bubble order after a search and the order of reductions,
- * which moves FP64 sums by rounding only). No counterpart in the reference,
- * whose launch shape is fixed (5120 x 384, src/data_definitions.h:28-29) and
+ * which moves FP64 sums by rounding only). Contexts that advance by resident
+ * runs (capacity up to 5 10^6) use cell_scale alone: the other knobs shape the
+ * kernels of the launch per phase. No counterpart in the reference, whose
+ * launch shape is fixed (5120 x 384, src/data_definitions.h:28-29) and
  * whose cell edge is 2 (maxR + skin) (src/simulator.cu:69-75). */
 typedef struct cb_tuning {
     double cell_scale;   /* cell edge of the neighbour search in units of
@@ -322,7 +324,8 @@ CB_API int cb_get_tuning(cb_context *ctx, cb_tuning *tuning);
 /* Autotuner: on the loaded, searched state, times the pair kernel for every
  * (pair_run, pair_blocks) candidate and the predict + correct kernels for
  * every step_blocks candidate (`reps` attempts each, not accepted: the state
- * does not advance), and one neighbour search per cell_scale candidate (the
+ * does not advance; contexts that advance by resident runs keep these knobs as
+ * they are), and one neighbour search per cell_scale candidate (the
  * state is left searched); keeps the fastest of each and returns them in
  * *best. The choice is also kept process-wide for contexts of the same
  * dimensionality, precision and capacity bucket (floor(log2(capacity))):
@@ -369,7 +372,9 @@ CB_API int cb_batch_set_tile(cb_batch *batch, int32_t bubbles_per_block);
  * each candidate tile (512 ... 8192 bubbles per block), then with each
  * cell_scale and, in the mixed form, each pair_run candidate of cb_tuning
  * (applied to every foam), keeps the fastest of each and returns the tile in
- * *tile (the other knobs: cb_get_tuning of any foam's context). */
+ * *tile (the other knobs: cb_get_tuning of any foam's context). A batch that
+ * advances by resident runs (up to 2 10^6 bubbles) has neither a tile nor
+ * pair_run in them: it keeps both and gives as many trials to cell_scale alone. */
 CB_API int cb_batch_autotune(cb_batch *batch, int32_t steps_per_trial, int32_t *tile);
 /* Applies the knobs of cb_tuning to every foam of the batch. */
 CB_API int cb_batch_set_tuning(cb_batch *batch, const cb_tuning *tuning);
