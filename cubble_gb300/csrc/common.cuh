@@ -857,7 +857,7 @@ struct RunRound {
 };
 // When a foam ends its run although it could go on, because others wait: once
 // the waiting adds up to about what a round costs beyond its attempts (the
-// decision and the batched deletions and searches, ~100 us). Kept by the first
+// decision and the batched deletions and searches, ~200 us). Kept by the first
 // thread of the foam's first block.
 struct RunWait {
     float idle = 0.f;

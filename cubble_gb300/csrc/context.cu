@@ -1,8 +1,10 @@
 // Host side of the C ABI (include/cubble_gb300.h): the context owns every
-// device buffer of one foam, runs the step loop either eagerly (one small
-// control-block read per attempt, like the reference's per-step copy at
-// src/simulator.cu:219-221) or as a single CUDA graph whose while/if
-// conditional nodes are driven by the device (no host round trip per step).
+// device buffer of one foam and runs the step loop: up to kRunCapacity bubbles
+// by resident runs (all attempts up to a deletion, a search or the end inside
+// one cooperative kernel), beyond that by a launch per phase, either from the
+// host (one small control-block read per attempt, like the reference's
+// per-step copy at src/simulator.cu:219-221) or as a single CUDA graph whose
+// while/if conditional nodes are driven by the device.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -576,10 +578,6 @@ void fill_report(const cb_context *c, cb_report *r) {
 
 }  // namespace cbg
 
-namespace {
-
-}  // namespace
-
 // ====================================================================== ABI
 extern "C" {
 
@@ -1117,7 +1115,7 @@ static int integrate_impl(cb_context *c, int64_t n_steps, bool fresh) {
 }
 
 int cb_integrate(cb_context *c, int64_t n_steps, cb_report *r) {
-    // back-to-back graph integrations skip the control-block read: no call
+    // back-to-back integrations skip the control-block read: no call
     // has run on any context since the last one returned
     const bool fresh = c && c->mirror_call == cbg::g_calls.load(std::memory_order_relaxed);
     CB_ENTER(c);

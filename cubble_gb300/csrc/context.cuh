@@ -60,8 +60,7 @@ struct cb_context {
     cudaGraphExec_t gexec = nullptr;
     int graph_key = -1;
     cbg::PhaseKernels graph_kernels;
-    long long graph_attempts0 = 0, graph_searches0 = 0, graph_deletes0 = 0;
-    // g_calls when a graph cb_integrate returned with hctrl equal to the
+    // g_calls when a cb_integrate returned with hctrl equal to the
     // device's control block and the stream idle
     unsigned long long mirror_call = ~0ull;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
