@@ -167,9 +167,9 @@ CB_KERNEL_PAIR((template <int DIM>), k_predict, (<DIM>), __launch_bounds__(kBloc
 //     instead of five (alone: 202 -> 177 us);
 //   * overlap areas are accumulated in units of ov_unit (pi in 3D, 2 in 2D);
 //     the unit is applied to the global sums and in the correct kernel.
-// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 123 us (2D 117 -> 84, 3D
-// without gas exchange 141 -> 96). Nothing is saturated now: issue 59 %, L1 62 %
-// of its wavefronts, FP64 31 %; three or four blocks per SM make no difference,
+// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 120 us (2D 117 -> 85, 3D
+// without gas exchange 141 -> 96). Nothing is saturated now: issue 61 %, L1 61 %
+// of its wavefronts, FP64 33 %; three or four blocks per SM make no difference,
 // record loads a chunk ahead (108 registers) cost 8 us.
 __device__ __forceinline__ void red_add(double *p, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v));
