@@ -229,15 +229,19 @@ CB_HD bool fx_pair(int64_t ex, int64_t ey, int64_t ez, int64_t q1, int64_t q2, i
         const int sc = 62 - u - B;                // R = R' 2^sc
         out.inside = M < fx_square(big);
         uint64_t w;  // units 2^-62
-        if (out.inside) {
-            w = (uint64_t)fx_square((R >> 1) - (D >> 1)) << 2;  // min(r1, r2)^2
+        int e2 = -62 + 2 * sc;
+        if (out.inside) {  // min(r1, r2)^2, at its own scale
+            const uint64_t q = (uint64_t)((R >> 1) - (D >> 1));
+            const int k = ff_clz((uint32_t)(q >> 32)) - 2;  // up to 30
+            w = (uint64_t)fx_square((int64_t)fx_shl(q, k)) << 2;
+            e2 -= 2 * k;
         } else {
             const int64_t p = fx_square(R) - M, q = M - fx_square(D);
             const uint64_t t = fx_mulhi((uint64_t)(p > 0 ? p : 0), (uint64_t)(q > 0 ? q : 0));
             const uint64_t YY = fx_mulhi(Y << 2, Y << 2);  // y^2 2^56, y <= 2
             w = (fx_mulhi(t, YY) << 12) | ((t * YY) >> 52);  // 4 a^2 2^60
         }
-        out.oa = fx_to_double(w, -62 + 2 * sc);
+        out.oa = fx_to_double(w, e2);
     }
     return true;
 }

@@ -248,15 +248,20 @@ static __device__ __noinline__ bool overlap_exact(long long ex, long long ey, lo
 }
 
 // The terms of a pair fx_pair does not take, in FP64: centres much closer than
-// the radii. The force goes to rs[0], rs[kT], ...; returns the overlap as
-// FxTerms::oa. Nothing for a marked bubble, whose pairs far_pairs takes.
+// the radii, or radii more than 1 : 31 apart (its absolute error of 2^-56 R^2 in
+// the overlap is then more than FP64's, which scales with the smaller radius; at
+// 1 : 1000 2 10^-12 against 6 10^-15 of it). A radius that its unit does not hold
+// exactly is predicted again from the rows. The force goes to rs[0], rs[kT], ...;
+// returns the overlap as FxTerms::oa. Nothing for a marked bubble, whose pairs
+// far_pairs takes.
 // Row length of the transposed results (32 pairs): the 8-byte loads of four
 // pairs' components fall on distinct banks, but for the fifth row.
 constexpr int kT = 36;
-template <int DIM>
+template <int DIM, bool GAS>
 static __device__ __noinline__ double pair_slow(long long ex, long long ey, long long ez,
                                                 long long q1, long long q2, int K,
-                                                const DevConst &k, double *rs) {
+                                                const DevConst &k, double *const *ds,
+                                                const Ctrl *c, const int2 *ij, double *rs) {
     if ((q1 | q2) < 0) {
 #pragma unroll
         for (int t = 0; t < DIM; t++) rs[t * kT] = 0.0;
@@ -264,7 +269,12 @@ static __device__ __noinline__ double pair_slow(long long ex, long long ey, long
     }
     const double unit = k.fix_unit, runit = ldexp(unit, -K), f0 = k.f0;
     const double dx = (double)ex * unit, dy = (double)ey * unit, dz = (double)ez * unit;
-    const double r1 = (double)q1 * runit, r2 = (double)q2 * runit;
+    auto radius = [&](long long q, int i) {
+        if (!GAS || q >= (1LL << 52)) return (double)q * runit;
+        const double *R = ds[c->drole[RR]], *V = ds[c->drole[RV3]], *O = ds[c->drole[RVO3]];
+        return fma(0.5 * c->dt, fma(3.0, V[i], -O[i]), R[i]);  // as k_predict
+    };
+    const double r1 = radius(q1, ij->x), r2 = radius(q2, ij->y);
     double m = dx * dx;
     m = fma(dy, dy, m);
     if (DIM == 3) m = fma(dz, dz, m);
@@ -272,10 +282,11 @@ static __device__ __noinline__ double pair_slow(long long ex, long long ey, long
     rs[0 * kT] = dx * s;
     rs[1 * kT] = dy * s;
     if (DIM == 3) rs[2 * kT] = dz * s;
-    const double r1sq = r1 * r1, r2sq = r2 * r2;
-    if (m < r1sq || m < r2sq) return fmin(r1sq, r2sq);
-    const double w = (r2sq - r1sq + m) * y;
-    return fabs(fma(-0.25 * w, w, r2sq));
+    // the half chord from the smaller bubble's side: its terms scale with it
+    const double lo = fmin(r1, r2), hi = fmax(r1, r2), losq = lo * lo, hisq = hi * hi;
+    if (m < hisq) return losq;
+    const double w = (losq + (m - hisq)) * y;
+    return fabs(fma(-0.25 * w, w, losq));
 }
 
 // A listed pair with a member that the fixed point does not hold, in FP64 from
@@ -357,6 +368,12 @@ static __device__ __noinline__ void scale_force(double f0, double *rs) {
     for (int a = 0; a < DIM; a++) rs[a * kT] *= f0;
 }
 
+// One radius (in its high words) less than 1/32 of the sum: see pair_slow.
+__device__ __forceinline__ bool uneven(long long q1, long long q2) {
+    const int a = (int)(q1 >> 32), b = (int)(q2 >> 32);
+    return min(a, b) < (a + b) >> 5;
+}
+
 // The difference of two fixed-point positions (modulo 2^64: one of them may be
 // the mark of a bubble beyond the range).
 __device__ __forceinline__ long long fix_diff(double a, double b) {
@@ -423,14 +440,14 @@ __device__ __forceinline__ void k_pairs_body(const Bufs &b, const int vb, const 
         double oa;
         FxTerms t;
         bool on = true;
-        if (fx_pair<DIM, GAS>(ex, ey, ez, q1, q2, fixb, t, radk)) {
+        if (!uneven(q1, q2) && fx_pair<DIM, GAS>(ex, ey, ez, q1, q2, fixb, t, radk)) {
             RS[0 * kT + e] = t.fx;
             RS[1 * kT + e] = t.fy;
             if (DIM == 3) RS[2 * kT + e] = t.fz;
             oa = t.oa;
             if (scaled) scale_force<DIM>(f0, RS + e);
         } else {
-            oa = pair_slow<DIM>(ex, ey, ez, q1, q2, radk, k, RS + e);
+            oa = pair_slow<DIM, GAS>(ex, ey, ez, q1, q2, radk, k, b.ds, c, QP + slot, RS + e);
             on = (q1 | q2) >= 0;
             if (GAS && !on) inv1 = inv2 = 0.0;
         }
@@ -833,7 +850,9 @@ __device__ __forceinline__ void k_correct_body(const Bufs &b, const int vb, cons
                 area = times4(ri.y);
             } else {
                 inv = p.w;
-                area = kPi * (is_far(p) ? CB_D(RVQ3)[i] : fx_to_double_signed(qr, -(fixb + radk)));
+                // too small for its unit (or marked): predicted again
+                area = kPi * (qr >= (1LL << 52) ? fx_to_double((uint64_t)qr, -(fixb + radk))
+                                                : fma(h, fma(3.0, v3, -CB_D(RVO3)[i]), r0));
             }
             double vr = mfa - inv;
             vr *= mfb * (area - ov);

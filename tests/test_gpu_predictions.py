@@ -199,3 +199,44 @@ def test_a_radius_beyond_what_the_search_saw(oracle_mod, dim, options, precision
     assert_rows_close(a, b, rows, 1e-13, "grown ")
     for k in ("total_overlap_area", "total_area", "max_error", "total_volume_new"):
         assert a[k] == pytest.approx(b[k], rel=1e-13), k
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_overlaps_of_bubbles_much_smaller_than_their_partner(dim, precision):
+    """Bubbles of 2^-4 ... 2^-14 of their one partner's radius, inside it or cut
+    by its surface, against exact rational arithmetic. Bar: a contained bubble's
+    area to 4 roundings of FP64; of a cut one the rounding of (r2^2 - r1^2 + d^2),
+    2^-53 R^2 a term, against r R: 2^-50 R / r."""
+    from fractions import Fraction as F
+
+    cfg, st = lattice(dim, 18.0, min_rad=0.0)
+    n = len(st["r"])
+    rng = np.random.default_rng(8)
+    at = np.arange(6) * 3.0 + 1.0
+    grid = np.meshgrid(*([at] * dim), indexing="ij")
+    big = {k: g.ravel() for k, g in zip("xyz", grid)}
+    small = np.round(2.0 ** -(4 + np.arange(n) % 11) * rng.uniform(1.0, 1.9, n) * 2.0 ** 40) / 2.0 ** 40
+    inside = np.arange(n) // 11 % 2 == 0
+    d = np.where(inside, 0.3, np.sqrt(1.0 + small ** 2 * rng.uniform(0.05, 0.5, n)))
+    d = np.round(d * 2.0 ** 44) / 2.0 ** 44  # from a box face at 0: exact sums
+    st = {"x": np.concatenate([big["x"], big["x"] + d]), "r": np.concatenate([np.ones(n), small])}
+    for k in "yz":
+        st[k] = np.tile(big.get(k, np.zeros(n)), 2)
+    cfg.capacity, cfg.pair_capacity = 2 * n, 64 * n
+    g = cb.GpuFoam(workloads.sweep_config_as(cfg, precision=precision))
+    g.load_state(st)
+    g.search_neighbors()
+    a, s = g.attempt(), g.get_state()
+    row = np.argsort(s["index"])
+    for i in range(n):
+        r = F(float(st["r"][n + i]))
+        m = (F(float(st["x"][n + i])) - F(float(st["x"][i]))) ** 2
+        if inside[i]:
+            q, bar = r * r, 4 * 2.0 ** -53
+        else:
+            assert m > 1 and m < (1 + r) ** 2
+            q, bar = r * r - (r * r - 1 + m) ** 2 / (4 * m), 2.0 ** -50 / float(r)
+        want = np.pi * float(q) if dim == 3 else 2.0 * np.sqrt(float(q))
+        got = a["overlap"][row[n + i]]
+        assert abs(got - want) <= bar * want, (i, inside[i], float(r), got, want)
