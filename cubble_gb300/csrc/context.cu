@@ -269,7 +269,7 @@ namespace {
 // phase inside a graph. us per attempt on one GB300 (searches included),
 // launches per phase -> resident run:
 //   FP64  2D  N = 10^3 52 -> 15, 10^4 52 -> 17, 2 10^5 97 -> 48,
-//             10^6 194 -> 175, 3 10^6 462 -> 449
+//             10^6 194 -> 180, 3 10^6 462 -> 449
 //         3D  4 10^3 53 -> 15, 3 10^4 59 -> 22, 3 10^5 145 -> 84,
 //             10^6 260 -> 235, 3 10^6 657 -> 643, 6 10^6 1254 -> 1257
 //   mixed 2D  10^4 34 -> 14, 2 10^5 45 -> 31, 10^6 103 -> 91, 3 10^6 246 -> 235

@@ -29,9 +29,10 @@ __device__ __forceinline__ double4_32a ld4(const double *p, int i) {
 // after a large dt or as it was loaded, its radius is negative or has outgrown
 // what the last search saw, or one of them is NaN) has a marked record, and its
 // state in spare rows that only a search uses: its terms are then evaluated in
-// FP64 (far_pairs, far_moves and RealPlace below).
-// The mark lies 2^62 units or more from every other bubble, and its radius is the
-// only one below zero: the loop over the pairs needs no test for it.
+// FP64 (far_pairs, far_moves and RealPlace below). The loop over the pairs needs
+// no test for the mark: it lies 2^62 units from every other bubble (before the
+// periodic image), and where that still counts as an overlap its radius, the only
+// one below zero, leads to pair_slow, which gives nothing.
 constexpr long long kFarRecord = (long long)0x8000000000000000ULL;
 __device__ __forceinline__ bool is_far(double4_32a p) {  // |q| < 2^62 in the others
     return __double2hiint(p.x) == (int)0x80000000;
@@ -167,7 +168,7 @@ CB_KERNEL_PAIR((template <int DIM>), k_predict, (<DIM>), __launch_bounds__(kBloc
 //     instead of five (alone: 202 -> 177 us);
 //   * overlap areas are accumulated in units of ov_unit (pi in 3D, 2 in 2D);
 //     the unit is applied to the global sums and in the correct kernel.
-// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 120 us (2D 117 -> 85, 3D
+// 3D, N = 10^6, 4.67 10^6 pairs, one GB300: 202 -> 121 us (2D 117 -> 89, 3D
 // without gas exchange 141 -> 96). Nothing is saturated now: issue 61 %, L1 61 %
 // of its wavefronts, FP64 33 %; three or four blocks per SM make no difference,
 // record loads a chunk ahead (108 registers) cost 8 us.
